@@ -880,47 +880,70 @@ cudaError_t f32_vterm(const WaveView &w, const EpiArgs &e, const float *scratch,
     return cudaGetLastError();
 }
 
-// Deterministic compensated sum of the per-job energies, fixed order: each of
-// kRedBlocks CTAs sums a fixed contiguous chunk (Neumaier), then one CTA sums
-// the partials in block order.
-constexpr int kRedBlocks = kReduceParts;
+// Deterministic compensated sum of the per-job energies, fixed order: each
+// CTA sums a fixed contiguous chunk (Neumaier pairs, merged down fixed shuffle
+// trees), then one CTA merges the partials the same way.  A single thread
+// merging the 2048 values of its CTA, and one more the 256 partials, took 57 us
+// whatever n was; the trees take 6 us at n = 220 and 9 us at n = 295,240.
+constexpr int kRedThreads = 256;
 
-__global__ void __launch_bounds__(1024) reduce_energy_part_kernel(const double *job_e, long long n, double *part) {
-    __shared__ double ss[1024], cc[1024];
+// the pair (s, c) of a CTA's threads merged in a fixed order; valid in thread 0
+__device__ __forceinline__ KSum block_ksum(KSum k) {
+    __shared__ double ws[32], wc[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    auto tree = [](KSum &x, int top) {
+        for (int m = top; m >= 1; m >>= 1) {
+            const double s2 = __shfl_down_sync(0xffffffffu, x.s, m), c2 = __shfl_down_sync(0xffffffffu, x.c, m);
+            x.c += c2;
+            x.add(s2);
+        }
+    };
+    tree(k, 16);
+    if (lane == 0) { ws[warp] = k.s; wc[warp] = k.c; }
+    __syncthreads();
+    if (warp == 0) {
+        k.s = lane < nw ? ws[lane] : 0.0;
+        k.c = lane < nw ? wc[lane] : 0.0;
+        tree(k, 16);
+    }
+    return k;
+}
+
+// out: nullable; with it (a single CTA) the sum itself, else this CTA's pair into part
+__global__ void __launch_bounds__(kRedThreads) reduce_energy_part_kernel(const double *job_e, long long n,
+                                                                         double *part, double *out) {
     const long long chunk = (n + gridDim.x - 1) / gridDim.x;
     const long long lo = blockIdx.x * chunk, hi = lo + chunk < n ? lo + chunk : n;
     KSum k;
-    for (long long i = lo + threadIdx.x; i < hi; i += blockDim.x) k.add(job_e[i]);
-    ss[threadIdx.x] = k.s;
-    cc[threadIdx.x] = k.c;
-    __syncthreads();
+    for (long long i = lo + threadIdx.x; i < hi; i += kRedThreads) k.add(job_e[i]);
+    k = block_ksum(k);
     if (threadIdx.x == 0) {
-        KSum t;
-        for (int i = 0; i < blockDim.x; ++i) { t.add(ss[i]); t.add(cc[i]); }
-        part[2 * blockIdx.x] = t.s;
-        part[2 * blockIdx.x + 1] = t.c;
+        if (out) {
+            out[0] = k.value();
+        } else {
+            part[2 * blockIdx.x] = k.s;
+            part[2 * blockIdx.x + 1] = k.c;
+        }
     }
 }
 
-__global__ void reduce_energy_final_kernel(const double *part, int nparts, double *out) {
-    KSum t;
-    for (int i = 0; i < 2 * nparts; ++i) t.add(part[i]);
-    out[0] = t.value();
+__global__ void __launch_bounds__(kRedThreads) reduce_energy_final_kernel(const double *part, int nparts,
+                                                                          double *out) {
+    KSum k;
+    for (int i = threadIdx.x; i < nparts; i += kRedThreads) {
+        k.add(part[2 * i]);
+        k.c += part[2 * i + 1];
+    }
+    k = block_ksum(k);
+    if (threadIdx.x == 0) out[0] = k.value();
 }
 
 // single-CTA variant (no work buffer)
 __global__ void __launch_bounds__(1024) reduce_energy_kernel(const double *job_e, long long n, double *out) {
-    __shared__ double ss[1024], cc[1024];
     KSum k;
     for (long long i = threadIdx.x; i < n; i += blockDim.x) k.add(job_e[i]);
-    ss[threadIdx.x] = k.s;
-    cc[threadIdx.x] = k.c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        KSum t;
-        for (int i = 0; i < blockDim.x; ++i) { t.add(ss[i]); t.add(cc[i]); }
-        out[0] = t.value();
-    }
+    k = block_ksum(k);
+    if (threadIdx.x == 0) out[0] = k.value();
 }
 
 cudaError_t reduce_energy_1cta(const double *job_e, long long n, double *e_out, cudaStream_t st) {
@@ -929,8 +952,10 @@ cudaError_t reduce_energy_1cta(const double *job_e, long long n, double *e_out, 
 }
 
 cudaError_t reduce_energy(const double *job_e, long long n, double *e_out, double *work, cudaStream_t st) {
-    reduce_energy_part_kernel<<<kRedBlocks, 1024, 0, st>>>(job_e, n, work);
-    reduce_energy_final_kernel<<<1, 1, 0, st>>>(work, kRedBlocks, e_out);
+    // one CTA up to 8 values a thread (the second launch costs more than it saves)
+    const int parts = n <= 8 * kRedThreads ? 1 : (int)(n / kRedThreads < kReduceParts ? n / kRedThreads : kReduceParts);
+    reduce_energy_part_kernel<<<parts, kRedThreads, 0, st>>>(job_e, n, work, parts == 1 ? e_out : nullptr);
+    if (parts > 1) reduce_energy_final_kernel<<<1, kRedThreads, 0, st>>>(work, parts, e_out);
     return cudaGetLastError();
 }
 

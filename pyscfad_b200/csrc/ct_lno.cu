@@ -333,12 +333,24 @@ static cudaError_t launch(const WaveView &w, const EpiArgs &e, CT *scratch, cuda
     return e.o <= 32 ? launch_nt<4, CT, QRT, VJP>(w, e, scratch, st) : launch_nt<8, CT, QRT, VJP>(w, e, scratch, st);
 }
 
-__global__ void mat_bar_kernel(const double *part, int n_jobs, int oo, double *mat_bar) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= oo) return;
+// mat_bar += the jobs' partials: 32 elements per CTA, 32 thread rows taking
+// every 32nd job, their sums merged in a fixed order (one thread per element
+// walking all jobs was bound by its chain of loads)
+__global__ void __launch_bounds__(1024) mat_bar_kernel(const double *part, int n_jobs, int oo, double *mat_bar) {
+    __shared__ double acc[32][33];
+    const int i = blockIdx.x * 32 + threadIdx.x;
     double s = 0.0;
-    for (int j = 0; j < n_jobs; ++j) s += part[(long long)j * oo + i];
-    mat_bar[i] += s;
+    if (i < oo) {
+#pragma unroll 4
+        for (int j = threadIdx.y; j < n_jobs; j += 32) s += part[(long long)j * oo + i];
+    }
+    acc[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    for (int m = 16; m >= 1; m >>= 1) {
+        if ((int)threadIdx.y < m) acc[threadIdx.y][threadIdx.x] += acc[threadIdx.y + m][threadIdx.x];
+        __syncthreads();
+    }
+    if (threadIdx.y == 0 && i < oo) mat_bar[i] += acc[0][threadIdx.x];
 }
 
 }  // namespace lnoproj
@@ -363,7 +375,7 @@ cudaError_t f32_lno_vjp_project(const WaveView &w, const EpiArgs &e, float *scra
 cudaError_t f64_lno_mat_bar(const WaveView &w, const EpiArgs &e, double *mat_bar, cudaStream_t st) {
     if (w.n_jobs <= 0) return cudaSuccess;
     const int oo = e.o * e.o;
-    lnoproj::mat_bar_kernel<<<(oo + 255) / 256, 256, 0, st>>>(e.lno_mat_bar_part, w.n_jobs, oo, mat_bar);
+    lnoproj::mat_bar_kernel<<<(oo + 31) / 32, dim3(32, 32), 0, st>>>(e.lno_mat_bar_part, w.n_jobs, oo, mat_bar);
     return cudaGetLastError();
 }
 
