@@ -497,13 +497,20 @@ static double scratch_budget_mb(Workspace &W) {
     return W.budget_mb;
 }
 
+// The float64 path that keeps a job's cube in shared memory (ct_cube.cu): its
+// largest cube, V tiles and partials take 193 KB at nocc = 24.  nocc = 1 stays
+// on the slot path (a cube of one element).
+static bool use_cube(int o, int mode) { return mode == CT_MODE_FP64 && o >= 2 && o <= kCubeMaxO; }
+
 // Jobs per wave: as many as the scratch budget holds (at most 8192), rounded
 // down to a multiple of two CTAs per SM so the per-job kernels fill whole
-// rounds of the GPU.
+// rounds of the GPU.  On the cube path a wave's w-bar cubes (o^3 doubles a
+// job) also stay below 96 MB, so that the t2-bar GEMM finds them in L2.
 static int max_wave_jobs(Workspace &W, int o, int mode) {
     const double per_job = (double)kSlots * o * o * o * scratch_elt(mode)
                          + (mode == CT_MODE_FP64 ? 0.0 : mixed_extra_bytes_per_job(o, mode));
     long long mw = (long long)(scratch_budget_mb(W) * 1048576.0 / per_job);
+    if (use_cube(o, mode)) mw = std::min<long long>(mw, (96LL << 20) / (8LL * o * o * o));
     mw = std::max<long long>(1, std::min<long long>(mw, 8192));
     const long long round = 2LL * (W.sm_count > 0 ? W.sm_count : 148);
     if (mw >= round) mw -= mw % round;
@@ -598,6 +605,13 @@ static int run_waves(Workspace &W, const Plan &P, const ct_problem *p, int mode,
                      const EpiArgs &ea, const MixedOperands &mo, double *lno_mat_bar, cudaStream_t st) {
     const int o = p->nocc, v = p->nvir, n = o + v;
     const double *lno_mat = ea.lno_mat;
+    const bool cube = use_cube(o, mode) && !ea.t3_c;
+    if (cube && !vjp && !lno_mat) {
+        // no scratch: every job of the plan in one launch
+        CT_PROF(PK_F1);
+        CT_CK(cube_energy(P.d_jobs, (int)P.jobs.size(), ea, p->vooo, st));
+        return CT_OK;
+    }
     for (int w = 0; w < P.n_waves(); ++w) {
         WaveView wv{};
         wv.o = o; wv.v = v; wv.n = n;
@@ -615,7 +629,29 @@ static int run_waves(Workspace &W, const Plan &P, const ct_problem *p, int mode,
         wv.xchunks = P.d_xchunks + 3 * P.xchunk_begin[w];
         wv.n_ochunks = P.ochunk_begin[w + 1] - P.ochunk_begin[w];
         wv.ochunks = P.d_ochunks + 3 * P.ochunk_begin[w];
-        if (mode == CT_MODE_FP64) {
+        if (cube) {
+            double *S = (double *)W.scratch;
+            long long stride = (long long)o * o * o;
+            if (lno_mat) {
+                EpiArgs ef = ea;
+                ef.with_vjp = 0;
+                ef.lno_phase = 1;
+                { CT_PROF(PK_F1); CT_CK(cube_lno_forward(wv, ef, p->vooo, S, st)); }
+                if (!vjp) {
+                    CT_PROF(PK_VT);
+                    CT_CK(f64_lno_contract(wv, ea, S, st));
+                    continue;
+                }
+                { CT_PROF(PK_RED); CT_CK(f64_lno_vjp_project(wv, ea, S, st)); }
+                { CT_PROF(PK_VB); CT_CK(cube_lno_backward(wv, ea, p->vooo, g->vooo, S, st)); }
+                { CT_PROF(PK_RED); CT_CK(f64_lno_mat_bar(wv, ea, lno_mat_bar, st)); }
+                stride *= kSlots;
+            } else {
+                CT_PROF(PK_F1);
+                CT_CK(cube_vjp(wv, ea, p->vooo, g->vooo, S, st));
+            }
+            { CT_PROF(PK_TB); CT_CK(cube_tb(wv, ea, S, stride, W.sm_count, st)); }
+        } else if (mode == CT_MODE_FP64) {
             double *S = (double *)W.scratch;
             { CT_PROF(PK_F1); CT_CK(f64_gemm(K_F1, wv, p->t2T, p->vvop, S, S, st)); }
             { CT_PROF(PK_F2); CT_CK(f64_gemm(K_F2, wv, p->vooo, p->t2T, S, S, st)); }

@@ -84,6 +84,21 @@ cudaError_t f64_gemm(GemmKind kind, const WaveView &w, const double *A, const do
                      double *scratch, cudaStream_t st);
 cudaError_t f64_epilogue(const WaveView &w, const EpiArgs &e, double *scratch, cudaStream_t st);
 cudaError_t f64_vterm(const WaveView &w, const EpiArgs &e, const double *scratch, cudaStream_t st);
+// float64 path for 2 <= nocc <= kCubeMaxO (ct_cube.cu): one CTA per job with its
+// cube in shared memory.  Energy over a job list (no scratch); per wave the
+// VJP (w-bar cube of job jl to cubes + jl o^3) or the two LNO passes (slots
+// 0-5 as f64_lno_* use them; the backward pass leaves w-bar in slot 0), then
+// the t2-bar GEMM over the wave's w-bar cubes
+constexpr int kCubeMaxO = 24;
+cudaError_t cube_energy(const int *jobs, int n_jobs, const EpiArgs &e, const double *vooo, cudaStream_t st);
+cudaError_t cube_vjp(const WaveView &w, const EpiArgs &e, const double *vooo, double *vooo_bar, double *cubes,
+                     cudaStream_t st);
+cudaError_t cube_lno_forward(const WaveView &w, const EpiArgs &e, const double *vooo, double *slots,
+                             cudaStream_t st);
+cudaError_t cube_lno_backward(const WaveView &w, const EpiArgs &e, const double *vooo, double *vooo_bar,
+                              double *slots, cudaStream_t st);
+cudaError_t cube_tb(const WaveView &w, const EpiArgs &e, const double *cubes, long long stride, int sms,
+                    cudaStream_t st);
 // LNO projections (ct_lno.cu).  The energy of each job of the wave from the
 // W and z/D cubes the epilogue leaves in slots 0 and 1 (writes e.job_e)
 cudaError_t f64_lno_contract(const WaveView &w, const EpiArgs &e, const double *scratch, cudaStream_t st);
