@@ -83,6 +83,12 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
                  : "+d"(d[0]), "+d"(d[1])
                  : "d"(a), "d"(b));
 }
+
+// 8-byte asynchronous global -> shared copy, zero-filled when !ok (src is then not read)
+__device__ __forceinline__ void cp_async8(void *smem_dst, const void *src, bool ok) {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
+}
 #endif
 
 }  // namespace ctb

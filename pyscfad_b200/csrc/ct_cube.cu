@@ -68,12 +68,6 @@ __device__ __forceinline__ int rtR(int s, int m) {
     return (int)((P >> (6 * s + 2 * m)) & 3);
 }
 
-// 8-byte asynchronous copy; zero-filled when !ok
-__device__ __forceinline__ void cp_async8(void *smem_dst, const void *gmem_src, bool ok) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(gmem_src), "r"(ok ? 8 : 0) : "memory");
-}
-
 template <int MT, int NT, int MODE, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
     extern __shared__ __align__(16) double sm[];

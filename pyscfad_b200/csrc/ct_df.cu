@@ -17,6 +17,7 @@
 // split as (x / div, x % div) and weighted by two strides, which covers every
 // permuted layout above.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <climits>
 #include "ct_common.cuh"
 #include "ct_internal.h"
@@ -37,89 +38,103 @@ struct Opd {
 __host__ __device__ inline Ix ix_plain(long long s) { return Ix{INT_MAX, 0, s}; }
 __host__ __device__ inline Ix ix_two(int div, long long s1, long long s0) { return Ix{div, s1, s0}; }
 
-constexpr int BM = 64, BN = 64, BK = 16, NTHR = 256, LD = 64 + 4;
+constexpr int BM = 128, BN = 64, BK = 8, NTHR = 256, STAGES = 4;
+constexpr int LDA = BM + 4, LDB = BN + 4;   // 4 mod 16 doubles: conflict-free fragments
+constexpr size_t kSmem = sizeof(double) * STAGES * BK * (LDA + LDB);
 
-// One operand's slice of a K step: 4 loads per thread.  mn_fast: consecutive
-// threads take consecutive rows (m or n), else consecutive k.  The k part of
-// each load's address is kept as (quotient, remainder) and advanced by BK
-// without divisions.
-struct Loader {
-    long long base[4];   // address part of the m (or n) index; -1 when out of range
-    int kq[4], kr[4];    // k = kq * div + kr for this load
-    int kl[4], ml[4];    // tile coordinates
-    __device__ void init(const Ix &mix, const Ix &kix, int m0, int M, bool mn_fast) {
-        const int t = threadIdx.x;
-        for (int j = 0; j < 4; ++j) {
-            int m, k;
-            if (mn_fast) { m = t % 64; k = t / 64 + 4 * j; }
-            else { k = t % 16; m = t / 16 + 16 * j; }
-            ml[j] = m;
-            kl[j] = k;
-            const int gm = m0 + m;
+// One operand's slice of a K step: W x BK elements, NL per thread.  MF:
+// consecutive threads take consecutive rows (m or n) of one k, so a thread's
+// loads share the row and differ in k; else consecutive k, one k per thread and
+// several rows.  The k part of an address is kept as (quotient, remainder) and
+// advanced by BK without divisions.
+template <int W, bool MF> struct Loader {
+    static constexpr int NL = W * BK / NTHR, NB = MF ? 1 : NL, NK = MF ? NL : 1;
+    long long base[NB];   // address part of the m (or n) index; -1 when out of range
+    int kq[NK], kr[NK];   // k = kq * div + kr
+    int off, k0;          // first position in the staged tile and its k within the step
+    __device__ __forceinline__ void init(const Ix &mix, const Ix &kix, int m0, int M, int kb) {
+        const int t = threadIdx.x, m = MF ? t % W : t / BK;
+        k0 = MF ? t / W : t % BK;
+        off = k0 * (W + 4) + m;
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+            const int gm = m0 + m + NTHR / BK * j;
             base[j] = gm < M ? (long long)(gm / mix.div) * mix.s1 + (long long)(gm % mix.div) * mix.s0 : -1;
+        }
+#pragma unroll
+        for (int j = 0; j < NK; ++j) {
+            const int k = kb + k0 + NTHR / W * j;
             kq[j] = k / kix.div;
             kr[j] = k % kix.div;
         }
     }
-    __device__ void load(const double *p, const Ix &kix, int kb, int K, double (&v)[4]) const {
-        for (int j = 0; j < 4; ++j) {
-            const bool ok = base[j] >= 0 && kb + kl[j] < K;
-            v[j] = ok ? p[base[j] + (long long)kq[j] * kix.s1 + (long long)kr[j] * kix.s0] : 0.0;
+    // copies the step at kb and moves on to the next one
+    __device__ __forceinline__ void copy(double *dst, const double *p, const Ix &kix, int kb, int K) {
+#pragma unroll
+        for (int j = 0; j < NL; ++j) {
+            const int jb = MF ? 0 : j, jk = MF ? j : 0;
+            const bool ok = base[jb] >= 0 && kb + k0 + (MF ? NTHR / W * j : 0) < K;
+            const long long a = base[jb] + (long long)kq[jk] * kix.s1 + (long long)kr[jk] * kix.s0;
+            cp_async8(dst + off + (MF ? NTHR / W * (W + 4) : NTHR / BK) * j, ok ? p + a : p, ok);
         }
-    }
-    __device__ void advance(const Ix &kix) {
-        for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int j = 0; j < NK; ++j) {
             kr[j] += BK;
             while (kr[j] >= kix.div) { kr[j] -= kix.div; ++kq[j]; }
         }
     }
 };
 
-// C[m,n] = alpha sum_k A[m,k] B[k,n] (+ C[m,n] when acc); 64 x 64 tiles, 8 warps
-// of 32 x 16 (4 x 2 DMMA tiles), K steps of 16 staged in shared memory with a
-// register prefetch of the next step.
-__global__ void __launch_bounds__(NTHR) gemm_strided_kernel(int M, int N, int K, Opd A, Opd B, double *C, Ix cr,
-                                                            Ix cc, double alpha, int acc, int a_mfast,
-                                                            int b_nfast) {
-    __shared__ double As[BK][LD], Bs[BK][LD];
+// C[m,n] = alpha sum_k A[m,k] B[k,n] (+ C[m,n] when acc); 128 x 64 tiles, 8 warps
+// of 32 x 32 (4 x 4 DMMA tiles), K steps of 8 in a four-stage cp.async ring.
+// Bound by the DMMA pipe: a 64 x 64 tile with one shared buffer and 8 DMMAs per
+// six fragment loads ran the nocc=16/nvir=120/naux=360 producer and its VJP
+// (69 GFLOP) in 4.6 ms of kernels, this one in 3.3 ms (21 of 37 TFLOP/s).
+template <bool AMF, bool BNF>
+__global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int K, Opd A, Opd B, double *C, Ix cr,
+                                                               Ix cc, double alpha, int acc) {
+    extern __shared__ __align__(16) double dsm[];
+    double *As = dsm, *Bs = dsm + STAGES * BK * LDA;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
-    const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16;
-    Loader la, lb;
-    la.init(A.r, A.c, m0, M, a_mfast != 0);
-    lb.init(B.c, B.r, n0, N, b_nfast != 0);
-    double d[4][2][2];
+    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+    Loader<BM, AMF> la;
+    Loader<BN, BNF> lb;
+    // gridDim.z parts of K (whole steps); more than one part adds atomically
+    const int steps = (K + BK - 1) / BK;
+    const int sb = (int)((long long)steps * blockIdx.z / gridDim.z);
+    const int nk = (int)((long long)steps * (blockIdx.z + 1) / gridDim.z) - sb;
+    la.init(A.r, A.c, m0, M, sb * BK);
+    lb.init(B.c, B.r, n0, N, sb * BK);
+    double d[4][4][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j) d[i][j][0] = d[i][j][1] = 0.0;
-    double va[4], vb[4];
-    la.load(A.p, A.c, 0, K, va);
-    lb.load(B.p, B.r, 0, K, vb);
-    for (int kb = 0; kb < K; kb += BK) {
-        __syncthreads();
-        for (int j = 0; j < 4; ++j) {
-            As[la.kl[j]][la.ml[j]] = va[j];
-            Bs[lb.kl[j]][lb.ml[j]] = vb[j];
+        for (int j = 0; j < 4; ++j) d[i][j][0] = d[i][j][1] = 0.0;
+    auto issue = [&](int s) {
+        if (s < nk) {
+            la.copy(As + (s % STAGES) * BK * LDA, A.p, A.c, (sb + s) * BK, K);
+            lb.copy(Bs + (s % STAGES) * BK * LDB, B.p, B.r, (sb + s) * BK, K);
         }
-        __syncthreads();
-        if (kb + BK < K) {
-            la.advance(A.c);
-            lb.advance(B.r);
-            la.load(A.p, A.c, kb + BK, K, va);
-            lb.load(B.p, B.r, kb + BK, K, vb);
-        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) issue(s);
+    for (int s = 0; s < nk; ++s) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();   // step s landed for every thread; step s - 1's buffer is free
+        issue(s + STAGES - 1);
+        const double *a_ = As + (s % STAGES) * BK * LDA + c * LDA + wm + g;
+        const double *b_ = Bs + (s % STAGES) * BK * LDB + c * LDB + wn + g;
 #pragma unroll
         for (int kk = 0; kk < BK; kk += 4) {
-            double a[4], b[2];
+            double a[4], b[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk + c][wm + 8 * i + g];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) b[j] = Bs[kk + c][wn + 8 * j + g];
+            for (int i = 0; i < 4; ++i) { a[i] = a_[kk * LDA + 8 * i]; b[i] = b_[kk * LDB + 8 * i]; }
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 2; ++j) dmma(d[i][j], a[i], b[j]);
+                for (int j = 0; j < 4; ++j) dmma(d[i][j], a[i], b[j]);
         }
     }
 #pragma unroll
@@ -128,13 +143,14 @@ __global__ void __launch_bounds__(NTHR) gemm_strided_kernel(int M, int N, int K,
         if (m >= M) continue;
         const long long rm = (long long)(m / cr.div) * cr.s1 + (long long)(m % cr.div) * cr.s0;
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int n = n0 + wn + 8 * j + 2 * c + h;
                 if (n >= N) continue;
                 double *dst = C + rm + (long long)(n / cc.div) * cc.s1 + (long long)(n % cc.div) * cc.s0;
-                *dst = acc ? *dst + alpha * d[i][j][h] : alpha * d[i][j][h];
+                if (gridDim.z > 1) atomicAdd(dst, alpha * d[i][j][h]);
+                else *dst = acc ? *dst + alpha * d[i][j][h] : alpha * d[i][j][h];
             }
     }
 }
@@ -144,10 +160,19 @@ static cudaError_t gemm(int M, int N, int K, const Opd &A, const Opd &B, double 
     if (M <= 0 || N <= 0 || K <= 0) return cudaSuccess;
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return cudaErrorInvalidValue;
-    const int a_mfast = A.r.s0 == 1 && A.r.div == INT_MAX ? 1 : (A.r.div != INT_MAX && A.r.s0 == 1 ? 1 : 0);
-    const int b_nfast = B.c.s0 == 1 ? 1 : 0;
-    gemm_strided_kernel<<<grid, NTHR, 0, st>>>(M, N, K, A, B, C, cr, cc, alpha, acc ? 1 : 0, a_mfast, b_nfast);
-    return cudaGetLastError();
+    // An accumulating product with few tiles (the factor gradients: naux rows)
+    // splits K so that two CTAs per SM have work, each part >= 64 steps
+    const long long tiles = (long long)grid.x * grid.y;
+    if (acc && tiles < 296) grid.z = (unsigned)std::max(1LL, std::min(592 / tiles, (long long)K / (64 * BK)));
+    auto go = [&](auto kern) {
+        const cudaError_t ce = smem_optin(reinterpret_cast<const void *>(kern), (int)kSmem);
+        if (ce != cudaSuccess) return ce;
+        kern<<<grid, NTHR, kSmem, st>>>(M, N, K, A, B, C, cr, cc, alpha, acc ? 1 : 0);
+        return cudaGetLastError();
+    };
+    // consecutive threads along the operand's contiguous index
+    if (A.r.s0 == 1) return B.c.s0 == 1 ? go(gemm_strided_kernel<true, true>) : go(gemm_strided_kernel<true, false>);
+    return B.c.s0 == 1 ? go(gemm_strided_kernel<false, true>) : go(gemm_strided_kernel<false, false>);
 }
 
 }  // namespace df
