@@ -388,6 +388,8 @@ struct Workspace {
     int n_orb = 0;
     double *e_tmp = nullptr;
     double *red_work = nullptr;     // 2 * kReduceParts partial sums
+    double *lno_part = nullptr;     // LNO VJP: per-job partials of mat_bar, one wave
+    long long lno_part_n = 0;
     HostPathCache hp;
     Prof prof;
     cudaEvent_t prof_open[kProfKinds] = {};
@@ -405,6 +407,9 @@ struct Workspace {
         if (orbits) cudaFree(orbits);
         if (e_tmp) cudaFree(e_tmp);
         if (red_work) cudaFree(red_work);
+        if (lno_part) cudaFree(lno_part);
+        lno_part = nullptr;
+        lno_part_n = 0;
         scratch = nullptr; job_e = nullptr; orbits = nullptr; e_tmp = nullptr; red_work = nullptr;
         scratch_bytes = 0; job_e_n = 0; orb_o = -1; n_orb = 0;
         hp.release();
@@ -905,17 +910,21 @@ static int run_lno_vjp_locked(Workspace &W, const ct_problem *p, int mode, const
         if ((rc = upload_plan(W.block)) != CT_OK) { W.block.free_dev(); W.block = Plan(); return rc; }
         P = &W.block;
     }
-    double *part = nullptr;
-    CT_CK(cudaMallocAsync(&part, (size_t)mw * p->nocc * p->nocc * sizeof(double), st));
+    const long long n_part = (long long)mw * p->nocc * p->nocc;
+    if (n_part > W.lno_part_n) {
+        if (W.lno_part) cudaFree(W.lno_part);
+        W.lno_part = nullptr;
+        W.lno_part_n = 0;
+        CT_CK(cudaMalloc(&W.lno_part, n_part * sizeof(double)));
+        W.lno_part_n = n_part;
+    }
     LnoSel sel;
     sel.mat = mat;
     sel.a0 = 0; sel.a1 = v;
     sel.b0 = b0; sel.b1 = b1; sel.c0 = c0; sel.c1 = c1;
     sel.mat_bar = mat_bar;
-    sel.part = part;
-    rc = run_plan(W, *P, p, mode, true, et_bar, g, W.job_e, e_out, st, &sel);
-    cudaFreeAsync(part, st);
-    return rc;
+    sel.part = W.lno_part;
+    return run_plan(W, *P, p, mode, true, et_bar, g, W.job_e, e_out, st, &sel);
 }
 
 static int run_full(const ct_problem *p, int mode, bool vjp, double et_bar, const ct_grads *g,
