@@ -245,6 +245,16 @@ int ct_t3_init(const ct_problem *p, double *t3_c, double *t3_x, void *stream);
 int ct_t3_update(int nocc, int nvir, const double *mo_energy, const double *t3_c, const double *tvv,
                  const double *too_m, const double *t3, const double *t3_x, double *t3_new,
                  double *t3_new_m, double *sums, void *stream);
+/*
+ * The same update from t3 and the occupied Fock block (its diagonal is ignored)
+ * instead of from too_m: t3_new = t3_c + (P3(tvv) - P3(foo' t3)) / d3, with the
+ * foo' products formed inside.  nocc <= 64.  t3_new must not alias the inputs.
+ * work: device, CT_T3_STEP_WORK doubles of scratch for the two sums.
+ */
+#define CT_T3_STEP_WORK 4096
+int ct_t3_step(int nocc, int nvir, const double *mo_energy, const double *foo, const double *t3_c,
+               const double *tvv, const double *t3, const double *t3_x, double *t3_new, double *sums,
+               double *work, void *stream);
 
 /*
  * E(T) restricted to an explicit list of sorted virtual triples (no reference

@@ -9,15 +9,13 @@ The reference forms t3[i,j,k,a,b,c] with JAX einsums.  Here:
     the orbit epilogue of the float64 (T) path, which write every element at
     all simultaneous permutations of (a, b, c) and (i, j, k) (``ct_t3_init``);
   * a step is t3 <- t3_c + (P3(fvv' t3) - P3(foo' t3)) / d3 with fvv', foo'
-    the Fock blocks without their diagonals: the two products are one plain
-    GEMM each (cuBLAS): fvv' on the first virtual index of the
-    [a][b][c][i][j][k] array, foo' on the first occupied index of an
-    occupied-major copy [i][a][b][c][j][k]; the P3 sums, the division, the next
-    step's occupied-major copy and the fixed-order sums of |t3_new - t3|^2 and
-    of the energy are one kernel (``ct_t3_update``).
+    the Fock blocks without their diagonals: fvv' t3 on the first virtual index
+    is one plain GEMM (cuBLAS); the foo' products, the P3 sums, the division
+    and the fixed-order sums of |t3_new - t3|^2 and of the energy are one
+    kernel (``ct_t3_step``).
 ``t3`` is returned as the reference's [i,j,k,a,b,c] view.  DIIS (the
 reference's optional ``run_diis``) and the implicit-differentiation backward
-of ``make_implicit_diff`` are not built.  Memory: eight (v^3 o^3) float64
+of ``make_implicit_diff`` are not built.  Memory: five (v^3 o^3) float64
 arrays on the device.
 """
 from __future__ import annotations
@@ -55,7 +53,7 @@ def t3_seed(L: dict):
 
 
 def _offdiag(f):
-    f = f.clone()
+    f = f.clone(memory_format=torch.contiguous_format)   # ct_t3_step reads foo by rows
     f.diagonal().zero_()
     return f
 
@@ -88,10 +86,9 @@ def iterative_kernel(mycc, eris=None, t1=None, t2=None, t3=None, max_cycle=50, t
     else:
         cur = torch.as_tensor(t3, dtype=torch.float64).to(dev).permute(3, 4, 5, 0, 1, 2).contiguous()
     et = float(torch.sum(cur * t3x))
-    cur_m = cur.permute(3, 0, 1, 2, 4, 5).contiguous()     # [i][a][b][c][j][k]
-    tvv, too_m = torch.empty_like(t3c), torch.empty_like(t3c)
-    new, new_m = torch.empty_like(t3c), torch.empty_like(t3c)
+    tvv, new = torch.empty_like(t3c), torch.empty_like(t3c)
     sums = torch.zeros(2, dtype=torch.float64, device=dev)
+    work = torch.empty(native.T3_STEP_WORK, dtype=torch.float64, device=dev)
     conv = False
     ncyc = 0
     ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)] if stats is not None else None
@@ -100,16 +97,13 @@ def iterative_kernel(mycc, eris=None, t1=None, t2=None, t3=None, max_cycle=50, t
             ev[0].record()
         for _ in range(max_cycle):
             ncyc += 1
-            # fvv' t3 on the first virtual index; foo' t3 on the first occupied
-            # index of the occupied-major copy
+            # fvv' t3 on the first virtual index; the step forms the foo' products itself
             torch.mm(fvv, cur.view(nvir, -1), out=tvv.view(nvir, -1))
-            torch.mm(foo, cur_m.view(nocc, -1), out=too_m.view(nocc, -1))
-            p = [ctypes.c_void_p(x.data_ptr()) for x in (L["mo_energy"], t3c, tvv, too_m, cur, t3x, new, new_m, sums)]
-            st = native.lib().ct_t3_update(nocc, nvir, *p, triples._stream(dev))
-            native.check(st, "ct_t3_update")
+            p = [ctypes.c_void_p(x.data_ptr()) for x in (L["mo_energy"], foo, t3c, tvv, cur, t3x, new, sums, work)]
+            st = native.lib().ct_t3_step(nocc, nvir, *p, triples._stream(dev))
+            native.check(st, "ct_t3_step")
             normt2, e_new = sums.tolist()
             cur, new = new, cur
-            cur_m, new_m = new_m, cur_m
             eold, et = et, e_new
             if abs(et - eold) < tol and normt2 ** 0.5 < tolnormt:
                 conv = True

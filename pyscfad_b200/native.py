@@ -22,10 +22,12 @@ EXPORTS = (
     "ct_profile_enable", "ct_profile_read", "ct_profile_reset", "ct_peak_probe",
     "ct_energy_noalloc", "ct_energy_jobs", "ct_lno_energy", "ct_lno_energy_mode", "ctb_lnoccsdt_contract",
     "ct_lno_energy_vjp",
-    "ct_lno_energy_vjp_block", "ct_lno_energy_vjp_mode", "ctb_lnoccsdt_energy_vjp", "ct_t3_init", "ct_t3_update",
+    "ct_lno_energy_vjp_block", "ct_lno_energy_vjp_mode", "ctb_lnoccsdt_energy_vjp", "ct_t3_init", "ct_t3_update", "ct_t3_step",
     "ct_mlp_forward", "ct_mlp_mse", "ct_mlp_work_floats", "ct_mlp_backward", "ct_mlp_adam",
     "ct_mlp_to_bf16", "ct_mlp_infer_bf16", "ct_surrogate_features", "ct_df_layouts", "ct_df_factor_bar",
 )
+
+T3_STEP_WORK = 4096     # doubles of ct_t3_step's work buffer (include/pyscfad_b200.h)
 
 # surrogate MLP shapes (include/pyscfad_b200.h)
 MLP_IN = 12
@@ -96,6 +98,8 @@ def lib():
     L.ct_t3_init.argtypes = [ctypes.POINTER(CtProblem), vp, vp, vp]
     L.ct_t3_update.restype = ci
     L.ct_t3_update.argtypes = [ci, ci, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
+    L.ct_t3_step.restype = ci
+    L.ct_t3_step.argtypes = [ci, ci, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
     L.ct_lno_energy_vjp_mode.restype = ci
     L.ct_lno_energy_vjp_mode.argtypes = [ctypes.POINTER(CtProblem), ci, vp, cd, ci, ci, ci, ci,
                                          ctypes.POINTER(CtGrads), vp, vp, vp]
