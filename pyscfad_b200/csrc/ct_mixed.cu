@@ -79,6 +79,7 @@ struct TcParams {
     unsigned o_magic;      // ceil(2^32 / o): i / o = umulhi(i, o_magic) for small i
     int pairs;              // work items cover two M-tiles (paired kinds)
     int nwork, m_tiles, n_tiles;
+    int tb_n;               // TB: accumulator columns per item (256 or 128)
     int stages, stage_bytes, a_bytes, b_bytes;   // a_bytes / b_bytes per operand plane
     const int *jobs;
     const int *groups;   // (key, e_begin, e_end) triples
@@ -151,8 +152,8 @@ __device__ __forceinline__ void decode(const TcParams &P, int w, Work &W) {
     case TK_VB: W.nk = (o2 + CK - 1) / CK;  W.N = ((W.nterms * o + 15) / 16) * 16; break;
     case TK_TB: {
         W.nk = W.nterms;
-        const int rem = o2 - W.nt * 256;
-        W.N = rem >= 256 ? 256 : ((rem + CK - 1) / CK) * CK;
+        const int rem = o2 - W.nt * P.tb_n;
+        W.N = rem >= P.tb_n ? P.tb_n : ((rem + CK - 1) / CK) * CK;
         break;
     }
     case TK_F2: W.nk = (o + CK - 1) / CK; W.N = W.nterms * P.ock; break;
@@ -161,16 +162,44 @@ __device__ __forceinline__ void decode(const TcParams &P, int w, Work &W) {
     }
 }
 
+// What a term's loads need, one term per lane of the producer warp: p0 and p1
+// are third tensor-map coordinates of its operands (vvop / t2T pair rows, W-bar slots)
+struct TermOps {
+    int p0, p1;
+};
+template <int KIND, int PREC>
+__device__ __forceinline__ TermOps term_ops(const TcParams &P, int eid, int job) {
+    const int jl = eid / 6, sg = eid - 6 * (eid / 6);
+    int a, b, c, x, y, z;
+    unpack_job(job, a, b, c);
+    term_xyz(sg, a, b, c, x, y, z);
+    const int xy = x * P.v + y, zy = z * P.v + y;
+    const int ws = PREC ? jl * 6 + sg : jl * kSlots + sg;
+    switch (KIND) {
+    case TK_F1: return {xy, 0};
+    case TK_VB: return {ws, 0};
+    case TK_TB: return {xy, ws};
+    case TK_F2: return {zy, 0};
+    case TK_OB1: return {zy, wsl_rot<PREC>(eid)};
+    default: return {wsl_rot<PREC>(eid), 0};   // OB2
+    }
+}
+
 // Issues the TMA loads of k-iteration kit into the stage at sA (planes
-// [A][A lo][B][B lo], each a_bytes / b_bytes); returns the bytes expected.
+// [A][A lo][B][B lo], each a_bytes / b_bytes).  Called by the whole producer
+// warp: lane 0 arms the full barrier, then every lane issues its own boxes (B
+// boxes of term t by lane t; A boxes, and the chunks of a one-term stage, by
+// consecutive lanes), so that a stage costs one or two issue slots instead of a
+// serial loop.  mine: this lane's term (F1, VB, F2, OB2: term `lane` of the
+// item; TB, OB1: the stage's term, the same in every lane).
 // CG2 (CTA pair, F1 only): this CTA (rank) loads its 128 rows of the item's
 // 256-row M-tile and its half of B, half-term boxes rank*nterms ..
 // (rank+1)*nterms - 1 of o/2 rows each; the bytes of both CTAs complete on
 // the leader's full barrier (cbar, shared::cluster address), whose
 // transaction count the leader sets.
 template <int KIND, int PREC, bool CG2 = false>
-__device__ __forceinline__ uint32_t issue_loads(const TcParams &P, const Work &W, int kit, uint32_t sA, uint32_t bar,
-                                                uint32_t rank = 0, uint32_t cbar = 0) {
+__device__ __forceinline__ void issue_loads(const TcParams &P, const Work &W, int kit, uint32_t sA, uint32_t bar,
+                                            const TermOps &mine, int lane, uint32_t rank = 0, uint32_t cbar = 0) {
     constexpr int CK = PREC ? 64 : 32;           // elements per 128-byte row
     constexpr uint32_t NP = PREC ? 2u : 1u;      // operand planes
     const int o = P.o;
@@ -193,65 +222,52 @@ __device__ __forceinline__ uint32_t issue_loads(const TcParams &P, const Work &W
             if (PREC) tc::tma_load_3d(sB + P.b_bytes + off, &P.mapB2, bar, c0, c1, c2);
         }
     };
+    // bytes: per plane
+    auto arm = [&](uint32_t bytes) {
+        if (lane == 0) tc::mbar_expect_tx(bar, NP * bytes);
+        __syncwarp();
+    };
     const uint32_t chunk = (uint32_t)CK * 128u;  // bytes of a CK x CK MN-major chunk
-    uint32_t bytes = 0;                          // per plane
     if constexpr (CG2) {
         static_assert(KIND == TK_F1, "CTA-pair loads are laid out for F1");
         const int hr = o / 2;                    // rows of a half-term box
-        bytes = 16384u + (uint32_t)W.nterms * hr * 128u;
-        if (rank == 0) tc::mbar_expect_tx(bar, 2u * NP * bytes);
-        const int z = W.key;
-        ldA(0, CK * kit, (2 * W.mt + (int)rank) * 128, z);
-        for (int i = 0; i < W.nterms; ++i) {
-            const int hb = (int)rank * W.nterms + i;
-            const Term T = term_of(P, P.entries[W.e0 + (hb >> 1)]);
-            ldB(i * hr * 128, CK * kit, (hb & 1) * hr, T.x * P.v + T.y);
-        }
-        return NP * bytes;
+        const int hb = (int)rank * W.nterms + lane;
+        const int xy = __shfl_sync(0xffffffffu, mine.p0, (hb >> 1) & 31);
+        if (rank == 0 && lane == 0) tc::mbar_expect_tx(bar, 2u * NP * (16384u + (uint32_t)W.nterms * hr * 128u));
+        __syncwarp();
+        if (lane == 31) ldA(0, CK * kit, (2 * W.mt + (int)rank) * 128, W.key);
+        if (lane < W.nterms) ldB(lane * hr * 128, CK * kit, (hb & 1) * hr, xy);
+        return;
     }
+    // a box shared by the item goes through the last lanes when the term lanes
+    // leave them free (nterms <= 32: nocc 8 fills all of them)
     switch (KIND) {
-    case TK_F1: {
-        constexpr int NT = paired(TK_F1, PREC) ? 2 : 1;   // M-tiles per item
-        bytes = NT * 16384u + (uint32_t)W.nterms * o * 128u;
-        tc::mbar_expect_tx(bar, NP * bytes);
-        const int z = W.key;
-        for (int u = 0; u < NT; ++u) ldA(u * 16384u, CK * kit, (NT * W.mt + u) * 128, z);
-        for (int t = 0; t < W.nterms; ++t) {
-            const Term T = term_of(P, P.entries[W.e0 + t]);
-            ldB(t * o * 128, CK * kit, 0, T.x * P.v + T.y);
-        }
-        break;
-    }
+    case TK_F1:
     case TK_VB: {
-        constexpr int NT = paired(TK_VB, PREC) ? 2 : 1;
-        bytes = NT * 16384u + (uint32_t)W.nterms * o * 128u;
-        tc::mbar_expect_tx(bar, NP * bytes);
-        for (int u = 0; u < NT; ++u) ldA(u * 16384u, CK * kit, (NT * W.mt + u) * 128, W.key);
-        for (int t = 0; t < W.nterms; ++t) {
-            const Term T = term_of(P, P.entries[W.e0 + t]);
-            ldB(t * o * 128, CK * kit, 0, wsl<PREC>(T));
+        constexpr int NT = paired(KIND, PREC) ? 2 : 1;   // M-tiles per item
+        arm(NT * 16384u + (uint32_t)W.nterms * o * 128u);
+        if (lane >= 32 - NT) {
+            const int u = lane - (32 - NT);
+            ldA(u * 16384u, CK * kit, (NT * W.mt + u) * 128, W.key);
         }
+        if (lane < W.nterms) ldB(lane * o * 128, CK * kit, 0, mine.p0);
         break;
     }
     case TK_TB: {
         const int kp = PREC ? (o + 15) / 16 * 16 : o;   // K rows (p) of one term, zero-filled past o
+        constexpr int nca = 128 / CK;
         const int nch = W.N / CK;
-        bytes = (uint32_t)(128 / CK + nch) * kp * 128u;
-        tc::mbar_expect_tx(bar, NP * bytes);
-        const Term T = term_of(P, P.entries[W.e0 + kit]);
-        for (int c = 0; c < 128 / CK; ++c) ldA(c * kp * 128, W.mt * 128 + CK * c, 0, T.x * P.v + T.y);
-        for (int c = 0; c < nch; ++c) ldB(c * kp * 128, W.nt * 256 + CK * c, 0, wsl<PREC>(T));
+        arm((uint32_t)(nca + nch) * kp * 128u);
+        if (lane < nca) ldA(lane * kp * 128, W.mt * 128 + CK * lane, 0, mine.p0);
+        else if (lane < nca + nch) ldB((lane - nca) * kp * 128, W.nt * P.tb_n + CK * (lane - nca), 0, mine.p1);
         break;
     }
     case TK_F2: {
         const int nch = P.ock / CK;
-        bytes = 16384u + (uint32_t)W.nterms * nch * chunk;
-        tc::mbar_expect_tx(bar, NP * bytes);
-        ldA(0, CK * kit, W.mt * 128, W.key);
-        for (int t = 0; t < W.nterms; ++t) {
-            const Term T = term_of(P, P.entries[W.e0 + t]);
-            for (int c = 0; c < nch; ++c) ldB((t * nch + c) * chunk, CK * c, CK * kit, T.z * P.v + T.y);
-        }
+        arm(16384u + (uint32_t)W.nterms * nch * chunk);
+        if (lane == 31) ldA(0, CK * kit, W.mt * 128, W.key);
+        if (lane < W.nterms)
+            for (int c = 0; c < nch; ++c) ldB((lane * nch + c) * chunk, CK * c, CK * kit, mine.p0);
         break;
     }
     case TK_OB1: {
@@ -261,13 +277,10 @@ __device__ __forceinline__ uint32_t issue_loads(const TcParams &P, const Work &W
         // positions, rows past o zero-filled); B = t2T rows l, K-major, one
         // box per CK of r
         const int kr8 = PREC ? (o + 15) / 16 * 16 : (o + 7) / 8 * 8, nkc = (kr8 + CK - 1) / CK;
-        bytes = (uint32_t)(128 / CK) * kr8 * 128u + (uint32_t)nkc * o * 128u;
-        tc::mbar_expect_tx(bar, NP * bytes);
-        const int eid = P.entries[W.e0 + kit];
-        const Term T = term_of(P, eid);
-        const int rs = wsl_rot<PREC>(eid);
-        for (int c = 0; c < 128 / CK; ++c) ldA(c * kr8 * 128u, W.mt * 128 + CK * c, 0, rs);
-        for (int kc = 0; kc < nkc; ++kc) ldB(kc * o * 128u, CK * kc, 0, T.z * P.v + T.y);
+        constexpr int nca = 128 / CK;
+        arm((uint32_t)nca * kr8 * 128u + (uint32_t)nkc * o * 128u);
+        if (lane < nca) ldA(lane * kr8 * 128u, W.mt * 128 + CK * lane, 0, mine.p1);
+        else if (lane < nca + nkc) ldB((lane - nca) * o * 128u, CK * (lane - nca), 0, mine.p0);
         break;
     }
     default: {  // TK_OB2
@@ -279,17 +292,16 @@ __device__ __forceinline__ uint32_t issue_loads(const TcParams &P, const Work &W
         const int PK = CK / 8, pk = kit / P.nb, Q = kit - pk * P.nb;
         const int p0 = PK * pk;
         const int koff = (p0 >> 3) * 8 * o + Q * 64 + (p0 & 7) * 8;
-        bytes = (uint32_t)nch * chunk + (uint32_t)W.nterms * o * 128u;
-        tc::mbar_expect_tx(bar, NP * bytes);
-        for (int c = 0; c < nch; ++c) {
+        arm((uint32_t)nch * chunk + (uint32_t)W.nterms * o * 128u);
+        if (lane >= 32 - nch) {
+            const int c = lane - (32 - nch);
             tc::tma_load_4d(sA + c * chunk, &P.mapA, bar, CK * c, 0, Q, W.key * o + p0);
             if (PREC) tc::tma_load_4d(sA + P.a_bytes + c * chunk, &P.mapA2, bar, CK * c, 0, Q, W.key * o + p0);
         }
-        for (int t = 0; t < W.nterms; ++t) ldB(t * o * 128, koff, 0, wsl_rot<PREC>(P.entries[W.e0 + t]));
+        if (lane < W.nterms) ldB(lane * o * 128, koff, 0, mine.p0);
         break;
     }
     }
-    return NP * bytes;
 }
 
 // MMAs of one stage.  TF32: K = 8 per instruction, MN-major operands in the
@@ -466,7 +478,7 @@ __device__ __forceinline__ void epilogue(const TcParams &P, const Work &W, uint3
             for (int j = 0; j < 16; ++j) ebuf[lane * 17 + j] = vals[j];
             __syncwarp();
             // column = qr-tiled pair index; t2T-bar is in the plain (q, r) order
-            const int qt = W.nt * 256 + c0 + (lane & 15);
+            const int qt = W.nt * P.tb_n + c0 + (lane & 15);
             const int Qb = (int)__umulhi((unsigned)qt, P.o_magic) >> 3;   // qt / (8 o)
             const int rem = qt - Qb * 8 * o;
             const int qr = (8 * Qb + ((rem >> 3) & 7)) * o + 8 * (rem >> 6) + (rem & 7);
@@ -630,27 +642,62 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
     int *err = P.err;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int it = 0;
-            bool ok = true;
-            for (int w = cid; w < P.nwork && ok; w += ncl) {
-                Work W;
-                decode<KIND, PREC>(P, w, W);
-                for (int kit = 0; kit < W.nk; ++kit, ++it) {
-                    const int s = it % S;
-                    if (it >= S && !tc::mbar_wait(bar(kBarEmpty + s), ((it / S) - 1) & 1, err)) { ok = false; break; }
-                    const uint32_t sA = sbase + s * P.stage_bytes;
-                    issue_loads<KIND, PREC, CG2>(P, W, kit, sA, bar(s), rank, CG2 ? tc::mapa(bar(s), 0) : 0u);
+        // The descriptors of the coming items are fetched ahead, each load one
+        // item before the one that depends on it: groups of item i + 3, entries
+        // of i + 2, jobs of i + 1 are requested while item i's loads are issued
+        // (a chain of three dependent loads at each item, or two at each stage
+        // of TB and OB1, left the tensor pipe waiting on this warp: at nocc=48/
+        // nvir=300 TF32, F1 112 -> 97 ms, VB 110 -> 92, TB 100 -> 86, OB1 55 -> 42,
+        // OB2 52 -> 38 ms of a step; at nocc=16/nvir=72 TB 11.6 -> 7.3 ms).
+        constexpr bool PER_STAGE = KIND == TK_TB || KIND == TK_OB1;   // one term per stage
+        auto get_work = [&](int w) {
+            Work W{};
+            if (w < P.nwork) decode<KIND, PREC>(P, w, W);
+            return W;
+        };
+        auto get_entry = [&](const Work &W, int first) {
+            return first + lane < W.nterms ? P.entries[W.e0 + first + lane] : 0;
+        };
+        Work W = get_work(cid), W1 = get_work(cid + ncl), W2 = get_work(cid + 2 * ncl);
+        int eid = get_entry(W, 0), eid1 = get_entry(W1, 0);
+        int job = P.jobs[eid / 6];
+        int it = 0;
+        bool ok = true;
+        for (int w = cid; w < P.nwork && ok; w += ncl) {
+            const Work W3 = get_work(w + 3 * ncl);
+            const int eid2 = get_entry(W2, 0), job1 = P.jobs[eid1 / 6];
+            TermOps mine = term_ops<KIND, PREC>(P, eid, job);
+            int eidb = 0, jobb = 0;   // TB, OB1: the next 32 terms of this item
+            for (int kit = 0; kit < W.nk; ++kit, ++it) {
+                if (PER_STAGE) {
+                    const int u = kit & 31;
+                    if (kit > 0 && u == 0) mine = term_ops<KIND, PREC>(P, eidb, jobb);
+                    if (u == 0) eidb = get_entry(W, kit + 32);
+                    if (u == 16) jobb = P.jobs[eidb / 6];
                 }
+                const int s = it % S;
+                if (it >= S && !tc::mbar_wait(bar(kBarEmpty + s), ((it / S) - 1) & 1, err)) ok = false;
+                if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+                TermOps T = mine;
+                if (PER_STAGE) {
+                    T.p0 = __shfl_sync(0xffffffffu, mine.p0, kit & 31);
+                    T.p1 = __shfl_sync(0xffffffffu, mine.p1, kit & 31);
+                }
+                issue_loads<KIND, PREC, CG2>(P, W, kit, sbase + s * P.stage_bytes, bar(s), T, lane, rank,
+                                             CG2 ? tc::mapa(bar(s), 0) : 0u);
             }
-            // drain: every issued copy has landed before this CTA can exit (on
-            // a CTA pair the leader's full barriers count the copies of both)
-            if (rank == 0) {
-                const int issued = it;
-                for (int k = issued - 1; k >= 0 && k >= issued - S; --k)
-                    tc::mbar_wait(bar(k % S), (k / S) & 1, err);
-            }
+            W = W1; W1 = W2; W2 = W3;
+            eid = eid1; eid1 = eid2;
+            job = job1;
         }
+        // drain: every issued copy has landed before this CTA can exit (on
+        // a CTA pair the leader's full barriers count the copies of both)
+        if (rank == 0 && lane == 0) {
+            const int issued = it;
+            for (int k = issued - 1; k >= 0 && k >= issued - S; --k)
+                tc::mbar_wait(bar(k % S), (k / S) & 1, err);
+        }
+        __syncwarp();
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
             int it = 0, wi = 0;
@@ -1096,12 +1143,12 @@ static int launch_tc(TcParams &P, cudaStream_t st) {
     return cudaGetLastError() == cudaSuccess ? CT_OK : CT_ERR_CUDA;
 }
 
-// CTA pairs for F1: off by default (CTB_CTA_PAIRS=1 selects them).  Measured
-// on the nocc=48/nvir=500 benchmark block, F1 took 466 ms per step on CTA
-// pairs against 374 ms with paired M-tiles in one CTA (same box): the pairs
-// overlap F1's G stores with the next item's MMAs, but each SM then carries
-// half the work per stage with its own loads and the cross-SM barriers, and
-// that costs more than the store phase it hides.
+// CTA pairs for F1: off by default (CTB_CTA_PAIRS=1 selects them).  They bring
+// the same operand bytes per MMA to each SM as two M-tiles in one CTA and
+// overlap F1's G stores with the next item's MMAs, but both forms are held by
+// L2 -> shared-memory traffic plus those stores: 96.4 against 97.0 ms for F1 of
+// a nocc=48/nvir=300 block of 82,000 jobs, 38.5 against 40.5 ms (BF16x3, nocc=32/
+// nvir=100).
 static bool cta_pairs_enabled() {
     static const bool on = [] {
         const char *e = std::getenv("CTB_CTA_PAIRS");
@@ -1274,11 +1321,14 @@ static int mixed_wave_p(const WaveView &w, const EpiArgs &e, const ct_grads *g, 
                 return CT_ERR_CUDA;
             if (!make_maps(&P.mapB, &P.mapB2, Wb, o2, o, wn, o2, ws, CK, kp, true, PREC)) return CT_ERR_CUDA;
             P.m_tiles = (v + 127) / 128;
-            P.n_tiles = (int)((o2 + 255) / 256);
+            // items of 256 columns; of 128 where those would leave SMs without one
+            // (few virtuals and a small o^2): the same sums per element either way
+            P.tb_n = w.n_tb_groups * P.m_tiles * (int)((o2 + 255) / 256) < md().sms ? 128 : 256;
+            P.n_tiles = (int)((o2 + P.tb_n - 1) / P.tb_n);
             P.groups = w.tb_groups; P.entries = w.tb_entries;
             P.nwork = w.n_tb_groups * P.m_tiles * P.n_tiles;
             P.out = g->t2T;
-            set_stages(P, (128 / CK) * kp * 128, (256 / CK) * kp * 128, PREC, TK_TB);
+            set_stages(P, (128 / CK) * kp * 128, (P.tb_n / CK) * kp * 128, PREC, TK_TB);
             if (prof) prof(PK_MTB, 0, pctx);
             if ((rc = launch_tc<TK_TB, PREC>(P, st)) != CT_OK) return rc;
             if (prof) prof(PK_MTB, 1, pctx);
