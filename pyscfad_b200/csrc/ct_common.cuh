@@ -89,6 +89,11 @@ __device__ __forceinline__ void cp_async8(void *smem_dst, const void *src, bool 
     const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
 }
+// 16-byte form; both addresses 16-byte aligned
+__device__ __forceinline__ void cp_async16z(void *smem_dst, const void *src, bool ok) {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
 #endif
 
 }  // namespace ctb

@@ -11,8 +11,8 @@
 //       added into the cube W through each term's index permutation
 //   F2  for each x: D[(h,r), pq] = sum_l t2T[z_h,y_h,l,r] vooo[x,pq,l], subtracted
 //   EPI element orbits from the cube: V, r3, energy, mo_energy bars; ybar
-//       replaces W in place, w-bar (ONE cube: the six W-bar_sigma are its index
-//       permutations) goes to the job's scratch cube
+//       replaces W in place, w-bar (one cube: the six W-bar_sigma are its index
+//       permutations) goes to the job's scratch
 //   VT  V-term bars from the ybar cube; then w-bar is read back in its place
 //   VB  vvop_bar[x_h,y_h,p,o+f] += sum_qr Wbar_h[p,qr] t2T[z,f,qr]   (2o x v x o^2)
 //   OB2 t2T_bar[z_h,y_h,l,r] -= sum_pq Wbar_h[pq,r] vooo[x,pq,l]
@@ -43,13 +43,16 @@ struct Args {
     int sj, si;           // padded strides of the shared cube (k has stride 1)
     int cube_sz, stage_sz, tmp_sz;   // doubles
     int passes;           // column passes of F1/F2
-    int vb_groups, vb_ks; // VB: column groups of 8 kVbNT virtuals, K splits
+    int kc, nch;          // K chunk of F1's staged operand (a multiple of 16) and their count
+    int vb_groups, vb_ks; // VB: column groups of 8 VbNT virtuals, K splits
     int ob2_ks;
     unsigned magic;       // ceil(2^32 / o)
 };
 
-constexpr int kKC = 48, kAS = kKC + 4;   // staged K chunk and its row stride (4 mod 16: conflict-free fragments)
-constexpr int kVbNT = 2;
+constexpr int VbNT = 2;   // 8-column tiles a warp takes per VB unit
+// a staged row is the K chunk + 4 (4 mod 16 doubles: conflict-free fragments);
+// a V-term tile row has an odd stride (its column reads walk all banks)
+__host__ __device__ constexpr int tile_ld(int o) { return o | 1; }
 
 // terms by shared index: F1/VB pair the terms with z = c, b, a; F2/OB the terms with x = a, b, c
 __host__ __device__ constexpr int term_z(int i, int h) { return (0x534120 >> (4 * (2 * i + h))) & 15; }
@@ -68,6 +71,17 @@ __device__ __forceinline__ int rtR(int s, int m) {
     return (int)((P >> (6 * s + 2 * m)) & 3);
 }
 
+// Neumaier pairs and a plain partial summed down a warp in a fixed order; valid in lane 0
+__device__ __forceinline__ void ksum_tree(KSum &k, double &v) {
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) {
+        const double s2 = __shfl_down_sync(0xffffffffu, k.s, m), c2 = __shfl_down_sync(0xffffffffu, k.c, m);
+        v += __shfl_down_sync(0xffffffffu, v, m);
+        k.c += c2;
+        k.add(s2);
+    }
+}
+
 template <int MT, int NT, int MODE, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
     extern __shared__ __align__(16) double sm[];
@@ -77,29 +91,34 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
     const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nthr >> 5;
     const int g = lane >> 2, c4 = lane & 3;
     const int sj = A.sj, si = A.si;
+    constexpr int HR = 4 * MT;   // F1/F2 rows of a term (o <= HR)
+    // k-steps of B requested ahead: one is enough with two CTAs per SM (two spill;
+    // nocc=16/nvir=120 energy 84 against 89 ms), two with one (31.5 against 33.0 ms)
+    constexpr int PF = MT == 6 ? 2 : 1;
     double *W = sm;                          // the cube, (i, j, k) at i si + j sj + k
     double *St = W + A.cube_sz;              // GEMM staging, later the V-term tiles
     double *Tm = St + A.stage_sz;            // per-orbit partials / reductions
     double *U = Tm + A.tmp_sz;               // t1T rows a, b, c
     double *F = U + 3 * o;                   // fvo rows a, b, c
     double *eocc = F + 3 * o;
-    double *VA = St, *VB = St + 6 * oo;      // vvop[x,y,:,:o] and t2T[y,x] tiles of the six terms
+    const int tl = tile_ld(o), tsz = o * tl;
+    double *VA = St, *VB = St + 6 * tsz;     // vvop[x,y,:,:o] and t2T[y,x] tiles of the six terms
     __shared__ double wred[3][MAXT / 32];
 
-    int a, b, c;
-    unpack_job(A.jobs[blockIdx.x], a, b, c);
+    int a, jb, c;
+    unpack_job(A.jobs[blockIdx.x], a, jb, c);
     double *Sj = A.cubes + (long long)blockIdx.x * A.stride;
     auto S = [&](int m) { return m == 0 ? si : (m == 1 ? sj : 1); };
     auto divo = [&](int x) { return (int)__umulhi((unsigned)x, A.magic); };
     auto xyz = [&](int s, int &x, int &y, int &z) {
-        x = pick(rtR(s, 0), a, b, c);
-        y = pick(rtR(s, 1), a, b, c);
-        z = pick(rtR(s, 2), a, b, c);
+        x = pick(rtR(s, 0), a, jb, c);
+        y = pick(rtR(s, 1), a, jb, c);
+        z = pick(rtR(s, 2), a, jb, c);
     };
 
     int fnz = 0;
     for (int i = tid; i < 3 * o; i += nthr) {
-        const int w = divo(i), r = i - w * o, z = pick(w, a, b, c);
+        const int w = divo(i), r = i - w * o, z = pick(w, a, jb, c);
         U[i] = e.t1T[z * o + r];
         const double f = e.fvo[z * o + r];
         F[i] = f;
@@ -117,87 +136,97 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
             for (int i = tid; i < A.cube_sz; i += nthr) W[i] = 0.0;
         // ---- F1 (phases 0-2) and F2 (3-5): iterations (phase, pass, K chunk),
         // the A operand of the next iteration copied while this one runs
-        const int nch = (v + kKC - 1) / kKC, per = A.passes * nch, n_it = 3 * per + 3 * A.passes;
-        auto locate = [&](int it, int &ph, int &pass, int &ch) {
-            if (it < 3 * per) {
-                ph = it / per;
-                const int q = it - ph * per;
-                pass = q / nch;
-                ch = q - pass * nch;
-            } else {
-                ph = (it - 3 * per) / A.passes;
-                pass = it - 3 * per - ph * A.passes;
-                ph += 3;
+        const int nch = A.nch, KC = A.kc, AS = KC + 4, per = A.passes * nch, n_it = 3 * per + 3 * A.passes;
+        // position of an iteration, stepped rather than divided out
+        struct Pos {
+            int ph = 0, pass = 0, ch = 0;
+            __device__ __forceinline__ void next(int passes, int nch) {
+                if (ph < 3 && ch + 1 < nch) { ++ch; return; }
                 ch = 0;
+                if (++pass == passes) { pass = 0; ++ph; }
             }
         };
-        auto stage = [&](int it) {
-            int ph, pass, ch;
-            locate(it, ph, pass, ch);
-            double *dst = St + (it & 1) * (8 * MT * kAS);
-            if (ph < 3) {
-                const int k0 = ch * kKC, kw = min(kKC, (v - k0 + 3) & ~3);
+        auto stage = [&](const Pos &q, int buf) {
+            double *dst = St + buf * (8 * MT * AS);
+            if (q.ph < 3) {
+                const int k0 = q.ch * KC, kw = min(KC, (v - k0 + 3) & ~3);
                 int x0, y0, z0, x1, y1, z1;
-                xyz(term_z(ph, 0), x0, y0, z0);
-                xyz(term_z(ph, 1), x1, y1, z1);
+                xyz(term_z(q.ph, 0), x0, y0, z0);
+                xyz(term_z(q.ph, 1), x1, y1, z1);
                 const double *r0 = e.vvop + ((long long)x0 * v + y0) * o * n + o + k0;
                 const double *r1 = e.vvop + ((long long)x1 * v + y1) * o * n + o + k0;
                 for (int m = warp; m < 8 * MT; m += nw) {
-                    const double *src = m < o ? r0 + (long long)m * n : r1 + (long long)(m - o) * n;
+                    const int p = m < HR ? m : m - HR;
+                    const double *src = (m < HR ? r0 : r1) + (long long)p * n;
                     for (int k = lane; k < kw; k += 32) {
-                        const bool ok = m < 2 * o && k0 + k < v;
-                        cp_async8(dst + m * kAS + k, ok ? src + k : e.vvop, ok);
+                        const bool ok = p < o && k0 + k < v;
+                        cp_async8(dst + m * AS + k, src + k, ok);
                     }
                 }
             } else {
                 int x0, y0, z0, x1, y1, z1;
-                xyz(term_x(ph - 3, 0), x0, y0, z0);
-                xyz(term_x(ph - 3, 1), x1, y1, z1);
+                xyz(term_x(q.ph - 3, 0), x0, y0, z0);
+                xyz(term_x(q.ph - 3, 1), x1, y1, z1);
                 const double *r0 = e.t2T + ((long long)z0 * v + y0) * oo, *r1 = e.t2T + ((long long)z1 * v + y1) * oo;
                 const int kw = (o + 3) & ~3;
                 for (int k = warp; k < kw; k += nw)
                     for (int m = lane; m < 8 * MT; m += 32) {
-                        const bool ok = m < 2 * o && k < o;
-                        const double *src = m < o ? r0 + k * o + m : r1 + k * o + m - o;
-                        cp_async8(dst + m * kAS + k, ok ? src : e.t2T, ok);
+                        const int r = m < HR ? m : m - HR;
+                        const bool ok = r < o && k < o;
+                        const double *src = (m < HR ? r0 : r1) + k * o + r;
+                        cp_async8(dst + m * AS + k, src, ok);
                     }
             }
             cp_async_commit();
         };
-        stage(0);
-        double acc[MT][NT][2];
-        for (int it = 0; it < n_it; ++it) {
-            int ph, pass, ch;
-            locate(it, ph, pass, ch);
-            const int n0 = (pass * nw + warp) * (8 * NT);
-            const bool f1 = ph < 3, on = n0 < oo;
-            // B fragments: lane (k = c4, column g) of each 8-column tile
-            const double *bp[NT];
-            long long kst;
-            int K;
-            {
-                int x, y, z;
-                xyz(f1 ? term_z(ph, 0) : term_x(ph - 3, 0), x, y, z);
-                const double *base = f1 ? e.t2T + (long long)z * v * oo + ((long long)ch * kKC + c4) * oo
-                                        : A.vooo + x * o3 + c4;
-                kst = f1 ? 4LL * oo : 4;
-                K = f1 ? min(kKC, v - ch * kKC) : o;
+        // B fragments of an iteration: lane (k = c4, column g) of each 8-column
+        // tile, PF k-steps in flight in registers.  The first ones are requested
+        // as soon as the previous iteration's products are done, under its adds
+        // into the cube.
+        const double *rp = nullptr;
+        int off[NT], full = 0, rem = 0;
+        long long kst = 0;
+        bool on = false;
+        double b[PF][NT], acc[MT][NT][2];
+        auto load_b = [&](int q, double (&d)[NT]) {
+            if (q < full) {
 #pragma unroll
-                for (int t = 0; t < NT; ++t) {
-                    const int col = min(n0 + 8 * t + g, oo - 1);
-                    bp[t] = base + (f1 ? (long long)col : (long long)col * o);
-                }
+                for (int t = 0; t < NT; ++t) d[t] = __ldg(rp + off[t]);
+            } else {
+                const bool in = q == full && c4 < rem;
+#pragma unroll
+                for (int t = 0; t < NT; ++t) d[t] = in ? __ldg(rp + off[t]) : 0.0;
             }
-            const int ks = (K + 3) >> 2;
-            double b0[NT], b1[NT];
+            rp += kst;
+        };
+        auto prep = [&](const Pos &q) {
+            const bool f1 = q.ph < 3;
+            const int n0 = (q.pass * nw + warp) * (8 * NT);
+            on = n0 < oo;
+            const int m = f1 ? 2 - q.ph : q.ph - 3, xz = pick(m, a, jb, c);   // z of F1 phases c, b, a; x of F2 phases
+            rp = f1 ? e.t2T + (long long)xz * v * oo + ((long long)q.ch * KC + c4) * oo : A.vooo + xz * o3 + c4;
+            kst = f1 ? 4LL * oo : 4;
+            const int K = f1 ? min(KC, v - q.ch * KC) : o;
+            full = K >> 2;
+            rem = K & 3;
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                const int col = min(n0 + 8 * t + g, oo - 1);
+                off[t] = f1 ? col : col * o;
+            }
             if (on) {
 #pragma unroll
-                for (int t = 0; t < NT; ++t) {
-                    b0[t] = c4 < K ? __ldg(bp[t]) : 0.0;
-                    b1[t] = c4 + 4 < K ? __ldg(bp[t] + kst) : 0.0;
-                }
+                for (int u = 0; u < PF; ++u) load_b(u, b[u]);
             }
-            if (ch == 0) {
+        };
+        Pos cur, nxt;
+        stage(cur, 0);
+        prep(cur);
+        nxt.next(A.passes, nch);
+        for (int it = 0; it < n_it; ++it, cur = nxt, nxt.next(A.passes, nch)) {
+            const int ph = cur.ph;
+            const bool f1 = ph < 3;
+            if (cur.ch == 0) {
 #pragma unroll
                 for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -205,62 +234,65 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
             }
             cp_async_wait_all();
             __syncthreads();   // this iteration's A operand; the other buffer and the last scatter are done
-            if (it + 1 < n_it) stage(it + 1);
-            if (on) {
-                const double *As = St + (it & 1) * (8 * MT * kAS) + g * kAS + c4;
-                for (int s = 0; s < ks; s += 2) {
-                    double nb0[NT], nb1[NT];
+            if (it + 1 < n_it) stage(nxt, (it + 1) & 1);
+            const bool mine = on;
+            if (mine) {
+                const int ks = full + (rem != 0);
+                const double *As = St + (it & 1) * (8 * MT * AS) + g * AS + c4;
+                for (int s = 0; s < ks; s += PF) {
 #pragma unroll
-                    for (int t = 0; t < NT; ++t) {
-                        nb0[t] = 4 * (s + 2) + c4 < K ? __ldg(bp[t] + (s + 2) * kst) : 0.0;
-                        nb1[t] = 4 * (s + 3) + c4 < K ? __ldg(bp[t] + (s + 3) * kst) : 0.0;
-                    }
+                    for (int u = 0; u < PF; ++u) {
+                        if (s + u < ks) {
 #pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        const double af = As[m * 8 * kAS + 4 * s];
+                            for (int m = 0; m < MT; ++m) {
+                                const double af = As[m * 8 * AS + 4 * (s + u)];
 #pragma unroll
-                        for (int t = 0; t < NT; ++t) dmma(acc[m][t], af, b0[t]);
-                    }
-                    if (s + 1 < ks) {
-#pragma unroll
-                        for (int m = 0; m < MT; ++m) {
-                            const double af = As[m * 8 * kAS + 4 * s + 4];
-#pragma unroll
-                            for (int t = 0; t < NT; ++t) dmma(acc[m][t], af, b1[t]);
+                                for (int t = 0; t < NT; ++t) dmma(acc[m][t], af, b[u][t]);
+                            }
+                            load_b(s + u + PF, b[u]);
                         }
                     }
-#pragma unroll
-                    for (int t = 0; t < NT; ++t) { b0[t] = nb0[t]; b1[t] = nb1[t]; }
                 }
             }
-            if (f1 && ch + 1 < nch) continue;
+            if (it + 1 < n_it) prep(nxt);
+            if (f1 && cur.ch + 1 < nch) continue;
             // add into the cube: the two terms one after the other (they may
-            // meet at the same element), different columns never meet
+            // meet at the same element), different columns never meet.  A
+            // column's loads go out before its stores.  No product runs meanwhile,
+            // so the instructions count: term h's rows are h HR + p with HR = 4 MT
+            // >= o, so only its first (odd MT) and last row tile are predicated,
+            // and columns only in the last group (energy at nocc=16/nvir=120
+            // 112 -> 87 ms against a predicate per element).
+            const int n0 = (cur.pass * nw + warp) * (8 * NT);
+            const double sgn = f1 ? 1.0 : -1.0;
+            const bool tail = n0 + 8 * NT > oo;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int s = f1 ? term_z(ph, h) : term_x(ph - 3, h);
                 // row index p (F1) or r (F2); column (q, r) or (p, q)
                 const int sr = S(rtR(s, f1 ? 0 : 2)), s1 = S(rtR(s, f1 ? 1 : 0)), s2 = S(rtR(s, f1 ? 2 : 1));
-                if (on) {
+                const bool set = fresh && ph == 0 && h == 0;
+                if (mine) {
+                    constexpr int MH = (MT + 1) / 2;           // row tiles of a term
+                    const int m0 = h * (MT / 2);               // its first tile
+                    const int p0 = 8 * m0 + g - h * HR;        // row of the first tile
+                    const bool lo = MT % 2 == 0 || h == 0 || g >= 4, hi = p0 + 8 * (MH - 1) < o;
+                    double *wr = W + p0 * sr;
 #pragma unroll
                     for (int t = 0; t < NT; ++t)
 #pragma unroll
                         for (int q = 0; q < 2; ++q) {
-                            const int col = n0 + 8 * t + 2 * c4 + q;
-                            if (col < oo) {
-                                const int i1 = divo(col), i2 = col - i1 * o;
-                                double *d = W + i1 * s1 + i2 * s2;
+                            const int col = n0 + 8 * t + 2 * c4 + q, i1 = divo(col), i2 = col - i1 * o;
+                            if (tail && col >= oo) continue;
+                            double *d = wr + i1 * s1 + i2 * s2;
+                            double x[MH];
 #pragma unroll
-                                for (int m = 0; m < MT; ++m) {
-                                    const int row = m * 8 + g - h * o;
-                                    if (row >= 0 && row < o) {
-                                        const double x = acc[m][t][q];
-                                        if (fresh && ph == 0 && h == 0) d[row * sr] = x;
-                                        else if (f1) d[row * sr] += x;
-                                        else d[row * sr] -= x;
-                                    }
-                                }
-                            }
+                            for (int m = 0; m < MH; ++m)
+                                x[m] = !set && (m > 0 || lo) && (m < MH - 1 || hi) ? d[m * 8 * sr] : 0.0;
+#pragma unroll
+                            for (int m = 0; m < MH; ++m)
+                                if ((m > 0 || lo) && (m < MH - 1 || hi))
+                                    d[m * 8 * sr] = fma(sgn, acc[h * (MT / 2) + m][t][q], x[m]);
                         }
                 }
                 if (h == 0) __syncthreads();
@@ -279,12 +311,15 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
     }
     {
         constexpr bool need_t2 = MODE == M_VJP || MODE == M_LNO_BWD;
-        for (int i = tid; i < 6 * oo; i += nthr) {
-            const int s = i / oo, pq = i - s * oo, p = divo(pq), q = pq - p * o;
+        for (int s = 0; s < 6; ++s) {
             int x, y, z;
             xyz(s, x, y, z);
-            cp_async8(VA + i, e.vvop + (((long long)x * v + y) * o + p) * n + q, true);
-            if (need_t2 || with_fvo) cp_async8(VB + i, e.t2T + ((long long)y * v + x) * oo + pq, true);
+            const double *sv = e.vvop + ((long long)x * v + y) * o * n, *st = e.t2T + ((long long)y * v + x) * oo;
+            for (int pq = tid; pq < oo; pq += nthr) {
+                const int p = divo(pq), q = pq - p * o, d = s * tsz + p * tl + q;
+                cp_async8(VA + d, sv + p * n + q, true);
+                if (need_t2 || with_fvo) cp_async8(VB + d, st + pq, true);
+            }
         }
         cp_async_commit();
         cp_async_wait_all();
@@ -292,8 +327,8 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
     }
 
     // ---- orbit epilogue (ccsd_t_vjp.c:9-117 per element; lno_ccsd_t.c:6-29)
-    const double fac = job_fac(a, b, c), eb = e.et_bar;
-    const double eabc = e.mo_energy[o + a] + e.mo_energy[o + b] + e.mo_energy[o + c];
+    const double fac = job_fac(a, jb, c), eb = e.et_bar;
+    const double eabc = e.mo_energy[o + a] + e.mo_energy[o + jb] + e.mo_energy[o + c];
     KSum eacc;
     double vir = 0.0;
     for (int t = tid; t < e.n_orb; t += nthr) {
@@ -331,25 +366,36 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
             for (int s = 0; s < 6; ++s) w6[s] = W[pos[s]];
             {
                 // V[s] = sum over terms of A_t[P,Q] u_z(t)[R] at the slot's rearranged position
-                double u[3][3], f[3][3];
+                double u[3][3];
 #pragma unroll
                 for (int w = 0; w < 3; ++w)
 #pragma unroll
-                    for (int m = 0; m < 3; ++m) {
-                        u[w][m] = U[w * o + ijk[m]];
-                        f[w][m] = with_fvo ? F[w * o + ijk[m]] : 0.0;
-                    }
+                    for (int m = 0; m < 3; ++m) u[w][m] = U[w * o + ijk[m]];
 #pragma unroll
                 for (int s = 0; s < 6; ++s) {
                     double vs = 0.0;
 #pragma unroll
                     for (int t6 = 0; t6 < 6; ++t6) {
                         const int cs = kComp(s, t6);
-                        const int vi = t6 * oo + ijk[kR(cs, 0)] * o + ijk[kR(cs, 1)];
-                        vs += VA[vi] * u[kR(t6, 2)][kR(cs, 2)];
-                        if (with_fvo) vs += VB[vi] * f[kR(t6, 2)][kR(cs, 2)];
+                        vs += VA[t6 * tsz + ijk[kR(cs, 0)] * tl + ijk[kR(cs, 1)]] * u[kR(t6, 2)][kR(cs, 2)];
                     }
                     y6[s] = w6[s] + 0.5 * vs;
+                }
+                if (with_fvo) {
+#pragma unroll
+                    for (int w = 0; w < 3; ++w)
+#pragma unroll
+                        for (int m = 0; m < 3; ++m) u[w][m] = F[w * o + ijk[m]];
+#pragma unroll
+                    for (int s = 0; s < 6; ++s) {
+                        double vs = 0.0;
+#pragma unroll
+                        for (int t6 = 0; t6 < 6; ++t6) {
+                            const int cs = kComp(s, t6);
+                            vs += VB[t6 * tsz + ijk[kR(cs, 0)] * tl + ijk[kR(cs, 1)]] * u[kR(t6, 2)][kR(cs, 2)];
+                        }
+                        y6[s] += 0.5 * vs;
+                    }
                 }
             }
             r3_orbit<double>(y6, z6);
@@ -387,34 +433,25 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
     }
     // job energy and the virtual mo_energy bar: a fixed shuffle tree per warp, then over the warps
     {
-        double es = eacc.s, ec = eacc.c, vt = vir;
-        for (int m = 16; m >= 1; m >>= 1) {
-            const double s2 = __shfl_down_sync(0xffffffffu, es, m), c2 = __shfl_down_sync(0xffffffffu, ec, m);
-            vt += __shfl_down_sync(0xffffffffu, vt, m);
-            KSum k;
-            k.s = es;
-            k.c = ec + c2;
-            k.add(s2);
-            es = k.s;
-            ec = k.c;
-        }
-        if (lane == 0) { wred[0][warp] = es; wred[1][warp] = ec; wred[2][warp] = vt; }
+        double vt = vir;
+        ksum_tree(eacc, vt);
+        if (lane == 0) { wred[0][warp] = eacc.s; wred[1][warp] = eacc.c; wred[2][warp] = vt; }
     }
     __syncthreads();   // wred, Tm, the ybar cube and w-bar are complete
-    if (tid == 0) {
+    if (warp == 0) {
         KSum k;
-        double vt = 0.0;
-        for (int w = 0; w < nw; ++w) {
-            k.add(wred[0][w]);
-            k.add(wred[1][w]);
-            vt += wred[2][w];
-        }
-        const long long amaj = (long long)a * (a + 1) * (a + 2) / 6 + (long long)b * (b + 1) / 2 + c;
-        if (MODE == M_ENERGY || MODE == M_VJP) e.job_e[amaj] = 2.0 * k.value();
-        if (MODE == M_VJP || MODE == M_LNO_BWD) {
-            atomicAdd(&e.mo_energy_bar[o + a], vt);
-            atomicAdd(&e.mo_energy_bar[o + b], vt);
-            atomicAdd(&e.mo_energy_bar[o + c], vt);
+        k.s = lane < nw ? wred[0][lane] : 0.0;
+        k.c = lane < nw ? wred[1][lane] : 0.0;
+        double vt = lane < nw ? wred[2][lane] : 0.0;
+        ksum_tree(k, vt);
+        if (lane == 0) {
+            const long long amaj = (long long)a * (a + 1) * (a + 2) / 6 + (long long)jb * (jb + 1) / 2 + c;
+            if (MODE == M_ENERGY || MODE == M_VJP) e.job_e[amaj] = 2.0 * k.value();
+            if (MODE == M_VJP || MODE == M_LNO_BWD) {
+                atomicAdd(&e.mo_energy_bar[o + a], vt);
+                atomicAdd(&e.mo_energy_bar[o + jb], vt);
+                atomicAdd(&e.mo_energy_bar[o + c], vt);
+            }
         }
     }
     if (MODE == M_LNO_FWD) {
@@ -429,17 +466,16 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
     // (i, j, k); lane x collects index x's sum (o <= 32)
     {
         double mine = 0.0;
-        int i = 0, j = 0;
-        for (int pr = 0; pr < o * (o + 1) / 2; ++pr) {
-            if (pr % nw == warp) {
-                const double t = lane <= j ? Tm[i * (i + 1) * (i + 2) / 6 + j * (j + 1) / 2 + lane] : 0.0;
-                double s = t;
+        int i = 0, j = warp;   // pair warp, warp + nw, ... in the order (i, j <= i)
+        for (;;) {
+            while (j > i) { ++i; j -= i; }
+            if (i >= o) break;
+            const double t = lane <= j ? Tm[i * (i + 1) * (i + 2) / 6 + j * (j + 1) / 2 + lane] : 0.0;
+            double s = t;
 #pragma unroll
-                for (int m = 16; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
-                mine += t + (lane == i ? s : 0.0) + (lane == j ? s : 0.0);
-            }
-            if (j < i) ++j;
-            else { ++i; j = 0; }
+            for (int m = 16; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+            mine += t + (lane == i ? s : 0.0) + (lane == j ? s : 0.0);
+            j += nw;
         }
         __syncthreads();   // Tm read by every warp
         Tm[warp * 32 + lane] = mine;
@@ -452,20 +488,28 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
         __syncthreads();
     }
     // ---- VT, pair part: contraction of ybar along r
-    for (int i = tid; i < 6 * oo; i += nthr) {
-        const int s = i / oo, pq = i - s * oo, p = divo(pq), q = pq - p * o;
+    for (int s = 0; s < 6; ++s) {
         int x, y, z;
         xyz(s, x, y, z);
-        const int zr = rtR(s, 2), st = S(zr);
-        const double *yp = W + p * S(rtR(s, 0)) + q * S(rtR(s, 1)), *u = U + zr * o, *f = F + zr * o;
-        double su = 0.0, sw = 0.0;
-        for (int r = 0; r < o; ++r) {
-            const double yv = yp[r * st];
-            su += yv * u[r];
-            sw += yv * f[r];
+        const int zr = rtR(s, 2), st = S(zr), sp = S(rtR(s, 0)), sq = S(rtR(s, 1));
+        const double *u = U + zr * o, *f = F + zr * o;
+        double *dv = e.vvop_bar + ((long long)x * v + y) * o * n, *dt = e.t2T_bar + ((long long)y * v + x) * oo;
+        for (int pq = tid; pq < oo; pq += nthr) {
+            const int p = divo(pq), q = pq - p * o;
+            const double *yp = W + p * sp + q * sq;
+            double su = 0.0, sw = 0.0;
+            if (with_fvo) {
+                for (int r = 0; r < o; ++r) {
+                    const double yv = yp[r * st];
+                    su += yv * u[r];
+                    sw += yv * f[r];
+                }
+                atomicAdd(dt + pq, 0.5 * sw);
+            } else {
+                for (int r = 0; r < o; ++r) su += yp[r * st] * u[r];
+            }
+            atomicAdd(dv + p * n + q, 0.5 * su);
         }
-        atomicAdd(e.vvop_bar + (((long long)x * v + y) * o + p) * n + q, 0.5 * su);
-        if (with_fvo) atomicAdd(e.t2T_bar + ((long long)y * v + x) * oo + pq, 0.5 * sw);
     }
     // ---- VT, r part: contraction of ybar along (p, q), split over the threads
     {
@@ -478,12 +522,12 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
                 for (int h = 0; h < 2; ++h) {
                     const int s = term_z(zi, h);
                     const int s0 = S(kR(s, 0)), s1 = S(kR(s, 1));
-                    const double *yp = W + r * S(kR(s, 2)), *va = VA + s * oo, *vb = VB + s * oo;
+                    const double *yp = W + r * S(kR(s, 2)), *va = VA + s * tsz, *vb = VB + s * tsz;
                     for (int pq = part; pq < oo; pq += parts) {
                         const int p = divo(pq), q = pq - p * o;
                         const double yv = yp[p * s0 + q * s1];
-                        a1 += yv * va[pq];
-                        a2 += yv * vb[pq];
+                        a1 += yv * va[p * tl + q];
+                        a2 += yv * vb[p * tl + q];
                     }
                 }
                 Tm[(zi * 2 * parts + part) * o + r] = a1;
@@ -495,17 +539,56 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
             const int w = divo(i), rr = i - w * o, zi = w >> 1;
             double s = 0.0;
             for (int q = 0; q < parts; ++q) s += Tm[(w * parts + q) * o + rr];
-            const int z = pick(2 - zi, a, b, c);
+            const int z = pick(2 - zi, a, jb, c);
             atomicAdd(((w & 1) ? e.fvo_bar : e.t1T_bar) + z * o + rr, 0.5 * s);
         }
     }
     // ---- w-bar back in the place of ybar (every warp is past its reads: the
-    // barrier above follows them)
+    // barrier above follows them), then its copies with j and with i contiguous,
+    // [i][k][j] and [j][k][i], so that the t2-bar GEMM reads every term along r
     for (int i = tid; i < (int)o3; i += nthr) {
         const int ij = divo(i), k = i - ij * o, ii = divo(ij), j = ij - ii * o;
         W[ii * si + j * sj + k] = Sj[i];
     }
     __syncthreads();
+    for (int i = tid; i < (int)o3; i += nthr) {
+        const int xy = divo(i), z = i - xy * o, x = divo(xy), y = xy - x * o;
+        Sj[o3 + i] = W[x * si + z * sj + y];
+        Sj[2 * o3 + i] = W[z * si + x * sj + y];
+    }
+
+    // A operand of VB and OB2, straight from the cube: row tile m of term h holds
+    // rows h HR + p; the address of (row, k) is its row part plus the k part of its
+    // term, stepped along k (k = 4 ks + c4 is a pair (k1, k2 < o) of the cube's axes)
+    struct KStep {
+        int k2, f0, f1;            // k2 and both terms' k parts
+        int d0, d1, w0, w1;        // steps of 4 along k2, and at a wrap to the next k1
+        __device__ __forceinline__ void init(int k, int k1, int o, int a0, int b0, int a1, int b1) {
+            k2 = k - k1 * o;
+            f0 = k1 * a0 + k2 * b0;
+            f1 = k1 * a1 + k2 * b1;
+            d0 = 4 * b0; d1 = 4 * b1;
+            w0 = a0 - o * b0; w1 = a1 - o * b1;
+        }
+        __device__ __forceinline__ void next(int o) {
+            k2 += 4; f0 += d0; f1 += d1;
+            while (k2 >= o) { k2 -= o; f0 += w0; f1 += w1; }
+        }
+    };
+    const bool second = MT % 2 == 1 && g >= 4;   // this lane's rows of the middle tile are term 1's
+    auto row_parts = [&](int sr0, int sr1, int (&ra)[MT]) {
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            const int row = m * 8 + g, p = row < HR ? row : row - HR;
+            ra[m] = p < o ? p * (row < HR ? sr0 : sr1) : 0;   // rows past o: any element, not stored
+        }
+    };
+    auto load_a = [&](const KStep &K, const int (&ra)[MT], double (&af)[MT]) {
+        const int fm = second ? K.f1 : K.f0;
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+            af[m] = W[ra[m] + (2 * m + 1 < MT ? K.f0 : (2 * m + 1 == MT ? fm : K.f1))];
+    };
 
     // ---- VB: units (z, column group, K split) over the warps
     {
@@ -513,53 +596,54 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
         for (int un = warp; un < units; un += nw) {
             const int zi = un / (A.vb_groups * A.vb_ks), rem = un - zi * (A.vb_groups * A.vb_ks);
             const int gr = rem / A.vb_ks, sp = rem - gr * A.vb_ks;
-            const int ka = k4 * sp / A.vb_ks, kb = k4 * (sp + 1) / A.vb_ks;
+            const int ka = k4 * sp / A.vb_ks, kb = k4 * (sp + 1) / A.vb_ks, kf = min(kb, oo >> 2);
             const int s0 = term_z(zi, 0), s1 = term_z(zi, 1);
-            const int z = pick(2 - zi, a, b, c);
-            const int q0 = S(rtR(s0, 1)), r0 = S(rtR(s0, 2)), q1 = S(rtR(s1, 1)), r1 = S(rtR(s1, 2));
-            const int p0 = S(rtR(s0, 0)), p1 = S(rtR(s1, 0));
+            const int z = pick(2 - zi, a, jb, c);
             int ra[MT];
-            unsigned hs = 0;
+            row_parts(S(rtR(s0, 0)), S(rtR(s1, 0)), ra);
+            KStep K;
+            const int kk = 4 * ka + c4;
+            K.init(kk, divo(kk), o, S(rtR(s0, 1)), S(rtR(s0, 2)), S(rtR(s1, 1)), S(rtR(s1, 2)));
+            const double *bp[VbNT];
 #pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                const int row = m * 8 + g;
-                ra[m] = row < o ? row * p0 : (row < 2 * o ? (row - o) * p1 : 0);
-                if (row >= o) hs |= 1u << m;
-            }
-            const double *bp[kVbNT];
-#pragma unroll
-            for (int t = 0; t < kVbNT; ++t)
-                bp[t] = e.t2T + ((long long)z * v + min(gr * 8 * kVbNT + 8 * t + g, v - 1)) * oo;
-            double acc[MT][kVbNT][2];
+            for (int t = 0; t < VbNT; ++t)
+                bp[t] = e.t2T + ((long long)z * v + min((gr * VbNT + t) * 8 + g, v - 1)) * oo + kk;
+            double acc[MT][VbNT][2];
 #pragma unroll
             for (int m = 0; m < MT; ++m)
 #pragma unroll
-                for (int t = 0; t < kVbNT; ++t) acc[m][t][0] = acc[m][t][1] = 0.0;
-            int kk = 4 * ka + c4;
-            double b0[kVbNT], b1[kVbNT];
+                for (int t = 0; t < VbNT; ++t) acc[m][t][0] = acc[m][t][1] = 0.0;
+            double b[VbNT], af[MT];
+            if (ka < kf)
 #pragma unroll
-            for (int t = 0; t < kVbNT; ++t) {
-                b0[t] = kk < oo ? __ldg(bp[t] + kk) : 0.0;
-                b1[t] = kk + 4 < oo ? __ldg(bp[t] + kk + 4) : 0.0;
-            }
-            int q = divo(min(kk, oo - 1)), r = kk - q * o;
-#pragma unroll 2
-            for (int ks = ka; ks < kb; ++ks, kk += 4) {
-                double nb[kVbNT];
+                for (int t = 0; t < VbNT; ++t) b[t] = __ldg(bp[t]);
+#pragma unroll 4
+            for (int ks = ka; ks < kf; ++ks) {
+                double nb[VbNT];
 #pragma unroll
-                for (int t = 0; t < kVbNT; ++t) nb[t] = kk + 8 < oo ? __ldg(bp[t] + kk + 8) : 0.0;
-                const bool in = kk < oo;
-                const int f0 = in ? q * q0 + r * r0 : 0, f1 = in ? q * q1 + r * r1 : 0;
-#pragma unroll
-                for (int m = 0; m < MT; ++m) {
-                    const double af = in ? W[ra[m] + ((hs >> m & 1) ? f1 : f0)] : 0.0;
-#pragma unroll
-                    for (int t = 0; t < kVbNT; ++t) dmma(acc[m][t], af, b0[t]);
+                for (int t = 0; t < VbNT; ++t) {
+                    bp[t] += 4;
+                    nb[t] = ks + 1 < kf ? __ldg(bp[t]) : 0.0;
                 }
-                r += 4;
-                while (r >= o) { r -= o; ++q; }
+                load_a(K, ra, af);
 #pragma unroll
-                for (int t = 0; t < kVbNT; ++t) { b0[t] = b1[t]; b1[t] = nb[t]; }
+                for (int m = 0; m < MT; ++m)
+#pragma unroll
+                    for (int t = 0; t < VbNT; ++t) dmma(acc[m][t], af[m], b[t]);
+                K.next(o);
+#pragma unroll
+                for (int t = 0; t < VbNT; ++t) b[t] = nb[t];
+            }
+            if (kf < kb) {   // the last k-step, part past o^2
+                const bool in = c4 < (oo & 3);
+                if (!in) K.f0 = K.f1 = 0;
+                load_a(K, ra, af);
+#pragma unroll
+                for (int t = 0; t < VbNT; ++t) b[t] = in ? __ldg(bp[t]) : 0.0;
+#pragma unroll
+                for (int m = 0; m < MT; ++m)
+#pragma unroll
+                    for (int t = 0; t < VbNT; ++t) dmma(acc[m][t], in ? af[m] : 0.0, b[t]);
             }
             int x0, y0, zz, x1, y1;
             xyz(s0, x0, y0, zz);
@@ -568,72 +652,90 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
             double *d1 = e.vvop_bar + ((long long)x1 * v + y1) * o * n + o;
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-                const int row = m * 8 + g;
-                if (row >= 2 * o) continue;
-                double *d = row < o ? d0 + (long long)row * n : d1 + (long long)(row - o) * n;
+                const int row = m * 8 + g, pr = row < HR ? row : row - HR;
+                if (pr >= o) continue;
+                double *d = (row < HR ? d0 : d1) + (long long)pr * n;
 #pragma unroll
-                for (int t = 0; t < kVbNT; ++t)
+                for (int t = 0; t < VbNT; ++t)
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const int f = gr * 8 * kVbNT + 8 * t + 2 * c4 + h;
+                        const int f = (gr * VbNT + t) * 8 + 2 * c4 + h;
                         if (f < v) atomicAdd(d + f, acc[m][t][h]);
                     }
             }
         }
     }
-    // ---- OB2: units (x, 8 columns l, K split): D[(h,r), l] = sum_pq Wbar_h[pq,r] vooo[x,pq,l]
+    // ---- OB2: units (x, 8 N2 columns l, K split): D[(h,r), l] = sum_pq Wbar_h[pq,r] vooo[x,pq,l]
     {
-        const int ln = (o + 7) >> 3, k4 = (oo + 3) >> 2, units = 3 * ln * A.ob2_ks;
+        constexpr int N2 = MT <= 2 ? 1 : 2;
+        const int ln = (o + 8 * N2 - 1) / (8 * N2), k4 = (oo + 3) >> 2, units = 3 * ln * A.ob2_ks;
         for (int un = warp; un < units; un += nw) {
             const int xi = un / (ln * A.ob2_ks), rem = un - xi * (ln * A.ob2_ks);
             const int lt = rem / A.ob2_ks, sp = rem - lt * A.ob2_ks;
-            const int ka = k4 * sp / A.ob2_ks, kb = k4 * (sp + 1) / A.ob2_ks;
+            const int ka = k4 * sp / A.ob2_ks, kb = k4 * (sp + 1) / A.ob2_ks, kf = min(kb, oo >> 2);
             const int s0 = 2 * xi, s1 = 2 * xi + 1;
             int x, y0, z0, x1, y1, z1;
             xyz(s0, x, y0, z0);
             xyz(s1, x1, y1, z1);
-            const int p0 = S(rtR(s0, 0)), q0 = S(rtR(s0, 1)), r0 = S(rtR(s0, 2));
-            const int p1 = S(rtR(s1, 0)), q1 = S(rtR(s1, 1)), r1 = S(rtR(s1, 2));
             int ra[MT];
-            unsigned hs = 0;
+            row_parts(S(rtR(s0, 2)), S(rtR(s1, 2)), ra);
+            KStep K;
+            const int kk = 4 * ka + c4;
+            K.init(kk, divo(kk), o, S(rtR(s0, 0)), S(rtR(s0, 1)), S(rtR(s1, 0)), S(rtR(s1, 1)));
+            const double *bp[N2];
 #pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                const int row = m * 8 + g;
-                ra[m] = row < o ? row * r0 : (row < 2 * o ? (row - o) * r1 : 0);
-                if (row >= o) hs |= 1u << m;
-            }
-            const double *bp = A.vooo + x * o3 + min(lt * 8 + g, o - 1);
-            double acc[MT][2];
+            for (int t = 0; t < N2; ++t)
+                bp[t] = A.vooo + x * o3 + (long long)kk * o + min((lt * N2 + t) * 8 + g, o - 1);
+            double acc[MT][N2][2];
 #pragma unroll
-            for (int m = 0; m < MT; ++m) acc[m][0] = acc[m][1] = 0.0;
-            int kk = 4 * ka + c4;
-            double b0 = kk < oo ? __ldg(bp + (long long)kk * o) : 0.0;
-            double b1 = kk + 4 < oo ? __ldg(bp + (long long)(kk + 4) * o) : 0.0;
-            int p = divo(min(kk, oo - 1)), q = kk - p * o;
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int t = 0; t < N2; ++t) acc[m][t][0] = acc[m][t][1] = 0.0;
+            double b[N2], af[MT];
+            if (ka < kf)
+#pragma unroll
+                for (int t = 0; t < N2; ++t) b[t] = __ldg(bp[t]);
 #pragma unroll 2
-            for (int ks = ka; ks < kb; ++ks, kk += 4) {
-                const double nb = kk + 8 < oo ? __ldg(bp + (long long)(kk + 8) * o) : 0.0;
-                const bool in = kk < oo;
-                const int f0 = in ? p * p0 + q * q0 : 0, f1 = in ? p * p1 + q * q1 : 0;
+            for (int ks = ka; ks < kf; ++ks) {
+                double nb[N2];
+#pragma unroll
+                for (int t = 0; t < N2; ++t) {
+                    bp[t] += 4 * o;
+                    nb[t] = ks + 1 < kf ? __ldg(bp[t]) : 0.0;
+                }
+                load_a(K, ra, af);
 #pragma unroll
                 for (int m = 0; m < MT; ++m)
-                    dmma(acc[m], in ? W[ra[m] + ((hs >> m & 1) ? f1 : f0)] : 0.0, b0);
-                q += 4;
-                while (q >= o) { q -= o; ++p; }
-                b0 = b1;
-                b1 = nb;
+#pragma unroll
+                    for (int t = 0; t < N2; ++t) dmma(acc[m][t], af[m], b[t]);
+                K.next(o);
+#pragma unroll
+                for (int t = 0; t < N2; ++t) b[t] = nb[t];
+            }
+            if (kf < kb) {
+                const bool in = c4 < (oo & 3);
+                if (!in) K.f0 = K.f1 = 0;
+                load_a(K, ra, af);
+#pragma unroll
+                for (int t = 0; t < N2; ++t) b[t] = in ? __ldg(bp[t]) : 0.0;
+#pragma unroll
+                for (int m = 0; m < MT; ++m)
+#pragma unroll
+                    for (int t = 0; t < N2; ++t) dmma(acc[m][t], in ? af[m] : 0.0, b[t]);
             }
             double *d0 = e.t2T_bar + ((long long)z0 * v + y0) * oo, *d1 = e.t2T_bar + ((long long)z1 * v + y1) * oo;
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-                const int row = m * 8 + g;
-                if (row >= 2 * o) continue;
-                double *d = row < o ? d0 + row : d1 + row - o;
+                const int row = m * 8 + g, pr = row < HR ? row : row - HR;
+                if (pr >= o) continue;
+                double *d = (row < HR ? d0 : d1) + pr;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int l = lt * 8 + 2 * c4 + h;
-                    if (l < o) atomicAdd(d + l * o, -acc[m][h]);
-                }
+                for (int t = 0; t < N2; ++t)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int l = (lt * N2 + t) * 8 + 2 * c4 + h;
+                        if (l < o) atomicAdd(d + l * o, -acc[m][t][h]);
+                    }
             }
         }
     }
@@ -643,7 +745,7 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
         const int ng = (oo + 8 * N1 - 1) / (8 * N1), units = 3 * ng;
         for (int un = warp; un < units; un += nw) {
             const int xi = un / ng, n0 = (un - xi * ng) * (8 * N1);
-            const int x = pick(xi, a, b, c);
+            const int x = pick(xi, a, jb, c);
             double acc[ML][N1][2];
 #pragma unroll
             for (int m = 0; m < ML; ++m)
@@ -652,7 +754,7 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int s = term_x(xi, h);
-                const double *T = VB + tile_zy(s) * oo;
+                const double *T = VB + tile_zy(s) * tsz;
                 const int sp = S(rtR(s, 0)), sq = S(rtR(s, 1)), sr = S(rtR(s, 2));
                 int cb[N1];
 #pragma unroll
@@ -669,7 +771,7 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
 #pragma unroll
                     for (int m = 0; m < ML; ++m) {
                         const int l = m * 8 + g;
-                        const double af = in && l < o ? T[l * o + r] : 0.0;
+                        const double af = in && l < o ? T[l * tl + r] : 0.0;
 #pragma unroll
                         for (int t = 0; t < N1; ++t) dmma(acc[m][t], af, bf[t]);
                     }
@@ -697,14 +799,18 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
 // wave's terms with that z.  64 (f) x 64 (qr) tiles, 4 warps of 32 x 32, one
 // stage = `tps` terms of op rows (o rounded up to the MMA's K); the term list
 // is split into `splits` parts per tile so that a wave with few z still fills
-// the GPU (the parts add into t2T_bar).
+// the GPU (the parts add into t2T_bar).  Each job's w-bar comes as three cubes,
+// the contiguous axis that of c, b or a: a term reads the one of its z, where
+// its r runs along memory (from one cube, a third of the terms were gathered
+// along p and a third along q in 8-byte pieces).  Even sizes copy 16 bytes.
 // ---------------------------------------------------------------------------
 struct TbArgs {
     const double *vvop, *cubes;
     double *t2T_bar;
     long long stride;
     int o, v, n, op, tps, splits, tiles_n;
-    unsigned magic, magic_op;
+    int vec_a, vec_b;     // 16-byte copies of the vvop rows / the cubes
+    unsigned magic;
     const int *jobs, *entries, *groups;
 };
 constexpr int kTbLD = 68, kTbTerms = 128;
@@ -725,9 +831,11 @@ __global__ void __launch_bounds__(128, 4) tb_kernel(const TbArgs P) {
     const int e0 = eb + (int)((long long)ne * sp / P.splits), e1 = eb + (int)((long long)ne * (sp + 1) / P.splits);
     const int nt = e1 - e0, nst = (nt + P.tps - 1) / P.tps;
     if (nt <= 0) return;
-    const int ml = tid & 63, kl = tid >> 6;
-    const int col = n0 + ml, cq = (int)__umulhi((unsigned)col, P.magic), cr = col - cq * o;
-    const bool f_ok = f0 + ml < v, c_ok = col < oo;
+    // this thread's column of the A and B copies and its first row (of every 2, or 4)
+    const int ca = P.vec_a ? 2 * (tid & 31) : tid & 63, ra = P.vec_a ? tid >> 5 : tid >> 6, da = P.vec_a ? 4 : 2;
+    const int cb = P.vec_b ? 2 * (tid & 31) : tid & 63, rb = P.vec_b ? tid >> 5 : tid >> 6, db = P.vec_b ? 4 : 2;
+    const int col = n0 + cb, cq = (int)__umulhi((unsigned)col, P.magic), cr = col - cq * o;
+    const bool f_ok = f0 + ca < v, c_ok = col < oo;
     auto load_terms = [&](int base) {
         const int i = base + tid;
         if (tid < kTbTerms && i < nt) {
@@ -738,35 +846,27 @@ __global__ void __launch_bounds__(128, 4) tb_kernel(const TbArgs P) {
             t_js[tid] = jl * 8 + s;
         }
     };
-    auto strd = [&](int m) { return m == 0 ? oo : (m == 1 ? o : 1); };
     auto stage = [&](int st) {
-        double *a_ = As + (st & 1) * buf, *b_ = Bs + (st & 1) * buf;
+        double *a_ = As + (st & 1) * buf + ca, *b_ = Bs + (st & 1) * buf + cb;
         for (int u = 0; u < P.tps; ++u) {
             const int t = st * P.tps + u;
             const bool t_ok = t < nt;
             const int xy = t_ok ? t_xy[t & (kTbTerms - 1)] : 0, js = t_ok ? t_js[t & (kTbTerms - 1)] : 0;
-            const double *src = P.vvop + (long long)xy * o * n + o + f0 + ml;
-            for (int p = kl; p < op; p += 2) {
+            const double *src = P.vvop + (long long)xy * o * n + o + f0 + ca;
+            for (int p = ra; p < op; p += da) {
                 const bool ok = t_ok && f_ok && p < o;
-                cp_async8(a_ + (u * op + p) * kTbLD + ml, ok ? src + (long long)p * n : P.vvop, ok);
+                if (P.vec_a) cp_async16z(a_ + (u * op + p) * kTbLD, src + p * n, ok);
+                else cp_async8(a_ + (u * op + p) * kTbLD, src + p * n, ok);
             }
-            const int s = js & 7;
-            const double *cb = P.cubes + (long long)(js >> 3) * P.stride;
-            const int sp0 = strd(rtR(s, 0)), sq = strd(rtR(s, 1)), sr = strd(rtR(s, 2));
-            if (s < 4) {
-                const double *q = cb + cq * sq + cr * sr;
-                for (int p = kl; p < op; p += 2) {
-                    const bool ok = t_ok && c_ok && p < o;
-                    cp_async8(b_ + (u * op + p) * kTbLD + ml, ok ? q + p * sp0 : P.cubes, ok);
-                }
-            } else {
-                // p is the contiguous index of the cube: consecutive threads along p
-                for (int i = tid; i < op * 64; i += 128) {
-                    const int nn = (int)__umulhi((unsigned)i, P.magic_op), p = i - nn * op;
-                    const int cl = n0 + nn, q = (int)__umulhi((unsigned)cl, P.magic), r = cl - q * o;
-                    const bool ok = t_ok && cl < oo && p < o;
-                    cp_async8(b_ + (u * op + p) * kTbLD + nn, ok ? cb + p + q * sq + r * sr : P.cubes, ok);
-                }
+            // cube of the term's z (0, 1, 0, 2, 1, 2) and which of its outer axes is p
+            const int s = js & 7, cube = (0x212010 >> (4 * s)) & 3;
+            const bool first = s != 2 && s < 4;
+            const int sp0 = first ? oo : o, sq = first ? o : oo;
+            const double *q = P.cubes + (long long)(js >> 3) * P.stride + (long long)cube * oo * o + cq * sq + cr;
+            for (int p = rb; p < op; p += db) {
+                const bool ok = t_ok && c_ok && p < o;
+                if (P.vec_b) cp_async16z(b_ + (u * op + p) * kTbLD, q + p * sp0, ok);
+                else cp_async8(b_ + (u * op + p) * kTbLD, q + p * sp0, ok);
             }
         }
         cp_async_commit();
@@ -791,10 +891,10 @@ __global__ void __launch_bounds__(128, 4) tb_kernel(const TbArgs P) {
             stage(st + 1);
         }
         const double *a_ = As + (st & 1) * buf + wm + g + c4 * kTbLD, *b_ = Bs + (st & 1) * buf + wn + g + c4 * kTbLD;
-        for (int k = 0; k < rows; k += 4) {
+        for (int k = 0; k < rows; k += 4, a_ += 4 * kTbLD, b_ += 4 * kTbLD) {
             double af[4], bf[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { af[i] = a_[k * kTbLD + 8 * i]; bf[i] = b_[k * kTbLD + 8 * i]; }
+            for (int i = 0; i < 4; ++i) { af[i] = a_[8 * i]; bf[i] = b_[8 * i]; }
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -846,22 +946,31 @@ static cudaError_t launch(Args &A, int n_jobs, cudaStream_t st) {
     const int nw = (groups + A.passes - 1) / A.passes;
     pick_strides(o, A.sj, A.si);
     A.cube_sz = (o * A.si + 1) & ~1;
-    A.stage_sz = std::max(2 * 8 * MT * kAS, 12 * oo);
+    const int tiles_sz = 12 * o * tile_ld(o);
     A.tmp_sz = (MODE == M_VJP || MODE == M_LNO_BWD) ? std::max(A.e.n_orb, 6 * nw * 32) : 0;
+    // the longest K chunk that still lets MINB CTAs share the SM (fewer, longer
+    // chunks: fewer barriers), split evenly over the virtuals
+    const int room = (228 * 1024 / MINB - 2048) / 8 - A.cube_sz - A.tmp_sz - 7 * o;
+    const int cap = std::max(32, std::min(128, (room / (2 * 8 * MT) - 4) / 16 * 16));
+    A.nch = (A.e.v + cap - 1) / cap;
+    A.kc = std::max(32, ((A.e.v + A.nch - 1) / A.nch + 15) / 16 * 16);
+    A.stage_sz = std::max(2 * 8 * MT * (A.kc + 4), tiles_sz);
     A.magic = (unsigned)(((1ull << 32) + o - 1) / o);
-    A.vb_groups = (A.e.v + 8 * kVbNT - 1) / (8 * kVbNT);
-    // K splits: enough units that the last round of warps is mostly full
+    A.vb_groups = (A.e.v + 8 * VbNT - 1) / (8 * VbNT);
+    // K splits: units to fill the rounds of warps to 70% (shorter units pay more
+    // for their start and their atomics than a fuller last round gains)
     auto splits = [&](int units, int kmax) {
         int ks = 1;
         while (ks < 8 && 2 * ks <= kmax) {
             const int u = units * ks, rounds = (u + nw - 1) / nw;
-            if (u * 10 >= rounds * nw * 9) break;
+            if (u * 10 >= rounds * nw * 7) break;
             ks *= 2;
         }
         return ks;
     };
     A.vb_ks = splits(3 * A.vb_groups, oo / 32);
-    A.ob2_ks = splits(3 * ((o + 7) / 8), oo / 32);
+    constexpr int N2 = MT <= 2 ? 1 : 2;   // job_kernel's OB2 tile
+    A.ob2_ks = splits(3 * ((o + 8 * N2 - 1) / (8 * N2)), oo / 32);
     const size_t smem = sizeof(double) * (size_t)(A.cube_sz + A.stage_sz + A.tmp_sz + 7 * o);
     const void *fn = reinterpret_cast<const void *>(job_kernel<MT, NT, MODE, MAXT, MINB>);
     cudaError_t ce = smem_optin(fn, (int)smem);
@@ -873,11 +982,13 @@ static cudaError_t launch(Args &A, int n_jobs, cudaStream_t st) {
 template <int MODE>
 static cudaError_t launch_o(Args &A, int n_jobs, cudaStream_t st) {
     switch ((A.e.o + 3) / 4) {   // tiles of 8 over the 2 o rows
-    case 1: return launch<1, 2, MODE, 256, 2>(A, n_jobs, st);
-    case 2: return launch<2, 2, MODE, 256, 2>(A, n_jobs, st);
-    case 3: return launch<3, 3, MODE, 256, 2>(A, n_jobs, st);
+    case 1: return launch<1, 2, MODE, 32, 16>(A, n_jobs, st);
+    case 2: return launch<2, 2, MODE, 128, 5>(A, n_jobs, st);
+    case 3: return launch<3, 3, MODE, 192, 3>(A, n_jobs, st);
     case 4: return launch<4, 4, MODE, 256, 2>(A, n_jobs, st);
-    case 5: return launch<5, 3, MODE, 256, 2>(A, n_jobs, st);
+    // nocc = 20 with the gradients' partials leaves room for one CTA per SM
+    case 5: return A.e.o == 20 && MODE != M_ENERGY ? launch<5, 2, MODE, 512, 1>(A, n_jobs, st)
+                                                   : launch<5, 3, MODE, 256, 2>(A, n_jobs, st);
     case 6: return launch<6, 3, MODE, 512, 1>(A, n_jobs, st);
     default: return cudaErrorInvalidValue;
     }
@@ -906,7 +1017,7 @@ cudaError_t cube_energy(const int *jobs, int n_jobs, const EpiArgs &e, const dou
 cudaError_t cube_vjp(const WaveView &w, const EpiArgs &e, const double *vooo, double *vooo_bar, double *cubes,
                      cudaStream_t st) {
     if (w.n_jobs <= 0) return cudaSuccess;
-    cube::Args A = cube::make_args(w.jobs, e, vooo, vooo_bar, cubes, (long long)e.o * e.o * e.o);
+    cube::Args A = cube::make_args(w.jobs, e, vooo, vooo_bar, cubes, 3LL * e.o * e.o * e.o);
     return cube::launch_o<cube::M_VJP>(A, w.n_jobs, st);
 }
 
@@ -938,7 +1049,8 @@ cudaError_t cube_tb(const WaveView &w, const EpiArgs &e, const double *cubes, lo
     if (P.tps == 3) P.tps = 2;   // a power of two divides the descriptor block
     P.tiles_n = (e.o * e.o + 63) / 64;
     P.magic = (unsigned)(((1ull << 32) + e.o - 1) / e.o);
-    P.magic_op = (unsigned)(((1ull << 32) + P.op - 1) / P.op);
+    P.vec_a = e.o % 2 == 0 && e.n % 2 == 0 && reinterpret_cast<uintptr_t>(e.vvop) % 16 == 0;
+    P.vec_b = e.o % 2 == 0 && stride % 2 == 0 && reinterpret_cast<uintptr_t>(cubes) % 16 == 0;
     P.jobs = w.jobs;
     P.entries = w.tb_entries;
     P.groups = w.tb_groups;

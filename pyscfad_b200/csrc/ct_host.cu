@@ -509,13 +509,13 @@ static bool use_cube(int o, int mode) { return mode == CT_MODE_FP64 && o >= 2 &&
 
 // Jobs per wave: as many as the scratch budget holds (at most 8192), rounded
 // down to a multiple of two CTAs per SM so the per-job kernels fill whole
-// rounds of the GPU.  On the cube path a wave's w-bar cubes (o^3 doubles a
-// job) also stay below 96 MB, so that the t2-bar GEMM finds them in L2.
+// rounds of the GPU.  (On the cube path waves whose w-bar cubes stay
+// in L2 were tried: shorter term lists per t2-bar tile cost more than the DRAM
+// round trip saves, 48.8 against 38.6 ms at nocc=16/nvir=100 with 888 and 5328 jobs.)
 static int max_wave_jobs(Workspace &W, int o, int mode) {
     const double per_job = (double)kSlots * o * o * o * scratch_elt(mode)
                          + (mode == CT_MODE_FP64 ? 0.0 : mixed_extra_bytes_per_job(o, mode));
     long long mw = (long long)(scratch_budget_mb(W) * 1048576.0 / per_job);
-    if (use_cube(o, mode)) mw = std::min<long long>(mw, (96LL << 20) / (8LL * o * o * o));
     mw = std::max<long long>(1, std::min<long long>(mw, 8192));
     const long long round = 2LL * (W.sm_count > 0 ? W.sm_count : 148);
     if (mw >= round) mw -= mw % round;
@@ -636,7 +636,7 @@ static int run_waves(Workspace &W, const Plan &P, const ct_problem *p, int mode,
         wv.ochunks = P.d_ochunks + 3 * P.ochunk_begin[w];
         if (cube) {
             double *S = (double *)W.scratch;
-            long long stride = (long long)o * o * o;
+            long long stride = 3LL * o * o * o;
             if (lno_mat) {
                 EpiArgs ef = ea;
                 ef.with_vjp = 0;
@@ -650,7 +650,7 @@ static int run_waves(Workspace &W, const Plan &P, const ct_problem *p, int mode,
                 { CT_PROF(PK_RED); CT_CK(f64_lno_vjp_project(wv, ea, S, st)); }
                 { CT_PROF(PK_VB); CT_CK(cube_lno_backward(wv, ea, p->vooo, g->vooo, S, st)); }
                 { CT_PROF(PK_RED); CT_CK(f64_lno_mat_bar(wv, ea, lno_mat_bar, st)); }
-                stride *= kSlots;
+                stride = (long long)kSlots * o * o * o;
             } else {
                 CT_PROF(PK_F1);
                 CT_CK(cube_vjp(wv, ea, p->vooo, g->vooo, S, st));

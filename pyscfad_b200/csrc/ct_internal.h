@@ -86,8 +86,9 @@ cudaError_t f64_epilogue(const WaveView &w, const EpiArgs &e, double *scratch, c
 cudaError_t f64_vterm(const WaveView &w, const EpiArgs &e, const double *scratch, cudaStream_t st);
 // float64 path for 2 <= nocc <= kCubeMaxO (ct_cube.cu): one CTA per job with its
 // cube in shared memory.  Energy over a job list (no scratch); per wave the
-// VJP (w-bar cube of job jl to cubes + jl o^3) or the two LNO passes (slots
-// 0-5 as f64_lno_* use them; the backward pass leaves w-bar in slot 0), then
+// VJP (three w-bar cubes of job jl to cubes + 3 jl o^3: [i][j][k], [i][k][j],
+// [j][k][i]) or the two LNO passes (slots 0-5 as f64_lno_* use them; the
+// backward pass leaves the same three cubes in slots 0-2), then
 // the t2-bar GEMM over the wave's w-bar cubes
 constexpr int kCubeMaxO = 24;
 cudaError_t cube_energy(const int *jobs, int n_jobs, const EpiArgs &e, const double *vooo, cudaStream_t st);
