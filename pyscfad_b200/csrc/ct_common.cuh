@@ -59,6 +59,12 @@ __host__ __device__ constexpr double kR3C(int t) {
     return T[t];
 }
 
+// The float64 paths keep a job's w-bar as three copies of its cube, 0: [i][j][k],
+// 1: [i][k][j], 2: [j][k][i].  Wbar_sigma[p,q,r] is element (p,q,r) (first) or (q,p,r)
+// of one of them, so that r is contiguous for every sigma.
+__host__ __device__ constexpr int wbar_cube(int s) { return (0x212010 >> (4 * s)) & 3; }
+__host__ __device__ constexpr bool wbar_first(int s) { return s != 2 && s < 4; }
+
 // symmetry factor of a sorted job (get_d3 callers, ccsd_t_vjp.c:298-304)
 __host__ __device__ inline double job_fac(int a, int b, int c) {
     return (a == c) ? (1.0 / 6.0) : ((a == b || b == c) ? 0.5 : 1.0);

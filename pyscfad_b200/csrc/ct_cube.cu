@@ -71,17 +71,6 @@ __device__ __forceinline__ int rtR(int s, int m) {
     return (int)((P >> (6 * s + 2 * m)) & 3);
 }
 
-// Neumaier pairs and a plain partial summed down a warp in a fixed order; valid in lane 0
-__device__ __forceinline__ void ksum_tree(KSum &k, double &v) {
-#pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) {
-        const double s2 = __shfl_down_sync(0xffffffffu, k.s, m), c2 = __shfl_down_sync(0xffffffffu, k.c, m);
-        v += __shfl_down_sync(0xffffffffu, v, m);
-        k.c += c2;
-        k.add(s2);
-    }
-}
-
 template <int MT, int NT, int MODE, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
     extern __shared__ __align__(16) double sm[];
@@ -797,9 +786,8 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
 // ---------------------------------------------------------------------------
 // TB: t2T_bar[z,f,qr] += sum_t sum_p vvop[x,y,p,o+f] Wbar_t[p,qr] over the
 // wave's terms with that z.  64 (f) x 64 (qr) tiles, 4 warps of 32 x 32, one
-// stage = `tps` terms of op rows (o rounded up to the MMA's K); the term list
-// is split into `splits` parts per tile so that a wave with few z still fills
-// the GPU (the parts add into t2T_bar).  Each job's w-bar comes as three cubes,
+// stage = `tps` terms of op rows (o rounded up to the MMA's K); one CTA per tile
+// and part of a z's term list (the parts add into t2T_bar).  Each job's w-bar comes as three cubes,
 // the contiguous axis that of c, b or a: a term reads the one of its z, where
 // its r runs along memory (from one cube, a third of the terms were gathered
 // along p and a third along q in 8-byte pieces).  Even sizes copy 16 bytes.
@@ -808,10 +796,10 @@ struct TbArgs {
     const double *vvop, *cubes;
     double *t2T_bar;
     long long stride;
-    int o, v, n, op, tps, splits, tiles_n;
+    int o, v, n, op, tps, tiles_n;
     int vec_a, vec_b;     // 16-byte copies of the vvop rows / the cubes
     unsigned magic;
-    const int *jobs, *entries, *groups;
+    const int *jobs, *entries, *parts;
 };
 constexpr int kTbLD = 68, kTbTerms = 128;
 
@@ -823,14 +811,10 @@ __global__ void __launch_bounds__(128, 4) tb_kernel(const TbArgs P) {
     double *As = tsm, *Bs = tsm + 2 * buf;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, c4 = lane & 3;
     const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
-    const int gi = blockIdx.x / P.splits, sp = blockIdx.x - gi * P.splits;
     const int tm = blockIdx.y / P.tiles_n, tn = blockIdx.y - tm * P.tiles_n;
     const int f0 = tm * 64, n0 = tn * 64;
-    const int z = P.groups[3 * gi];
-    const int eb = P.groups[3 * gi + 1], ne = P.groups[3 * gi + 2] - eb;
-    const int e0 = eb + (int)((long long)ne * sp / P.splits), e1 = eb + (int)((long long)ne * (sp + 1) / P.splits);
-    const int nt = e1 - e0, nst = (nt + P.tps - 1) / P.tps;
-    if (nt <= 0) return;
+    const int z = P.parts[3 * blockIdx.x], e0 = P.parts[3 * blockIdx.x + 1];
+    const int nt = P.parts[3 * blockIdx.x + 2] - e0, nst = (nt + P.tps - 1) / P.tps;
     // this thread's column of the A and B copies and its first row (of every 2, or 4)
     const int ca = P.vec_a ? 2 * (tid & 31) : tid & 63, ra = P.vec_a ? tid >> 5 : tid >> 6, da = P.vec_a ? 4 : 2;
     const int cb = P.vec_b ? 2 * (tid & 31) : tid & 63, rb = P.vec_b ? tid >> 5 : tid >> 6, db = P.vec_b ? 4 : 2;
@@ -858,9 +842,8 @@ __global__ void __launch_bounds__(128, 4) tb_kernel(const TbArgs P) {
                 if (P.vec_a) cp_async16z(a_ + (u * op + p) * kTbLD, src + p * n, ok);
                 else cp_async8(a_ + (u * op + p) * kTbLD, src + p * n, ok);
             }
-            // cube of the term's z (0, 1, 0, 2, 1, 2) and which of its outer axes is p
-            const int s = js & 7, cube = (0x212010 >> (4 * s)) & 3;
-            const bool first = s != 2 && s < 4;
+            const int s = js & 7, cube = wbar_cube(s);
+            const bool first = wbar_first(s);
             const int sp0 = first ? oo : o, sq = first ? o : oo;
             const double *q = P.cubes + (long long)(js >> 3) * P.stride + (long long)cube * oo * o + cq * sq + cr;
             for (int p = rb; p < op; p += db) {
@@ -1035,9 +1018,8 @@ cudaError_t cube_lno_backward(const WaveView &w, const EpiArgs &e, const double 
     return cube::launch_o<cube::M_LNO_BWD>(A, w.n_jobs, st);
 }
 
-cudaError_t cube_tb(const WaveView &w, const EpiArgs &e, const double *cubes, long long stride, int sms,
-                    cudaStream_t st) {
-    if (w.n_tb_groups <= 0) return cudaSuccess;
+cudaError_t cube_tb(const WaveView &w, const EpiArgs &e, const double *cubes, long long stride, cudaStream_t st) {
+    if (w.n_zparts <= 0) return cudaSuccess;
     cube::TbArgs P{};
     P.vvop = e.vvop;
     P.cubes = cubes;
@@ -1053,16 +1035,12 @@ cudaError_t cube_tb(const WaveView &w, const EpiArgs &e, const double *cubes, lo
     P.vec_b = e.o % 2 == 0 && stride % 2 == 0 && reinterpret_cast<uintptr_t>(cubes) % 16 == 0;
     P.jobs = w.jobs;
     P.entries = w.tb_entries;
-    P.groups = w.tb_groups;
+    P.parts = w.zparts;
     const int tiles = ((e.v + 63) / 64) * P.tiles_n;
-    // about eight rounds of four CTAs per SM, parts of at least 16 terms
-    const long long want = 32LL * sms, have = (long long)w.n_tb_groups * tiles;
-    const long long by_terms = 6LL * w.n_jobs / (16LL * w.n_tb_groups);
-    P.splits = (int)std::max<long long>(1, std::min<long long>((want + have - 1) / have, by_terms));
     const size_t smem = sizeof(double) * 4 * (size_t)P.op * P.tps * cube::kTbLD;
     cudaError_t ce = smem_optin(reinterpret_cast<const void *>(cube::tb_kernel), (int)smem);
     if (ce != cudaSuccess) return ce;
-    cube::tb_kernel<<<dim3(w.n_tb_groups * P.splits, tiles), 128, smem, st>>>(P);
+    cube::tb_kernel<<<dim3(w.n_zparts, tiles), 128, smem, st>>>(P);
     return cudaGetLastError();
 }
 

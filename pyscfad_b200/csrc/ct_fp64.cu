@@ -1,16 +1,10 @@
-// Float64 path of the B200 CCSD(T) energy + VJP.
-//
-// Per wave of sorted jobs (a>=b>=c) the host runs:
-//   F1  G_sigma[p,qr]   = sum_f vvop[x,y,p,o+f] t2T[z,f,qr]        (get_wv dgemm 1, ccsd_t.c:137-139)
-//   F2  G_sigma[pq,r]  -= sum_l vooo[x,pq,l] t2T[z,y,l,r]           (get_wv dgemm 2, ccsd_t.c:140-142)
+// Float64 orbit epilogue and V-term bars, the mixed path's V-term bars and the
+// energy reduction.  Per wave of sorted jobs (a>=b>=c) the float64 slot path runs:
+//   W   G_sigma[p,qr]   = sum_f vvop[x,y,p,o+f] t2T[z,f,qr] - sum_l vooo[x,pq,l] t2T[z,y,l,r]   (ct_pair.cu)
 //   EPI orbit epilogue: W, V, r3, D, energy, zbar/d3bar/wbar/vbar, mo_energy_bar
 //                                                                   (ccsd_t_vjp.c:9-117, lno_ccsd_t.c:6-29)
 //   VT  V-term bars of t1T, fvo, vvop[:,:,:,:o], t2T                (ccsd_t_vjp.c:171-246 gemv parts)
-//   VB  vvop_bar[x,y,p,o+f] += sum_qr t2T[z,f,qr] Wbar_sigma[p,qr]  (get_vvov_bar, :139-152)
-//   TB  t2T_bar[z,f,qr]     += sum_{terms with z} vvop[x,y,p,o+f] Wbar[p,qr]  (get_t2T_bar dgemm 1)
-//   OB1 vooo_bar[x,pq,l]    -= sum_r t2T[z,y,l,r] Wbar[pq,r]        (get_vooo_bar, :154-169)
-//   OB2 t2T_bar[z,y,l,r]    -= sum_pq vooo[x,pq,l] Wbar[pq,r]       (get_t2T_bar dgemm 2)
-// The GEMMs run on the float64 tensor pipe (DMMA, mma.sync m8n8k4 .f64).
+//   VB, TB, OB1, OB2  the bars of the two products                  (ct_pair.cu)
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cstdio>
@@ -20,491 +14,251 @@
 
 namespace ctb {
 
-enum OutMode { OUT_STORE = 0, OUT_ADD = 1, OUT_ATOMIC = 2 };
-
-struct GemmParams {
-    const double *A, *B;
-    double *C;
-    long long sAm, sAk, sBn, sBk, sCm, sCn;
-    int M, N, K;
-    double alpha;
-    int o, v, n;
-    const int *jobs;
-    const int *tb_entries;
-    const int *tb_groups;
-};
-
-template <int KIND> struct KindTraits;
-template <> struct KindTraits<K_F1>  { static constexpr bool A_MC = true,  B_NC = false; static constexpr int OUT = OUT_STORE; };
-template <> struct KindTraits<K_F2>  { static constexpr bool A_MC = false, B_NC = true;  static constexpr int OUT = OUT_ADD; };
-template <> struct KindTraits<K_VB>  { static constexpr bool A_MC = false, B_NC = false; static constexpr int OUT = OUT_ATOMIC; };
-template <> struct KindTraits<K_TB>  { static constexpr bool A_MC = true,  B_NC = true;  static constexpr int OUT = OUT_ATOMIC; };
-template <> struct KindTraits<K_OB1> { static constexpr bool A_MC = false, B_NC = false; static constexpr int OUT = OUT_ATOMIC; };
-template <> struct KindTraits<K_OB2> { static constexpr bool A_MC = true,  B_NC = true;  static constexpr int OUT = OUT_ATOMIC; };
-
-// element offsets of A, B and C for term id e = jl*6 + sigma of the wave
-template <int KIND>
-__device__ __forceinline__ void entry_offsets(const GemmParams &p, int e, long long &ao, long long &bo,
-                                              long long &co) {
-    const int jl = e / 6, sg = e - 6 * (e / 6);
-    int a, b, c, x, y, z;
-    unpack_job(p.jobs[jl], a, b, c);
-    term_xyz(sg, a, b, c, x, y, z);
-    const long long o = p.o, v = p.v, n = p.n, o2 = o * o, o3 = o2 * o;
-    const long long slot = ((long long)jl * kSlots + sg) * o3;
-    const long long vv_row = ((long long)(x * v + y) * o) * n + o;
-    switch (KIND) {
-    case K_F1:  ao = z * v * o2;       bo = vv_row;             co = slot; break;
-    case K_F2:  ao = x * o3;           bo = (z * v + y) * o2;   co = slot; break;
-    case K_VB:  ao = z * v * o2;       bo = slot;               co = vv_row; break;
-    case K_TB:  ao = vv_row;           bo = slot;               co = z * v * o2; break;
-    case K_OB1: ao = slot;             bo = (z * v + y) * o2;   co = x * o3; break;
-    default:    ao = x * o3;           bo = slot;               co = (z * v + y) * o2; break;
-    }
-}
-
-// C[m,n] (op)= alpha * sum_{entries} sum_k A_e[m,k] B_e[n,k]; CTA tile 64 x BN x 16,
-// 4 warps of 32 x BN/2, double-buffered shared memory with register prefetch.
-template <int BN, int KIND>
-__global__ void __launch_bounds__(128) gemm_f64_kernel(const GemmParams p) {
-    using T = KindTraits<KIND>;
-    constexpr int BM = 64, BK = 16;
-    constexpr int A_LD = T::A_MC ? (BM + 8) : (BK + 4);
-    constexpr int A_SZ = T::A_MC ? BK * A_LD : BM * A_LD;
-    constexpr int B_LD = T::B_NC ? (BN + 8) : (BK + 4);
-    constexpr int B_SZ = T::B_NC ? BK * B_LD : BN * B_LD;
-    constexpr int NT = BN / 16;
-    constexpr int BPT = BN * BK / 128;
-    __shared__ double As[2][A_SZ];
-    __shared__ double Bs[2][B_SZ];
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp & 1, wn = warp >> 1;
-    const int tiles_n = (p.N + BN - 1) / BN;
-    const int tm = blockIdx.y / tiles_n, tn = blockIdx.y - tm * tiles_n;
-    const int m0 = tm * BM, n0 = tn * BN;
-
-    int e_begin, e_end;
-    long long coff = 0;
-    if (KIND == K_TB) {
-        const int z = p.tb_groups[3 * blockIdx.x];
-        e_begin = p.tb_groups[3 * blockIdx.x + 1];
-        e_end = p.tb_groups[3 * blockIdx.x + 2];
-        coff = (long long)z * p.v * p.o * p.o;
-    } else {
-        e_begin = blockIdx.x;
-        e_end = blockIdx.x + 1;
-    }
-    const int kt_per = (p.K + BK - 1) / BK;
-    const int ntiles = (e_end - e_begin) * kt_per;
-
-    double acc[4][NT][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-    double ra[8], rb[BPT];
-    int cur_e = -1;
-    const double *Ae = nullptr, *Be = nullptr;
-
-    auto load_tile = [&](int t) {
-        const int e = e_begin + t / kt_per;
-        const int k0 = (t - (t / kt_per) * kt_per) * BK;
-        if (e != cur_e) {
-            cur_e = e;
-            const int eid = (KIND == K_TB) ? p.tb_entries[e] : e;
-            long long ao, bo, co;
-            entry_offsets<KIND>(p, eid, ao, bo, co);
-            Ae = p.A + ao;
-            Be = p.B + bo;
-            if (KIND != K_TB) coff = co;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int idx = tid + i * 128;
-            int m, k;
-            if (T::A_MC) { k = idx >> 6; m = idx & 63; } else { m = idx >> 4; k = idx & 15; }
-            const int gm = m0 + m, gk = k0 + k;
-            ra[i] = (gm < p.M && gk < p.K) ? __ldg(Ae + gm * p.sAm + gk * p.sAk) : 0.0;
-        }
-#pragma unroll
-        for (int i = 0; i < BPT; ++i) {
-            const int idx = tid + i * 128;
-            int nn, k;
-            if (T::B_NC) { k = idx / BN; nn = idx - k * BN; } else { nn = idx >> 4; k = idx & 15; }
-            const int gn = n0 + nn, gk = k0 + k;
-            rb[i] = (gn < p.N && gk < p.K) ? __ldg(Be + gn * p.sBn + gk * p.sBk) : 0.0;
-        }
-    };
-    auto store_tile = [&](int buf) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int idx = tid + i * 128;
-            if (T::A_MC) { const int k = idx >> 6, m = idx & 63; As[buf][k * A_LD + m] = ra[i]; }
-            else { const int m = idx >> 4, k = idx & 15; As[buf][m * A_LD + k] = ra[i]; }
-        }
-#pragma unroll
-        for (int i = 0; i < BPT; ++i) {
-            const int idx = tid + i * 128;
-            if (T::B_NC) { const int k = idx / BN, nn = idx - k * BN; Bs[buf][k * B_LD + nn] = rb[i]; }
-            else { const int nn = idx >> 4, k = idx & 15; Bs[buf][nn * B_LD + k] = rb[i]; }
-        }
-    };
-
-    if (ntiles > 0) {
-        load_tile(0);
-        store_tile(0);
-        __syncthreads();
-        for (int t = 0; t < ntiles; ++t) {
-            const int buf = t & 1;
-            if (t + 1 < ntiles) load_tile(t + 1);
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-                double af[4], bf[NT];
-                const int kk = ks * 4 + (lane & 3);
-#pragma unroll
-                for (int mt = 0; mt < 4; ++mt) {
-                    const int m = wm * 32 + mt * 8 + (lane >> 2);
-                    af[mt] = T::A_MC ? As[buf][kk * A_LD + m] : As[buf][m * A_LD + kk];
-                }
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    const int nn = wn * (BN / 2) + nt * 8 + (lane >> 2);
-                    bf[nt] = T::B_NC ? Bs[buf][kk * B_LD + nn] : Bs[buf][nn * B_LD + kk];
-                }
-#pragma unroll
-                for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-                    for (int nt = 0; nt < NT; ++nt) dmma(acc[mt][nt], af[mt], bf[nt]);
-            }
-            if (t + 1 < ntiles) store_tile(buf ^ 1);
-            __syncthreads();
-        }
-    }
-
-    double *C = p.C + coff;
-#pragma unroll
-    for (int mt = 0; mt < 4; ++mt) {
-        const int m = m0 + wm * 32 + mt * 8 + (lane >> 2);
-        if (m >= p.M) continue;
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int nn = n0 + wn * (BN / 2) + nt * 8 + (lane & 3) * 2 + h;
-                if (nn >= p.N) continue;
-                double *c = C + m * p.sCm + nn * p.sCn;
-                const double val = p.alpha * acc[mt][nt][h];
-                if (T::OUT == OUT_STORE) *c = val;
-                else if (T::OUT == OUT_ADD) *c += val;
-                else atomicAdd(c, val);
-            }
-    }
-}
-
-template <int KIND>
-static cudaError_t launch_kind(const GemmParams &p, int groups, cudaStream_t st) {
-    const int bn = p.N <= 16 ? 16 : (p.N <= 32 ? 32 : (p.N <= 48 ? 48 : 64));
-    const int tiles = ((p.M + 63) / 64) * ((p.N + bn - 1) / bn);
-    if (groups <= 0) return cudaSuccess;
-    if (tiles > 65535) return cudaErrorInvalidConfiguration;
-    dim3 grid(groups, tiles);
-    switch (bn) {
-    case 16: gemm_f64_kernel<16, KIND><<<grid, 128, 0, st>>>(p); break;
-    case 32: gemm_f64_kernel<32, KIND><<<grid, 128, 0, st>>>(p); break;
-    case 48: gemm_f64_kernel<48, KIND><<<grid, 128, 0, st>>>(p); break;
-    default: gemm_f64_kernel<64, KIND><<<grid, 128, 0, st>>>(p); break;
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t f64_gemm(GemmKind kind, const WaveView &w, const double *A, const double *B, double *C,
-                     double *scratch, cudaStream_t st) {
-    (void)scratch;
-    GemmParams p{};
-    p.A = A; p.B = B; p.C = C;
-    p.o = w.o; p.v = w.v; p.n = w.n;
-    p.jobs = w.jobs; p.tb_entries = w.tb_entries; p.tb_groups = w.tb_groups;
-    const long long o = w.o, v = w.v, n = w.n, o2 = o * o;
-    const int terms = w.n_jobs * 6;
-    switch (kind) {
-    case K_F1:
-        p.sAm = 1; p.sAk = o2; p.sBn = n; p.sBk = 1; p.sCm = 1; p.sCn = o2;
-        p.M = (int)o2; p.N = (int)o; p.K = (int)v; p.alpha = 1.0;
-        return launch_kind<K_F1>(p, terms, st);
-    case K_F2:
-        p.sAm = o; p.sAk = 1; p.sBn = 1; p.sBk = o; p.sCm = o; p.sCn = 1;
-        p.M = (int)o2; p.N = (int)o; p.K = (int)o; p.alpha = -1.0;
-        return launch_kind<K_F2>(p, terms, st);
-    case K_VB:
-        p.sAm = o2; p.sAk = 1; p.sBn = o2; p.sBk = 1; p.sCm = 1; p.sCn = n;
-        p.M = (int)v; p.N = (int)o; p.K = (int)o2; p.alpha = 1.0;
-        return launch_kind<K_VB>(p, terms, st);
-    case K_TB:
-        p.sAm = 1; p.sAk = n; p.sBn = 1; p.sBk = o2; p.sCm = o2; p.sCn = 1;
-        p.M = (int)v; p.N = (int)o2; p.K = (int)o; p.alpha = 1.0;
-        return launch_kind<K_TB>(p, w.n_tb_groups, st);
-    case K_OB1:
-        p.sAm = o; p.sAk = 1; p.sBn = o; p.sBk = 1; p.sCm = o; p.sCn = 1;
-        p.M = (int)o2; p.N = (int)o; p.K = (int)o; p.alpha = -1.0;
-        return launch_kind<K_OB1>(p, terms, st);
-    default:
-        p.sAm = 1; p.sAk = o; p.sBn = 1; p.sBk = o; p.sCm = o; p.sCn = 1;
-        p.M = (int)o; p.N = (int)o; p.K = (int)o2; p.alpha = -1.0;
-        return launch_kind<K_OB2>(p, terms, st);
-    }
-}
-
 // ---------------------------------------------------------------------------
-// Orbit epilogue, tiled.  One CTA per job.  The occupied cube is cut into
-// T^3 blocks; a block-orbit is a sorted block triple I>=J>=K together with
-// its (up to 6) permuted blocks.  For each block-orbit the CTA stages, with
-// coalesced T-element rows, the permuted blocks of all six G slots and the
-// V-term tiles in shared memory; each thread then owns whole element orbits
-// {perm(i,j,k)}, so W, V, r3, the denominator and the backward quantities
-// never leave registers; W-bar is written back block by block and ybar
-// straight to its slot.
+// Orbit epilogue.  One CTA per job; a thread owns whole element orbits
+// {perm(i,j,k)}, so W, V, r3, the denominator and the backward quantities never
+// leave registers and nobody else touches an orbit's elements: they are read
+// from the six G slots and written back in place, no shared memory and no
+// barrier between orbits.  A warp takes half a block-orbit at a time: the
+// orbits i >= j >= k of a 2 x 4 x 4 block (I, J, K), whose accesses in every
+// permuted order run along 32-byte pieces.  It is bound by the latency of those
+// loads: staging the blocks in shared memory (64-thread CTAs, 36 tiles of 4^3)
+// spent 4000 instructions per block-orbit on addresses, copies and barriers and
+// wrote six W-bar cubes: 50 -> 31 ms over the 6,213 jobs of a nocc=48/nvir=300
+// slab block, 307 -> 94 ms for all jobs of nocc=33/nvir=64 with fvo.  w-bar goes to slots 0-2 as three copies of one cube,
+// [i][j][k], [i][k][j] and [j][k][i]: each W-bar_sigma is one of them with r
+// contiguous (ct_pair.cu).
 // ---------------------------------------------------------------------------
-template <typename ST, int T, typename VT>
-struct EpiSmem {
-    static constexpr int T3 = T * T * T, T2 = T * T;
-    // tile layout: element (u, w, t) of a staged block at u*TP + w*T + t.  For
-    // T = 8 each u-plane is padded by 4 elements, which (with the thread
-    // mapping of loc_of) keeps the six permuted access patterns of a warp at
-    // most 2-way bank-conflicted.
-    static constexpr int TP = T2 + (T == 8 ? 4 : 0), BLK = T * TP;
-    static constexpr size_t g_off = 0;                                       // ST[6][6][BLK]
-    static constexpr size_t va_off = g_off + sizeof(ST) * 36 * BLK;          // VT[6][6][T2]
-    static constexpr size_t vb_off = va_off + sizeof(VT) * 36 * T2;          // VT[6][6][T2]
-    static constexpr size_t u_off = vb_off + sizeof(VT) * 36 * T2;           // VT[6][64]
-    static constexpr size_t w_off = u_off + sizeof(VT) * 6 * 64;             // VT[6][64]
-    static constexpr size_t occ_off = w_off + sizeof(VT) * 6 * 64;           // double[64]
-    static constexpr size_t eocc_off = occ_off + sizeof(double) * 64;        // double[64]
-    static constexpr size_t tmp_off = eocc_off + sizeof(double) * 64;        // double[T3]
-    static size_t bytes(int nthr) {
-        (void)nthr;  // the final reduction reuses the G-tile area
-        return tmp_off + sizeof(double) * T3;
-    }
-    __device__ static int pidx(int e3) { return (e3 / T2) * TP + e3 % T2; }
-};
+enum EpiMode { E_ENERGY, E_VJP, E_LNO_FWD, E_LNO_BWD, E_T3 };
+constexpr int kEpiThreads = 256, kEpiWarps = kEpiThreads / 32;
 
-// T3M: the iterative (T) seed build (orbit_t3), a separate instance so the
-// other modes keep their register allocation
-template <typename ST, int T, typename VT, int NTHR, int WB, bool T3M = false>
-__global__ void __launch_bounds__(NTHR, (NTHR >= 256 ? 2 : 4)) epi_kernel(const WaveView w, const EpiArgs e, ST *scratch) {
-    using L = EpiSmem<ST, T, VT>;
-    constexpr int T3 = L::T3, T2 = L::T2, TP = L::TP, BLK = L::BLK;
-    extern __shared__ __align__(16) uint8_t esm[];
-    ST *Gs = reinterpret_cast<ST *>(esm + L::g_off);
-    VT *VA = reinterpret_cast<VT *>(esm + L::va_off);
-    VT *VB = reinterpret_cast<VT *>(esm + L::vb_off);
-    VT *Us = reinterpret_cast<VT *>(esm + L::u_off);
-    VT *Ws = reinterpret_cast<VT *>(esm + L::w_off);
-    double *occ_acc = reinterpret_cast<double *>(esm + L::occ_off);
-    double *tmp_s = reinterpret_cast<double *>(esm + L::tmp_off);
-    double *eocc = reinterpret_cast<double *>(esm + L::eocc_off);
-    double *red = reinterpret_cast<double *>(esm + L::g_off);  // used after the last block-orbit
-    static_assert(sizeof(ST) * 36 * BLK >= sizeof(double) * 3 * NTHR, "reduction area");
-
+template <int MODE>
+__global__ void __launch_bounds__(kEpiThreads, 2) epi_kernel(const WaveView w, const EpiArgs e, double *scratch) {
+    constexpr bool BAR = MODE == E_VJP || MODE == E_LNO_BWD;
+    __shared__ double U[3][64], F[3][64], eocc[64], occ[kEpiWarps][64], wred[3][kEpiWarps];
+    __shared__ const double *va[6], *vb[6];   // vvop[x,y] and t2T[y,x] of the six terms
     const int o = e.o, v = e.v, n = e.n;
     const long long o3 = (long long)o * o * o;
-    const int jl = blockIdx.x, tid = threadIdx.x;
+    const int jl = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int a, b, c;
     unpack_job(w.jobs[jl], a, b, c);
-    const double fac = job_fac(a, b, c);
+    double *S = scratch + (long long)jl * kSlots * o3;
+    const double fac = job_fac(a, b, c), eb = e.et_bar;
     const double eabc = e.mo_energy[o + a] + e.mo_energy[o + b] + e.mo_energy[o + c];
-    ST *S = scratch + (long long)jl * kSlots * o3;
-    const bool vjp = e.with_vjp != 0;
-    const bool lno = e.lno_phase == 1 && !vjp;    // LNO forward: W and z/D cubes
-    const bool lbar = e.lno_phase == 2 && vjp;    // LNO backward pass
-    const bool t3m = T3M && !vjp;                 // iterative (T) seed: 6-D arrays
-
-    // per-term offsets of the V-term operand rows vvop[x,y] and t2T[y,x]
-    // (shared memory: read with a runtime term index, no local-memory array)
-    __shared__ long long vv_off[6], tt_off[6];
     if (tid < 6) {
         int x, y, z;
         term_xyz(tid, a, b, c, x, y, z);
-        vv_off[tid] = ((long long)(x * v + y) * o) * n;
-        tt_off[tid] = ((long long)(y * v + x) * o) * o;
+        va[tid] = e.vvop + ((long long)(x * v + y) * o) * n;
+        vb[tid] = e.t2T + ((long long)(y * v + x) * o) * o;
     }
-    for (int i = tid; i < o; i += NTHR) { occ_acc[i] = 0.0; eocc[i] = e.mo_energy[i]; }
-    for (int i = tid; i < 6 * o; i += NTHR) {
-        const int sg = i / o, r = i - sg * o;
-        int x, y, z;
-        term_xyz(sg, a, b, c, x, y, z);
-        Us[sg * 64 + r] = (VT)e.t1T[z * o + r];
-        Ws[sg * 64 + r] = (VT)e.fvo[z * o + r];
+    int fnz = 0;
+    for (int i = tid; i < 3 * 64; i += kEpiThreads) {
+        const int m = i >> 6, r = i & 63, z = m == 0 ? a : (m == 1 ? b : c);
+        const double f = r < o ? e.fvo[z * o + r] : 0.0;
+        U[m][r] = r < o ? e.t1T[z * o + r] : 0.0;
+        F[m][r] = f;
+        fnz |= f != 0.0;
     }
+    for (int i = tid; i < o; i += kEpiThreads) eocc[i] = e.mo_energy[i];
+    for (int i = tid; i < kEpiWarps * 64; i += kEpiThreads) occ[i >> 6][i & 63] = 0.0;
+    // with zero fvo rows the fvo part of V adds zeros: skipped
+    const bool with_fvo = __syncthreads_or(fnz) != 0;
 
     KSum eacc;
-    double vir_acc = 0.0;
-    const double eb = e.et_bar;
-    const int nb = (o + T - 1) / T;
+    double vir = 0.0;
+    const int half = warp & 1, nb = (o + 3) / 4, nbo = nb * (nb + 1) * (nb + 2) / 6;
     int BI = 0, BJ = 0, BK = 0;
-    const int nbo = nb * (nb + 1) * (nb + 2) / 6;
-    for (int bo = 0; bo < nbo; ++bo) {
-        if (bo > 0) {  // next sorted block triple (I >= J >= K), K fastest
+    auto next = [&](int steps) {   // sorted block triples I >= J >= K, K fastest
+        for (int q = 0; q < steps; ++q) {
             if (BK < BJ) ++BK;
             else if (BJ < BI) { ++BJ; BK = 0; }
             else { ++BI; BJ = 0; BK = 0; }
         }
-        const int blk[3] = {BI, BJ, BK};
-        // permuted blocks of the orbit; dmap[s]: staging buffer of slot s's block,
-        // fresh[s]: slot s is the first with that block (all indices compile-time)
-        int bs[6][3], dmap[6], nd = 0;
-        bool fresh[6];
-#pragma unroll
-        for (int s = 0; s < 6; ++s) {
-#pragma unroll
-            for (int m = 0; m < 3; ++m) bs[s][m] = blk[kR(s, m)];
-            int found = -1;
-#pragma unroll
-            for (int t = 0; t < s; ++t)
-                if (found < 0 && bs[t][0] == bs[s][0] && bs[t][1] == bs[s][1] && bs[t][2] == bs[s][2]) found = dmap[t];
-            fresh[s] = found < 0;
-            dmap[s] = found < 0 ? nd++ : found;
-        }
-        __syncthreads();  // previous block-orbit fully written back
-        // stage G blocks of the six slots (T-element rows, full-row vector loads)
-        const bool full = (BI + 1) * T <= o;  // every block of this orbit lies inside the cube
-#pragma unroll
-        for (int s = 0; s < 6; ++s) {
-            if (!fresh[s]) continue;
-            const int d = dmap[s];
-            const int p0 = bs[s][0] * T, q0 = bs[s][1] * T, r0 = bs[s][2] * T;
-            // LNO backward: the z/D cube and the two parts of A and B (slots 1-5)
-            // into tile groups 0-4
-            for (int sg = 0; sg < (lbar ? 5 : 6); ++sg) {
-                const ST *src = S + (sg + (lbar ? 1 : 0)) * o3;
-                ST *dst = Gs + (sg * 6 + d) * BLK;
-                if (full && sizeof(ST) * T % 16 == 0 && (sizeof(ST) * o) % 16 == 0) {
-                    constexpr int VEC = 16 / sizeof(ST), NV = T3 / VEC;
-                    for (int i = tid; i < NV; i += NTHR) {
-                        const int e3 = i * VEC;
-                        const int u = e3 / T2, ww = (e3 / T) % T, t = e3 % T;
-                        cp_async16(dst + L::pidx(e3), src + ((long long)(p0 + u) * o + q0 + ww) * o + r0 + t);
-                    }
-                } else {
-                    for (int e3 = tid; e3 < T3; e3 += NTHR) {
-                        const int p = p0 + e3 / T2, q = q0 + (e3 / T) % T, r = r0 + e3 % T;
-                        dst[L::pidx(e3)] = (p < o && q < o && r < o) ? src[((long long)p * o + q) * o + r] : ST(0);
-                    }
-                }
-            }
-        }
-        // stage V-term tiles: A = vvop[x,y,P,Q], B = t2T[y,x,P,Q] on the block pair of each
-        // slot; all loads of a thread are issued before its shared-memory stores
-        if (!lbar) {
-            constexpr int NV = (36 * T2 + NTHR - 1) / NTHR;
-            double la[NV], lb[NV];
-#pragma unroll
-            for (int k = 0; k < NV; ++k) {
-                const int idx = tid + k * NTHR;
-                la[k] = lb[k] = 0.0;
-                if (idx < 36 * T2) {
-                    const int sg = idx / (6 * T2), cc = (idx / T2) % 6, uw = idx % T2;
-                    // blocks of slot cc's first two axes: blk[kR(cc,0)], blk[kR(cc,1)]
-                    constexpr unsigned int KR01 = (0u | 1u << 2) | (0u | 2u << 2) << 4 | (1u | 0u << 2) << 8 |
-                                                  (1u | 2u << 2) << 12 | (2u | 0u << 2) << 16 | (2u | 1u << 2) << 20;
-                    const int k0 = (KR01 >> (4 * cc)) & 3, k1 = (KR01 >> (4 * cc + 2)) & 3;
-                    const int P = (k0 == 0 ? BI : (k0 == 1 ? BJ : BK)) * T + uw / T;
-                    const int Q = (k1 == 0 ? BI : (k1 == 1 ? BJ : BK)) * T + uw % T;
-                    if (P < o && Q < o) {
-                        la[k] = __ldg(e.vvop + vv_off[sg] + (long long)P * n + Q);
-                        lb[k] = __ldg(e.t2T + tt_off[sg] + (long long)P * o + Q);
-                    }
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < NV; ++k) {
-                const int idx = tid + k * NTHR;
-                if (idx < 36 * T2) {
-                    VA[idx] = (VT)la[k];
-                    VB[idx] = (VT)lb[k];
-                }
-            }
-        }
-        cp_async_wait_all();
-        __syncthreads();
-        for (int q = tid; q < T3; q += NTHR) {
-            int loc[3];
-            loc_of<T, NTHR>(q, loc);
-            if (lbar)
-                orbit_lno_bar<ST, T, TP, BLK>(loc, BI, BJ, BK, dmap, Gs, eocc, tmp_s, S + 6 * o3, o, eabc, eb,
-                                              vir_acc);
-            else if (t3m)
-                orbit_t3<ST, VT, T, TP, BLK>(loc, BI, BJ, BK, dmap, Gs, VA, VB, Us, Ws, eocc, o, v, eabc, a, b, c,
-                                             e.t3_c, e.t3_x);
-            else
-                orbit_element<double, ST, VT, T, TP, BLK, WB>(loc, BI, BJ, BK, dmap, Gs, VA, VB, Us, Ws, eocc, tmp_s,
-                                                              S + 6 * o3, o, fac, eabc, eb, vjp, eacc, vir_acc, true,
-                                                              nullptr, nullptr, lno);
-        }
-        if (vjp || lno) {
-            __syncthreads();
-            // occupied-energy bar: orbit partials summed per block row (no contended atomics)
-            if (vjp && tid < 3 * T) {
-                const int axis = tid / T, u = tid % T;
-                const int gi = blk[axis] * T + u;
-                double acc = 0.0;
-                for (int r2 = 0; r2 < T2; ++r2) {
-                    const int qq = axis == 0 ? u * T2 + r2 : (axis == 1 ? (r2 / T) * T2 + u * T + r2 % T
-                                                                      : r2 * T + u);
-                    acc += tmp_s[qq];
-                }
-                if (gi < o) atomicAdd(&occ_acc[gi], -acc);
-            }
+    };
+    next(warp >> 1);
+    for (int bo = warp >> 1; bo < nbo; bo += kEpiWarps / 2, next(kEpiWarps / 2)) {
+        const int ijk[3] = {4 * BI + 2 * half + (lane >> 4), 4 * BJ + ((lane >> 2) & 3), 4 * BK + (lane & 3)};
+        const bool mine = ijk[0] < o && ijk[0] >= ijk[1] && ijk[1] >= ijk[2];
+        if (!__any_sync(0xffffffffu, mine)) continue;
+        double tmp = 0.0;
+        if (mine) {
+            int pos[6];
+            bool first[6];
 #pragma unroll
             for (int s = 0; s < 6; ++s) {
-                if (!fresh[s]) continue;
-                const int d = dmap[s];
-                const int p0 = bs[s][0] * T, q0 = bs[s][1] * T, r0 = bs[s][2] * T;
-                for (int sg = 0; sg < (vjp ? 6 : 2); ++sg) {   // LNO: the W and z/D cubes only
-                    ST *dstg = S + sg * o3;
-                    const ST *srcs = Gs + (sg * 6 + d) * BLK;
-                    if (full && sizeof(ST) * T % 16 == 0 && (sizeof(ST) * o) % 16 == 0) {
-                        constexpr int VEC = 16 / sizeof(ST), NV = T3 / VEC;
-                        for (int i = tid; i < NV; i += NTHR) {
-                            const int e3 = i * VEC;
-                            const int u = e3 / T2, ww = (e3 / T) % T, t = e3 % T;
-                            *reinterpret_cast<float4 *>(dstg + ((long long)(p0 + u) * o + q0 + ww) * o + r0 + t) =
-                                *reinterpret_cast<const float4 *>(srcs + L::pidx(e3));
-                        }
-                    } else {
-                        for (int e3 = tid; e3 < T3; e3 += NTHR) {
-                            const int p = p0 + e3 / T2, q = q0 + (e3 / T) % T, r = r0 + e3 % T;
-                            if (p < o && q < o && r < o) dstg[((long long)p * o + q) * o + r] = srcs[L::pidx(e3)];
+                pos[s] = (ijk[kR(s, 0)] * o + ijk[kR(s, 1)]) * o + ijk[kR(s, 2)];
+                bool f = true;
+#pragma unroll
+                for (int t = 0; t < s; ++t) f = f && pos[t] != pos[s];
+                first[s] = f;
+            }
+            const double rden = 1.0 / (eocc[ijk[0]] + eocc[ijk[1]] + eocc[ijk[2]] - eabc);
+            double yb[6], wb[6];
+            if (MODE == E_LNO_BWD) {
+                // (lno_ccsd_t_vjp.c:73-140 on the sorted job's cubes) q = z/D from slot 1,
+                // A and B in two parts from slots 2, 4 and 3, 5: the energy is sum A q,
+                // z_bar = eb A / D, w_bar = eb B + r3(z_bar), v_bar = r3(z_bar)
+                double zb[6], aq = 0.0;
+#pragma unroll
+                for (int s = 0; s < 6; ++s) {
+                    const double q = S[o3 + pos[s]], Ax = S[2 * o3 + pos[s]] + S[4 * o3 + pos[s]];
+                    const double Bx = S[3 * o3 + pos[s]] + S[5 * o3 + pos[s]];
+                    zb[s] = eb * Ax * rden;
+                    wb[s] = eb * Bx;
+                    if (first[s]) aq += Ax * q;
+                }
+                tmp = eb * rden * aq;
+                r3_orbit<double>(zb, yb);
+#pragma unroll
+                for (int s = 0; s < 6; ++s) wb[s] += yb[s];
+            } else {
+                double w6[6], y6[6], z6[6];
+#pragma unroll
+                for (int s = 0; s < 6; ++s) w6[s] = y6[s] = 0.0;
+#pragma unroll
+                for (int sg = 0; sg < 6; ++sg) {
+                    const double *G = S + sg * o3;
+                    double x[6];
+#pragma unroll
+                    for (int q = 0; q < 6; ++q) x[q] = G[pos[q]];
+#pragma unroll
+                    for (int s = 0; s < 6; ++s) w6[s] += x[kComp(s, sg)];
+                }
+                auto add_v = [&](const double (&L)[3][64], const double *const (&base)[6], int ld) {
+                    double u[3][3];
+                    int at[6];
+#pragma unroll
+                    for (int m = 0; m < 3; ++m)
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) u[m][q] = L[m][ijk[q]];
+#pragma unroll
+                    for (int q = 0; q < 6; ++q) at[q] = ijk[kR(q, 0)] * ld + ijk[kR(q, 1)];
+#pragma unroll
+                    for (int sg = 0; sg < 6; ++sg) {
+                        const double *A = base[sg];
+                        double x[6];
+#pragma unroll
+                        for (int q = 0; q < 6; ++q) x[q] = __ldg(A + at[q]);
+#pragma unroll
+                        for (int s = 0; s < 6; ++s) {
+                            const int cs = kComp(s, sg);
+                            y6[s] += x[cs] * u[kR(sg, 2)][kR(cs, 2)];
                         }
                     }
+                };
+                add_v(U, va, n);
+                if (with_fvo) add_v(F, vb, o);
+#pragma unroll
+                for (int s = 0; s < 6; ++s) y6[s] = w6[s] + 0.5 * y6[s];
+                if (MODE == E_T3) {
+                    // the iterative solver's seed (pyscfad/cc/ccsd_t_slow.py:188-220 on the 6-D
+                    // amplitudes): W and W + V are P6(w)[., a, b, c] and P6(w + v)[., a, b, c];
+                    // P6 makes the 6-D arrays invariant under a simultaneous permutation of
+                    // (i, j, k) and (a, b, c), and D under any permutation of either, so
+                    // t3_c[pi(a,b,c)][pi(pos)] = (W + V) / D and t3_x[...] = r3(W) / 3 (the energy
+                    // is sum t3 t3_x, :210-220) for each permutation pi
+                    r3_orbit<double>(w6, z6);
+                    const int abc[3] = {a, b, c};
+#pragma unroll
+                    for (int s = 0; s < 6; ++s) {
+                        const double yc = y6[s] * rden, xr = z6[s] * (1.0 / 3.0);
+#pragma unroll
+                        for (int pi = 0; pi < 6; ++pi) {
+                            const long long ia = ((long long)abc[kR(pi, 0)] * v + abc[kR(pi, 1)]) * v + abc[kR(pi, 2)];
+                            e.t3_c[ia * o3 + pos[kComp(s, pi)]] = yc;
+                            e.t3_x[ia * o3 + pos[kComp(s, pi)]] = xr;
+                        }
+                    }
+                    continue;
                 }
+                r3_orbit<double>(y6, z6);
+                // one reciprocal per orbit: d3 = fac / D; its distinct W.Z products share d3,
+                // so they are summed before the compensated add, and the mo_energy-bar
+                // partial eb d3^2 / fac = eb fac / D^2 reuses 1/D
+                const double d3 = fac * rden;
+                double wz = 0.0;
+#pragma unroll
+                for (int s = 0; s < 6; ++s)
+                    if (first[s]) wz += w6[s] * z6[s];
+                eacc.add(wz * d3);
+                if (MODE == E_LNO_FWD) {
+#pragma unroll
+                    for (int s = 0; s < 6; ++s) {
+                        S[pos[s]] = w6[s];
+                        S[o3 + pos[s]] = z6[s] * rden;
+                    }
+                }
+                if (MODE == E_VJP) {
+                    const double ebd3 = eb * d3;
+                    tmp = eb * d3 * rden * wz;
+                    double zb[6];
+#pragma unroll
+                    for (int s = 0; s < 6; ++s) zb[s] = ebd3 * w6[s];
+                    r3_orbit<double>(zb, yb);
+#pragma unroll
+                    for (int s = 0; s < 6; ++s) wb[s] = ebd3 * z6[s] + yb[s];
+                }
+            }
+            if (BAR) {
+                vir += tmp;
+#pragma unroll
+                for (int s = 0; s < 6; ++s)
+                    if (first[s]) {
+                        S[pos[s]] = wb[s];
+                        S[o3 + pos[s]] = wb[kComp(s, 1)];
+                        S[2 * o3 + pos[s]] = wb[kComp(s, 4)];
+                        S[6 * o3 + pos[s]] = yb[s];
+                    }
+            }
+        }
+        if (BAR) {
+            // occupied mo_energy bar: sums over two of the block's axes (lane bits 0-1 are
+            // k's, 2-3 j's, 4 i's), one axis after the other (blocks may coincide)
+            double s2 = tmp, s1 = tmp, s0;
+            s2 += __shfl_xor_sync(0xffffffffu, s2, 4);
+            s2 += __shfl_xor_sync(0xffffffffu, s2, 8);
+            s2 += __shfl_xor_sync(0xffffffffu, s2, 16);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
+            s0 = s1;
+            s1 += __shfl_xor_sync(0xffffffffu, s1, 16);
+            s0 += __shfl_xor_sync(0xffffffffu, s0, 4);
+            s0 += __shfl_xor_sync(0xffffffffu, s0, 8);
+            if (lane < 4) occ[warp][4 * BK + lane] += s2;
+            __syncwarp();
+            if (lane < 16 && (lane & 3) == 0) occ[warp][4 * BJ + (lane >> 2)] += s1;
+            __syncwarp();
+            if ((lane & 15) == 0) occ[warp][4 * BI + 2 * half + (lane >> 4)] += s0;
+            __syncwarp();
+        }
+    }
+    if (MODE == E_T3) return;
+    // job energy and the virtual mo_energy bar: a fixed shuffle tree per warp, then over the warps
+    ksum_tree(eacc, vir);
+    if (lane == 0) { wred[0][warp] = eacc.s; wred[1][warp] = eacc.c; wred[2][warp] = vir; }
+    __syncthreads();
+    if (warp == 0) {
+        KSum k;
+        k.s = lane < kEpiWarps ? wred[0][lane] : 0.0;
+        k.c = lane < kEpiWarps ? wred[1][lane] : 0.0;
+        double vt = lane < kEpiWarps ? wred[2][lane] : 0.0;
+        ksum_tree(k, vt);
+        if (lane == 0) {
+            const long long amaj = (long long)a * (a + 1) * (a + 2) / 6 + (long long)b * (b + 1) / 2 + c;
+            if (MODE != E_LNO_BWD) e.job_e[amaj] = 2.0 * k.value();   // there the projection kernel's energy stands
+            if (BAR) {
+                atomicAdd(&e.mo_energy_bar[o + a], vt);
+                atomicAdd(&e.mo_energy_bar[o + b], vt);
+                atomicAdd(&e.mo_energy_bar[o + c], vt);
             }
         }
     }
-    __syncthreads();  // last block-orbit done with the G tiles
-    red[tid] = eacc.s;
-    red[NTHR + tid] = eacc.c;
-    red[2 * NTHR + tid] = vir_acc;
-    __syncthreads();
-    if (tid == 0) {
-        KSum tot;
-        double vt = 0.0;
-        for (int t = 0; t < NTHR; ++t) {
-            tot.add(red[t]);
-            tot.add(red[NTHR + t]);
-            vt += red[2 * NTHR + t];
-        }
-        const long long amaj = (long long)a * (a + 1) * (a + 2) / 6 + (long long)b * (b + 1) / 2 + c;
-        if (!lbar) e.job_e[amaj] = 2.0 * tot.value();   // LNO: the projection kernel's energy stands
-        if (vjp) {
-            atomicAdd(&e.mo_energy_bar[o + a], vt);
-            atomicAdd(&e.mo_energy_bar[o + b], vt);
-            atomicAdd(&e.mo_energy_bar[o + c], vt);
-        }
+    if (BAR && tid < o) {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < kEpiWarps; ++q) s += occ[q][tid];
+        atomicAdd(&e.mo_energy_bar[tid], -s);
     }
-    if (vjp)
-        for (int i = tid; i < o; i += NTHR) atomicAdd(&e.mo_energy_bar[i], occ_acc[i]);
 }
 
 // V-term bars of one job.  With Vbar_sigma[p,q,r] = ybar[idx_sigma(p,q,r)]:
@@ -687,25 +441,22 @@ static cudaError_t launch_vterm(const WaveView &w, const EpiArgs &e, const ST *s
     return cudaGetLastError();
 }
 
-template <typename ST, int T, typename VT, int NTHR, int WB, bool T3M>
-static cudaError_t launch_epi(const WaveView &w, const EpiArgs &e, ST *scratch, cudaStream_t st) {
+cudaError_t f64_epilogue(const WaveView &w, const EpiArgs &e, double *scratch, cudaStream_t st) {
     if (w.n_jobs <= 0) return cudaSuccess;
     if (e.o > 64) return cudaErrorInvalidValue;
-    const size_t smem = EpiSmem<ST, T, VT>::bytes(NTHR);
-    {
-        cudaError_t ce = smem_optin(reinterpret_cast<const void *>(epi_kernel<ST, T, VT, NTHR, WB, T3M>), (int)smem);
-        if (ce != cudaSuccess) return ce;
-    }
-    epi_kernel<ST, T, VT, NTHR, WB, T3M><<<w.n_jobs, NTHR, smem, st>>>(w, e, scratch);
-    return cudaGetLastError();
-}
-
-cudaError_t f64_epilogue(const WaveView &w, const EpiArgs &e, double *scratch, cudaStream_t st) {
+    const dim3 grid(w.n_jobs), block(kEpiThreads);
     if (e.t3_c) {
         if (!e.t3_x || e.with_vjp) return cudaErrorInvalidValue;
-        return launch_epi<double, 4, double, 64, 0, true>(w, e, scratch, st);
+        epi_kernel<E_T3><<<grid, block, 0, st>>>(w, e, scratch);
+    } else if (e.with_vjp) {
+        if (e.lno_phase == 2) epi_kernel<E_LNO_BWD><<<grid, block, 0, st>>>(w, e, scratch);
+        else epi_kernel<E_VJP><<<grid, block, 0, st>>>(w, e, scratch);
+    } else if (e.lno_phase == 1) {
+        epi_kernel<E_LNO_FWD><<<grid, block, 0, st>>>(w, e, scratch);
+    } else {
+        epi_kernel<E_ENERGY><<<grid, block, 0, st>>>(w, e, scratch);
     }
-    return launch_epi<double, 4, double, 64, 0, false>(w, e, scratch, st);
+    return cudaGetLastError();
 }
 
 cudaError_t f64_vterm(const WaveView &w, const EpiArgs &e, const double *scratch, cudaStream_t st) {

@@ -53,25 +53,50 @@ cudaError_t smem_optin(const void *kernel, int bytes) {
     return cudaSuccess;
 }
 
+// The float64 path that keeps a job's cube in shared memory (ct_cube.cu): its
+// largest cube, V tiles and partials take 193 KB at nocc = 24.  nocc = 1 stays
+// on the slot path (a cube of one element).
+static bool cube_size(int o) { return o >= 2 && o <= kCubeMaxO; }
+
 struct Plan {
     int o = 0, v = 0, max_wave = 0;
     std::vector<int> jobs, wave_begin, tb_entries, tb_groups, tb_group_begin;
     std::vector<int> zchunks, zchunk_begin, x_entries, xgroups, xgroup_begin, xchunks, xchunk_begin;
     std::vector<int> ochunks, ochunk_begin;
+    std::vector<int> zparts, zpart_begin, xparts, xpart_begin;   // float64 path
     int *d_jobs = nullptr, *d_tb_entries = nullptr, *d_tb_groups = nullptr;
     int *d_zchunks = nullptr, *d_x_entries = nullptr, *d_xgroups = nullptr, *d_xchunks = nullptr;
-    int *d_ochunks = nullptr;
+    int *d_ochunks = nullptr, *d_zparts = nullptr, *d_xparts = nullptr;
     int n_waves() const { return (int)wave_begin.size() - 1; }
     void free_dev() {
         if (d_jobs) cudaFree(d_jobs);
         if (d_tb_entries) cudaFree(d_tb_entries);
         if (d_tb_groups) cudaFree(d_tb_groups);
-        for (int *q : {d_zchunks, d_x_entries, d_xgroups, d_xchunks, d_ochunks})
+        for (int *q : {d_zchunks, d_x_entries, d_xgroups, d_xchunks, d_ochunks, d_zparts, d_xparts})
             if (q) cudaFree(q);
         d_jobs = d_tb_entries = d_tb_groups = nullptr;
-        d_zchunks = d_x_entries = d_xgroups = d_xchunks = d_ochunks = nullptr;
+        d_zchunks = d_x_entries = d_xgroups = d_xchunks = d_ochunks = d_zparts = d_xparts = nullptr;
     }
 };
+
+// Cuts a wave's groups (key, e0, e1) into parts of about equal length, at least
+// 16 terms, so that parts x tiles make about 64 CTAs per SM.  The groups of one
+// wave differ widely (in a slab block of nocc=48/nvir=300 two thirds of the terms
+// meet the six slab indices, the rest a hundred others), so parts of equal length
+// and not equal numbers of parts per group keep the last round short.
+static void cut_parts(const std::vector<int> &groups, int g0, int g1, long long tiles, std::vector<int> &parts) {
+    long long terms = 0;
+    for (int g = g0; g < g1; ++g) terms += groups[3 * g + 2] - groups[3 * g + 1];
+    const long long len = std::max<long long>(16, terms * tiles / (64 * 148));
+    for (int g = g0; g < g1; ++g) {
+        const long long e0 = groups[3 * g + 1], ne = groups[3 * g + 2] - e0, np = (ne + len - 1) / len;
+        for (long long q = 0; q < np; ++q) {
+            parts.push_back(groups[3 * g]);
+            parts.push_back((int)(e0 + ne * q / np));
+            parts.push_back((int)(e0 + ne * (q + 1) / np));
+        }
+    }
+}
 
 // Fill waves/TB groups of a plan from super-blocks (each a list of jobs).
 static void finish_plan(Plan &P, const std::vector<std::vector<int>> &blocks) {
@@ -140,6 +165,8 @@ static void finish_plan(Plan &P, const std::vector<std::vector<int>> &blocks) {
     P.x_entries.clear(); P.xgroups.clear(); P.xgroup_begin.assign(1, 0);
     P.xchunks.clear(); P.xchunk_begin.assign(1, 0);
     P.ochunks.clear(); P.ochunk_begin.assign(1, 0);
+    P.zparts.clear(); P.zpart_begin.assign(1, 0);
+    P.xparts.clear(); P.xpart_begin.assign(1, 0);
     for (int w = 0; w < P.n_waves(); ++w) {
         for (int g = P.tb_group_begin[w]; g < P.tb_group_begin[w + 1]; ++g) {
             const int z = P.tb_groups[3 * g], e0 = P.tb_groups[3 * g + 1], e1 = P.tb_groups[3 * g + 2];
@@ -190,6 +217,13 @@ static void finish_plan(Plan &P, const std::vector<std::vector<int>> &blocks) {
                 }
             }
         P.xgroup_begin.push_back((int)P.xgroups.size() / 3);
+        // tiles of the kernels that take the parts: cube_tb / TB and OB1 of ct_pair.cu
+        const long long oo = (long long)P.o * P.o, fz = (P.v + 63) / 64;
+        cut_parts(P.tb_groups, P.tb_group_begin[w], P.tb_group_begin[w + 1],
+                  fz * (cube_size(P.o) ? (oo + 63) / 64 : (oo + 127) / 128), P.zparts);
+        P.zpart_begin.push_back((int)P.zparts.size() / 3);
+        cut_parts(P.xgroups, P.xgroup_begin[w], P.xgroup_begin[w + 1], (oo + 127) / 128, P.xparts);
+        P.xpart_begin.push_back((int)P.xparts.size() / 3);
         P.xchunk_begin.push_back((int)P.xchunks.size() / 3);
         P.ochunk_begin.push_back((int)P.ochunks.size() / 3);
     }
@@ -215,6 +249,8 @@ static int upload_plan(Plan &P) {
     CT_CK(up(&P.d_xgroups, P.xgroups));
     CT_CK(up(&P.d_xchunks, P.xchunks));
     CT_CK(up(&P.d_ochunks, P.ochunks));
+    CT_CK(up(&P.d_zparts, P.zparts));
+    CT_CK(up(&P.d_xparts, P.xparts));
     return CT_OK;
 }
 
@@ -502,10 +538,7 @@ static double scratch_budget_mb(Workspace &W) {
     return W.budget_mb;
 }
 
-// The float64 path that keeps a job's cube in shared memory (ct_cube.cu): its
-// largest cube, V tiles and partials take 193 KB at nocc = 24.  nocc = 1 stays
-// on the slot path (a cube of one element).
-static bool use_cube(int o, int mode) { return mode == CT_MODE_FP64 && o >= 2 && o <= kCubeMaxO; }
+static bool use_cube(int o, int mode) { return mode == CT_MODE_FP64 && cube_size(o); }
 
 // Jobs per wave: as many as the scratch budget holds (at most 8192), rounded
 // down to a multiple of two CTAs per SM so the per-job kernels fill whole
@@ -632,6 +665,10 @@ static int run_waves(Workspace &W, const Plan &P, const ct_problem *p, int mode,
         wv.xgroups = P.d_xgroups + 3 * P.xgroup_begin[w];
         wv.n_xchunks = P.xchunk_begin[w + 1] - P.xchunk_begin[w];
         wv.xchunks = P.d_xchunks + 3 * P.xchunk_begin[w];
+        wv.n_zparts = P.zpart_begin[w + 1] - P.zpart_begin[w];
+        wv.zparts = P.d_zparts + 3 * P.zpart_begin[w];
+        wv.n_xparts = P.xpart_begin[w + 1] - P.xpart_begin[w];
+        wv.xparts = P.d_xparts + 3 * P.xpart_begin[w];
         wv.n_ochunks = P.ochunk_begin[w + 1] - P.ochunk_begin[w];
         wv.ochunks = P.d_ochunks + 3 * P.ochunk_begin[w];
         if (cube) {
@@ -655,11 +692,13 @@ static int run_waves(Workspace &W, const Plan &P, const ct_problem *p, int mode,
                 CT_PROF(PK_F1);
                 CT_CK(cube_vjp(wv, ea, p->vooo, g->vooo, S, st));
             }
-            { CT_PROF(PK_TB); CT_CK(cube_tb(wv, ea, S, stride, W.sm_count, st)); }
+            { CT_PROF(PK_TB); CT_CK(cube_tb(wv, ea, S, stride, st)); }
         } else if (mode == CT_MODE_FP64) {
             double *S = (double *)W.scratch;
-            { CT_PROF(PK_F1); CT_CK(f64_gemm(K_F1, wv, p->t2T, p->vvop, S, S, st)); }
-            { CT_PROF(PK_F2); CT_CK(f64_gemm(K_F2, wv, p->vooo, p->t2T, S, S, st)); }
+            auto gemm = [&](GemmKind k, double *out) {
+                return f64_gemm(k, wv, p->t2T, p->vooo, p->vvop, S, out, st);
+            };
+            { CT_PROF(PK_F1); CT_CK(gemm(K_W, nullptr)); }
             if (lno_mat && vjp) {
                 // LNO VJP: forward pass (W, z/D cubes), projections A, B with the
                 // energy and mat_bar partials, backward pass (W-bar, ybar), then
@@ -677,10 +716,10 @@ static int run_waves(Workspace &W, const Plan &P, const ct_problem *p, int mode,
             }
             if (vjp) {
                 { CT_PROF(PK_VT); CT_CK(f64_vterm(wv, ea, S, st)); }
-                { CT_PROF(PK_VB); CT_CK(f64_gemm(K_VB, wv, p->t2T, S, g->vvop, S, st)); }
-                { CT_PROF(PK_TB); CT_CK(f64_gemm(K_TB, wv, p->vvop, S, g->t2T, S, st)); }
-                { CT_PROF(PK_OB1); CT_CK(f64_gemm(K_OB1, wv, S, p->t2T, g->vooo, S, st)); }
-                { CT_PROF(PK_OB2); CT_CK(f64_gemm(K_OB2, wv, p->vooo, S, g->t2T, S, st)); }
+                { CT_PROF(PK_VB); CT_CK(gemm(K_VB, g->vvop)); }
+                { CT_PROF(PK_TB); CT_CK(gemm(K_TB, g->t2T)); }
+                { CT_PROF(PK_OB1); CT_CK(gemm(K_OB1, g->vooo)); }
+                { CT_PROF(PK_OB2); CT_CK(gemm(K_OB2, g->t2T)); }
             }
         } else {
             ProfCtx pc{&W, st};

@@ -6,8 +6,8 @@
 
 namespace ctb {
 
-// GEMM kinds of one wave (offsets per (job, sigma) term; see entry_offsets)
-enum GemmKind { K_F1 = 0, K_F2 = 1, K_VB = 2, K_TB = 3, K_OB1 = 4, K_OB2 = 5 };
+// float64 GEMM kinds of one wave (ct_pair.cu)
+enum GemmKind { K_W = 0, K_VB, K_TB, K_OB1, K_OB2 };
 
 struct WaveView {
     int o, v, n;
@@ -27,6 +27,12 @@ struct WaveView {
     const int *xchunks;
     int n_ochunks;        // x-sorted terms in chunks of <= 256 / o (OB2)
     const int *ochunks;
+    // float64 path: the groups by z (into tb_entries) and by x (into x_entries)
+    // cut into parts of about equal length, (key, e_begin, e_end) each
+    int n_zparts;
+    const int *zparts;
+    int n_xparts;
+    const int *xparts;
 };
 
 struct EpiArgs {
@@ -75,13 +81,16 @@ cudaError_t smem_optin(const void *kernel, int bytes);
 enum ProfKind { PK_F1 = 0, PK_F2, PK_EPI, PK_VT, PK_VB, PK_TB, PK_OB1, PK_OB2, PK_RED,
                 PK_MPREP, PK_MF, PK_MVB, PK_MTB, PK_MOO, PK_MOB1, PK_MOB2, kProfKinds };
 
-// scratch layout per job: 7 slots of o^3 (slots 0..5: G_sigma then Wbar_sigma,
-// slot 6: ybar = r3^T(zbar))
+// scratch layout per job: 7 slots of o^3 (slots 0..5: G_sigma, then Wbar_sigma on the
+// mixed path and the three w-bar cubes in slots 0..2 on the float64 path; slot 6:
+// ybar = r3^T(zbar))
 constexpr int kSlots = 7;
 
-// float64 path (ct_fp64.cu)
-cudaError_t f64_gemm(GemmKind kind, const WaveView &w, const double *A, const double *B, double *C,
-                     double *scratch, cudaStream_t st);
+// float64 slot path: GEMMs (ct_pair.cu; nocc <= 64) from the inputs and the wave's
+// slots into the slots (K_W) or `out`, the gradient the kind adds to (vvop_bar for
+// K_VB, t2T_bar for K_TB and K_OB2, vooo_bar for K_OB1); epilogue and V terms (ct_fp64.cu)
+cudaError_t f64_gemm(GemmKind kind, const WaveView &w, const double *t2T, const double *vooo, const double *vvop,
+                     double *slots, double *out, cudaStream_t st);
 cudaError_t f64_epilogue(const WaveView &w, const EpiArgs &e, double *scratch, cudaStream_t st);
 cudaError_t f64_vterm(const WaveView &w, const EpiArgs &e, const double *scratch, cudaStream_t st);
 // float64 path for 2 <= nocc <= kCubeMaxO (ct_cube.cu): one CTA per job with its
@@ -98,8 +107,7 @@ cudaError_t cube_lno_forward(const WaveView &w, const EpiArgs &e, const double *
                              cudaStream_t st);
 cudaError_t cube_lno_backward(const WaveView &w, const EpiArgs &e, const double *vooo, double *vooo_bar,
                               double *slots, cudaStream_t st);
-cudaError_t cube_tb(const WaveView &w, const EpiArgs &e, const double *cubes, long long stride, int sms,
-                    cudaStream_t st);
+cudaError_t cube_tb(const WaveView &w, const EpiArgs &e, const double *cubes, long long stride, cudaStream_t st);
 // LNO projections (ct_lno.cu).  The energy of each job of the wave from the
 // W and z/D cubes the epilogue leaves in slots 0 and 1 (writes e.job_e)
 cudaError_t f64_lno_contract(const WaveView &w, const EpiArgs &e, const double *scratch, cudaStream_t st);

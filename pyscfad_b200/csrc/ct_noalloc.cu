@@ -91,8 +91,7 @@ extern "C" int ct_energy_noalloc(const ct_problem *p, double *e_out, void *strea
         wv.o = (int)o; wv.v = (int)v; wv.n = (int)(o + v);
         wv.n_jobs = count;
         wv.jobs = jobs;
-        if (f64_gemm(K_F1, wv, p->t2T, p->vvop, scratch, scratch, st) != cudaSuccess) return CT_ERR_CUDA;
-        if (f64_gemm(K_F2, wv, p->vooo, p->t2T, scratch, scratch, st) != cudaSuccess) return CT_ERR_CUDA;
+        if (f64_gemm(K_W, wv, p->t2T, p->vooo, p->vvop, scratch, nullptr, st) != cudaSuccess) return CT_ERR_CUDA;
         if (f64_epilogue(wv, ea, scratch, st) != cudaSuccess) return CT_ERR_CUDA;
     }
     if (reduce_energy_1cta(job_e, njobs, e_out, st) != cudaSuccess) return CT_ERR_CUDA;
