@@ -42,6 +42,7 @@
 // into CT_ERR_TIMEOUT.
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cuda_bf16.h>
 #include <cstdio>
 #include <cstdlib>
@@ -222,6 +223,11 @@ __device__ __forceinline__ void issue_loads(const TcParams &P, const Work &W, in
             if (PREC) tc::tma_load_3d(sB + P.b_bytes + off, &P.mapB2, bar, c0, c1, c2);
         }
     };
+    // all chunks of an MN-major operand as one box (CK, K rows, chunks) of term row c3
+    auto ld4 = [&](uint32_t dst, int plane, const CUtensorMap *m, const CUtensorMap *m2, int chunk0, int c3) {
+        tc::tma_load_4d(dst, m, bar, 0, 0, chunk0, c3);
+        if (PREC) tc::tma_load_4d(dst + plane, m2, bar, 0, 0, chunk0, c3);
+    };
     // bytes: per plane
     auto arm = [&](uint32_t bytes) {
         if (lane == 0) tc::mbar_expect_tx(bar, NP * bytes);
@@ -256,10 +262,10 @@ __device__ __forceinline__ void issue_loads(const TcParams &P, const Work &W, in
     case TK_TB: {
         const int kp = PREC ? (o + 15) / 16 * 16 : o;   // K rows (p) of one term, zero-filled past o
         constexpr int nca = 128 / CK;
-        const int nch = W.N / CK;
+        const int nch = P.tb_n / CK;                    // chunks past o^2 are zero-filled
         arm((uint32_t)(nca + nch) * kp * 128u);
-        if (lane < nca) ldA(lane * kp * 128, W.mt * 128 + CK * lane, 0, mine.p0);
-        else if (lane < nca + nch) ldB((lane - nca) * kp * 128, W.nt * P.tb_n + CK * (lane - nca), 0, mine.p1);
+        if (lane == 0) ld4(sA, P.a_bytes, &P.mapA, &P.mapA2, W.mt * nca, mine.p0);
+        if (lane == 1) ld4(sB, P.b_bytes, &P.mapB, &P.mapB2, W.nt * nch, mine.p1);
         break;
     }
     case TK_F2: {
@@ -279,8 +285,8 @@ __device__ __forceinline__ void issue_loads(const TcParams &P, const Work &W, in
         const int kr8 = PREC ? (o + 15) / 16 * 16 : (o + 7) / 8 * 8, nkc = (kr8 + CK - 1) / CK;
         constexpr int nca = 128 / CK;
         arm((uint32_t)nca * kr8 * 128u + (uint32_t)nkc * o * 128u);
-        if (lane < nca) ldA(lane * kr8 * 128u, W.mt * 128 + CK * lane, 0, mine.p1);
-        else if (lane < nca + nkc) ldB((lane - nca) * o * 128u, CK * (lane - nca), 0, mine.p0);
+        if (lane == 0) ld4(sA, P.a_bytes, &P.mapA, &P.mapA2, W.mt * nca, mine.p1);
+        else if (lane <= nkc) ldB((lane - 1) * o * 128u, CK * (lane - 1), 0, mine.p0);
         break;
     }
     default: {  // TK_OB2
@@ -1317,14 +1323,19 @@ static int mixed_wave_p(const WaveView &w, const EpiArgs &e, const ct_grads *g, 
         // ---- TB: D[f,qr], A = vvf (f,p,xy) MN-major, B = Wbar (qr,p,slot) MN-major
         {
             TcParams P = base;
-            if (!make_maps(&P.mapA, &P.mapA2, vv, vp, o, (long long)v * v, vp, (long long)o * vp, CK, kp, true, PREC))
-                return CT_ERR_CUDA;
-            if (!make_maps(&P.mapB, &P.mapB2, Wb, o2, o, wn, o2, ws, CK, kp, true, PREC)) return CT_ERR_CUDA;
             P.m_tiles = (v + 127) / 128;
             // items of 256 columns; of 128 where those would leave SMs without one
             // (few virtuals and a small o^2): the same sums per element either way
             P.tb_n = w.n_tb_groups * P.m_tiles * (int)((o2 + 255) / 256) < md().sms ? 128 : 256;
             P.n_tiles = (int)((o2 + P.tb_n - 1) / P.tb_n);
+            // a row's last chunk runs into the next row (and past the last row into the
+            // vooo copy): virtuals past v, whose output rows are not stored
+            const long long dA[4] = {std::min(vp, CK), o, (vp + CK - 1) / CK, (long long)v * v};
+            const long long sA[3] = {vp, CK, (long long)o * vp};
+            const long long dB[4] = {CK, o, o2 / CK, wn}, sB[3] = {o2, CK, ws};
+            const int bA[4] = {CK, kp, 128 / CK, 1}, bB[4] = {CK, kp, P.tb_n / CK, 1};
+            if (!make_maps_nd(&P.mapA, &P.mapA2, vv, 4, dA, sA, bA, true, PREC)) return CT_ERR_CUDA;
+            if (!make_maps_nd(&P.mapB, &P.mapB2, Wb, 4, dB, sB, bB, true, PREC)) return CT_ERR_CUDA;
             P.groups = w.tb_groups; P.entries = w.tb_entries;
             P.nwork = w.n_tb_groups * P.m_tiles * P.n_tiles;
             P.out = g->t2T;
@@ -1338,7 +1349,9 @@ static int mixed_wave_p(const WaveView &w, const EpiArgs &e, const ct_grads *g, 
         {
             TcParams P = base;
             const int kr8 = PREC ? (o + 15) / 16 * 16 : (o + 7) / 8 * 8;   // K rows: whole k-steps
-            if (!make_maps(&P.mapA, &P.mapA2, Wb, o2, o, wn, o2, ws, CK, kr8, true, PREC)) return CT_ERR_CUDA;
+            const long long dA[4] = {CK, o, o2 / CK, wn}, sA[3] = {o2, CK, ws};
+            const int bA[4] = {CK, kr8, 128 / CK, 1};
+            if (!make_maps_nd(&P.mapA, &P.mapA2, Wb, 4, dA, sA, bA, true, PREC)) return CT_ERR_CUDA;
             if (!make_maps(&P.mapB, &P.mapB2, t2, o, o, (long long)v * v, o, o2, CK, o, false, PREC)) return CT_ERR_CUDA;
             P.m_tiles = (int)((o2 + 127) / 128);
             P.groups = w.xgroups; P.entries = w.x_entries;

@@ -46,12 +46,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // Bounded wait on an mbarrier phase: gives up after ~2 s (or as soon as another
 // thread has flagged an error), sets *err and returns false.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *err) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = global_ns();
+    uint64_t t0 = 0;
     for (uint32_t i = 0;; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((i & 255) == 255) {
             if (*(volatile int *)err) return false;
+            if (t0 == 0) t0 = global_ns();
             if (global_ns() - t0 > 2000000000ull) {
                 atomicExch(err, 1);
                 return false;
