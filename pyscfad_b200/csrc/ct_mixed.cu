@@ -315,78 +315,78 @@ __device__ __forceinline__ void issue_loads(const TcParams &P, const Work &W, in
 // instruction, MN-major operands in the plain 128-B swizzle (8-row atoms, SBO
 // 1024); three MMAs per k-step (hi*hi, hi*lo, lo*hi).  K-major operands: 128-B
 // swizzle, SBO 1024, +32 bytes per k-step in both.
-template <int KIND, int PREC, bool CG2 = false>
-__device__ __forceinline__ void issue_mmas(const TcParams &P, const Work &W, int kit, uint32_t sA, uint32_t tacc,
-                                           bool first) {
+// A descriptor holds its address in 16-byte units in its low bits (below 2^14:
+// shared memory ends before a carry), so stages and k-steps are additions to the
+// descriptors of the first stage; the one issuing thread built two descriptors
+// per MMA before.
+struct MmaOps {
+    uint64_t a, b;        // first stage, first k-step (hi planes)
+    uint32_t da, db;      // steps per k-step
+    uint32_t lo_a, lo_b;  // distance of the lo planes (BF16x3)
+    int ksteps;           // k-steps of a stage
+};
+template <int KIND, int PREC>
+__device__ __forceinline__ MmaOps mma_ops(const TcParams &P, uint32_t sbase) {
     constexpr int CK = PREC ? 64 : 32;
     constexpr int KS = PREC ? 16 : 8;                    // K per MMA
     constexpr uint32_t MN_SBO = PREC ? 1024u : 512u;
     constexpr uint32_t MN_LAYOUT = PREC ? tc::kSw128 : tc::kSw128Base32;
     constexpr uint32_t MN_STEP = KS * 128u;              // bytes per k-step along K rows
-    constexpr uint32_t NP = PREC ? 2u : 1u;
-    const int o = P.o;
-    const uint32_t sB = sA + NP * (uint32_t)P.a_bytes;
-    const uint32_t chunk = (uint32_t)CK * 128u;
-    int ksteps = CK / KS;
-    // K = l (F2) runs past o in the last chunk: its zero-filled k-steps are
-    // not issued
-    if (KIND == TK_F2) {
-        const int valid = o - CK * kit < CK ? o - CK * kit : CK;
-        ksteps = (valid + KS - 1) / KS;
-    }
-    // OB1: one stage holds all of K = r (kr8 rows of A; B in CK-wide K chunks of o rows)
-    const int kr8 = PREC ? (o + 15) / 16 * 16 : (o + 7) / 8 * 8;
-    if (KIND == TK_OB1) ksteps = (kr8 + KS - 1) / KS;
-    bool amn, bmn;
-    uint32_t a_lbo, b_lbo;
-    switch (KIND) {
-    case TK_F1: amn = false; bmn = false; a_lbo = 16; b_lbo = 16; break;
-    case TK_VB: amn = false; bmn = false; a_lbo = 16; b_lbo = 16; break;
-    case TK_TB: {
-        const int kp = PREC ? (o + 15) / 16 * 16 : o;
-        ksteps = kp / KS; amn = true; bmn = true; a_lbo = kp * 128; b_lbo = kp * 128;
-        break;
-    }
-    case TK_F2: amn = false; bmn = true; a_lbo = 16; b_lbo = chunk; break;
-    case TK_OB1: amn = true; bmn = false; a_lbo = kr8 * 128; b_lbo = 16; break;
-    default: amn = true; bmn = false; a_lbo = chunk; b_lbo = 16; break;   // OB2
-    }
-    // CTA pair: M = 256 (128 rows in each CTA), B rows split between the CTAs
-    const uint32_t id = tc::idesc(PREC ? 1 : 2, CG2 ? 256 : 128, W.N, amn, bmn);
-    // K-major k-step kk: 32 bytes along a 128-byte row; OB1's B has one such
-    // row block (o rows) per CK of K
-    auto desc = [&](uint32_t base, bool mn, uint32_t lbo, int kk) {
-        if (mn) return tc::sdesc(base + kk * MN_STEP, lbo, MN_SBO, MN_LAYOUT);
-        if (KIND == TK_OB1) {
-            constexpr int KPC = CK / KS;   // k-steps per 128-byte row
-            return tc::sdesc(base + (kk / KPC) * (uint32_t)o * 128u + (kk % KPC) * 32u, lbo, 1024);
-        }
-        return tc::sdesc(base + kk * 32u, lbo, 1024);
-    };
+    constexpr uint32_t chunk = (uint32_t)CK * 128u;
+    constexpr bool amn = KIND == TK_TB || KIND == TK_OB1 || KIND == TK_OB2, bmn = KIND == TK_TB || KIND == TK_F2;
+    const uint32_t o = (uint32_t)P.o;
+    // K rows of a TB / OB1 stage (all of p or r, in whole k-steps)
+    const uint32_t kr = KIND == TK_TB ? (PREC ? (o + 15) / 16 * 16 : o) : (o + KS - 1) / KS * KS;
+    const uint32_t a_lbo = !amn ? 16u : (KIND == TK_OB2 ? chunk : kr * 128u);
+    const uint32_t b_lbo = !bmn ? 16u : (KIND == TK_F2 ? chunk : kr * 128u);
+    const uint32_t sB = sbase + (PREC ? 2u : 1u) * (uint32_t)P.a_bytes;
+    MmaOps M;
+    M.a = amn ? tc::sdesc(sbase, a_lbo, MN_SBO, MN_LAYOUT) : tc::sdesc(sbase, a_lbo, 1024);
+    M.b = bmn ? tc::sdesc(sB, b_lbo, MN_SBO, MN_LAYOUT) : tc::sdesc(sB, b_lbo, 1024);
+    M.da = (amn ? MN_STEP : 32u) >> 4;
+    M.db = (bmn ? MN_STEP : 32u) >> 4;
+    M.lo_a = (uint32_t)P.a_bytes >> 4;
+    M.lo_b = (uint32_t)P.b_bytes >> 4;
+    M.ksteps = KIND == TK_TB || KIND == TK_OB1 ? (int)kr / KS : CK / KS;
+    return M;
+}
+
+// off: the stage's offset in 16-byte units; id: instruction descriptor of the item
+template <int KIND, int PREC, bool CG2 = false>
+__device__ __forceinline__ void issue_mmas(const TcParams &P, const MmaOps &M, uint32_t id, int kit, uint32_t off,
+                                           uint32_t tacc, bool first) {
+    constexpr int CK = PREC ? 64 : 32, KS = PREC ? 16 : 8;
+    int ksteps = M.ksteps;
+    // K = l (F2) runs past o in the last chunk: its zero-filled k-steps are not issued
+    if (KIND == TK_F2) ksteps = min(ksteps, (P.o - CK * kit + KS - 1) / KS);
+    uint64_t da = M.a + off, db = M.b + off;
+    uint32_t acc = first ? 0u : 1u;
+#pragma unroll 4
     for (int kk = 0; kk < ksteps; ++kk) {
-        const uint64_t da = desc(sA, amn, a_lbo, kk), db = desc(sB, bmn, b_lbo, kk);
-        const uint32_t acc = (first && kk == 0) ? 0u : 1u;
         if (CG2) {
             if (PREC) {
-                const uint64_t da2 = desc(sA + P.a_bytes, amn, a_lbo, kk), db2 = desc(sB + P.b_bytes, bmn, b_lbo, kk);
                 tc::mma_f16_cg2(tacc, da, db, id, acc);
-                tc::mma_f16_cg2(tacc, da, db2, id, 1u);
-                tc::mma_f16_cg2(tacc, da2, db, id, 1u);
+                tc::mma_f16_cg2(tacc, da, db + M.lo_b, id, 1u);
+                tc::mma_f16_cg2(tacc, da + M.lo_a, db, id, 1u);
             } else {
                 tc::mma_tf32_cg2(tacc, da, db, id, acc);
             }
         } else if (paired(KIND, PREC)) {
             // second M-tile: A rows at +16 KB, accumulator in TMEM columns 256..
             tc::mma_tf32(tacc, da, db, id, acc);
-            tc::mma_tf32(tacc + 256u, desc(sA + 16384u, amn, a_lbo, kk), db, id, acc);
+            tc::mma_tf32(tacc + 256u, da + (16384u >> 4), db, id, acc);
         } else if (PREC) {
-            const uint64_t da2 = desc(sA + P.a_bytes, amn, a_lbo, kk), db2 = desc(sB + P.b_bytes, bmn, b_lbo, kk);
             tc::mma_f16(tacc, da, db, id, acc);
-            tc::mma_f16(tacc, da, db2, id, 1u);
-            tc::mma_f16(tacc, da2, db, id, 1u);
+            tc::mma_f16(tacc, da, db + M.lo_b, id, 1u);
+            tc::mma_f16(tacc, da + M.lo_a, db, id, 1u);
         } else {
             tc::mma_tf32(tacc, da, db, id, acc);
         }
+        acc = 1u;
+        da += M.da;
+        db += M.db;
+        // OB1's B is K-major with one row block (o rows of 128 bytes) per CK of K
+        if (KIND == TK_OB1 && (kk + 1) % (CK / KS) == 0) db += (uint32_t)P.o * 8u - 8u;
     }
 }
 
@@ -667,22 +667,22 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
         Work W = get_work(cid), W1 = get_work(cid + ncl), W2 = get_work(cid + 2 * ncl);
         int eid = get_entry(W, 0), eid1 = get_entry(W1, 0);
         int job = P.jobs[eid / 6];
-        int it = 0;
+        int s = 0, issued = 0;
+        uint32_t ph = 1;   // phase of the empty barrier waited for: the first round's is complete from the start
         bool ok = true;
         for (int w = cid; w < P.nwork && ok; w += ncl) {
             const Work W3 = get_work(w + 3 * ncl);
             const int eid2 = get_entry(W2, 0), job1 = P.jobs[eid1 / 6];
             TermOps mine = term_ops<KIND, PREC>(P, eid, job);
             int eidb = 0, jobb = 0;   // TB, OB1: the next 32 terms of this item
-            for (int kit = 0; kit < W.nk; ++kit, ++it) {
+            for (int kit = 0; kit < W.nk; ++kit) {
                 if (PER_STAGE) {
                     const int u = kit & 31;
                     if (kit > 0 && u == 0) mine = term_ops<KIND, PREC>(P, eidb, jobb);
                     if (u == 0) eidb = get_entry(W, kit + 32);
                     if (u == 16) jobb = P.jobs[eidb / 6];
                 }
-                const int s = it % S;
-                if (it >= S && !tc::mbar_wait(bar(kBarEmpty + s), ((it / S) - 1) & 1, err)) ok = false;
+                if (!tc::mbar_wait(bar(kBarEmpty + s), ph, err)) ok = false;
                 if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
                 TermOps T = mine;
                 if (PER_STAGE) {
@@ -691,6 +691,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
                 }
                 issue_loads<KIND, PREC, CG2>(P, W, kit, sbase + s * P.stage_bytes, bar(s), T, lane, rank,
                                              CG2 ? tc::mapa(bar(s), 0) : 0u);
+                ++issued;
+                if (++s == S) { s = 0; ph ^= 1u; }
             }
             W = W1; W1 = W2; W2 = W3;
             eid = eid1; eid1 = eid2;
@@ -699,31 +701,34 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
         // drain: every issued copy has landed before this CTA can exit (on
         // a CTA pair the leader's full barriers count the copies of both)
         if (rank == 0 && lane == 0) {
-            const int issued = it;
             for (int k = issued - 1; k >= 0 && k >= issued - S; --k)
                 tc::mbar_wait(bar(k % S), (k / S) & 1, err);
         }
         __syncwarp();
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
-            int it = 0, wi = 0;
+            constexpr bool amn = KIND == TK_TB || KIND == TK_OB1 || KIND == TK_OB2, bmn = KIND == TK_TB || KIND == TK_F2;
+            const MmaOps M = mma_ops<KIND, PREC>(P, sbase);
+            int s = 0, wi = 0;
+            uint32_t ph = 0;   // stage and its phase, stepped (a division by S each stage cost more than its MMAs)
             bool ok = true;
             for (int w = cid; w < P.nwork && ok; w += ncl, ++wi) {
                 Work W;
                 decode<KIND, PREC>(P, w, W);
+                // CTA pair: M = 256 (128 rows in each CTA), B rows split between the CTAs
+                const uint32_t id = tc::idesc(PREC ? 1 : 2, CG2 ? 256 : 128, W.N, amn, bmn);
                 // paired kinds use both TMEM halves for one item: single-buffered
                 const int buf = PAIRED ? 0 : (wi & 1), use = PAIRED ? wi : (wi >> 1);
                 if (use > 0 && !tc::mbar_wait(bar(kBarAccEmpty + buf), (use - 1) & 1, err)) break;
                 tc::fence_after();
                 const uint32_t tacc = tmem + (uint32_t)(buf * 256);
-                for (int kit = 0; kit < W.nk; ++kit, ++it) {
-                    const int s = it % S;
-                    if (!tc::mbar_wait(bar(s), (it / S) & 1, err)) { ok = false; break; }
+                for (int kit = 0; kit < W.nk; ++kit) {
+                    if (!tc::mbar_wait(bar(s), ph, err)) { ok = false; break; }
                     tc::fence_after();
-                    const uint32_t sA = sbase + s * P.stage_bytes;
-                    issue_mmas<KIND, PREC, CG2>(P, W, kit, sA, tacc, kit == 0);
+                    issue_mmas<KIND, PREC, CG2>(P, M, id, kit, (uint32_t)(s * P.stage_bytes) >> 4, tacc, kit == 0);
                     if (CG2) tc::mma_commit_pair(bar(kBarEmpty + s));
                     else tc::mma_commit(bar(kBarEmpty + s));
+                    if (++s == S) { s = 0; ph ^= 1u; }
                 }
                 if (!ok) break;
                 if (CG2) tc::mma_commit_pair(bar(kBarAccFull + buf));
