@@ -128,7 +128,7 @@ struct Work {
     int N;      // MMA N
 };
 
-template <int KIND, int PREC>
+template <int KIND, int PREC, int TPS>
 __device__ __forceinline__ void decode(const TcParams &P, int w, Work &W) {
     constexpr int CK = PREC ? 64 : 32;   // elements per 128-byte row
     if (KIND == TK_TB) {
@@ -152,13 +152,13 @@ __device__ __forceinline__ void decode(const TcParams &P, int w, Work &W) {
     case TK_F1: W.nk = (P.v + CK - 1) / CK; W.N = ((W.nterms * o + 15) / 16) * 16; break;
     case TK_VB: W.nk = (o2 + CK - 1) / CK;  W.N = ((W.nterms * o + 15) / 16) * 16; break;
     case TK_TB: {
-        W.nk = W.nterms;
+        W.nk = (W.nterms + TPS - 1) / TPS;
         const int rem = o2 - W.nt * P.tb_n;
         W.N = rem >= P.tb_n ? P.tb_n : ((rem + CK - 1) / CK) * CK;
         break;
     }
     case TK_F2: W.nk = (o + CK - 1) / CK; W.N = W.nterms * P.ock; break;
-    case TK_OB1: W.nk = W.nterms; W.N = ((o + 15) / 16) * 16; break;   // one stage per term: all r
+    case TK_OB1: W.nk = (W.nterms + TPS - 1) / TPS; W.N = ((o + 15) / 16) * 16; break;   // stages of whole terms: all r
     default: W.nk = (o / (CK / 8)) * P.nb; W.N = ((W.nterms * o + 15) / 16) * 16; break;   // (p-group, Q) K chunks
     }
 }
@@ -192,13 +192,14 @@ __device__ __forceinline__ TermOps term_ops(const TcParams &P, int eid, int job)
 // boxes of term t by lane t; A boxes, and the chunks of a one-term stage, by
 // consecutive lanes), so that a stage costs one or two issue slots instead of a
 // serial loop.  mine: this lane's term (F1, VB, F2, OB2: term `lane` of the
-// item; TB, OB1: the stage's term, the same in every lane).
+// item; TB, OB1: term lane / 2 of the stage, whose A the even and whose B the
+// odd lane requests).
 // CG2 (CTA pair, F1 only): this CTA (rank) loads its 128 rows of the item's
 // 256-row M-tile and its half of B, half-term boxes rank*nterms ..
 // (rank+1)*nterms - 1 of o/2 rows each; the bytes of both CTAs complete on
 // the leader's full barrier (cbar, shared::cluster address), whose
 // transaction count the leader sets.
-template <int KIND, int PREC, bool CG2 = false>
+template <int KIND, int PREC, bool CG2, int TPS>
 __device__ __forceinline__ void issue_loads(const TcParams &P, const Work &W, int kit, uint32_t sA, uint32_t bar,
                                             const TermOps &mine, int lane, uint32_t rank = 0, uint32_t cbar = 0) {
     constexpr int CK = PREC ? 64 : 32;           // elements per 128-byte row
@@ -263,9 +264,12 @@ __device__ __forceinline__ void issue_loads(const TcParams &P, const Work &W, in
         const int kp = PREC ? (o + 15) / 16 * 16 : o;   // K rows (p) of one term, zero-filled past o
         constexpr int nca = 128 / CK;
         const int nch = P.tb_n / CK;                    // chunks past o^2 are zero-filled
-        arm((uint32_t)(nca + nch) * kp * 128u);
-        if (lane == 0) ld4(sA, P.a_bytes, &P.mapA, &P.mapA2, W.mt * nca, mine.p0);
-        if (lane == 1) ld4(sB, P.b_bytes, &P.mapB, &P.mapB2, W.nt * nch, mine.p1);
+        const int nt = TPS == 1 ? 1 : min(TPS, W.nterms - kit * TPS), u = lane >> 1;
+        arm((uint32_t)nt * (nca + nch) * kp * 128u);
+        if (u < nt) {
+            if (lane & 1) ld4(sB + u * nch * kp * 128, P.b_bytes, &P.mapB, &P.mapB2, W.nt * nch, mine.p1);
+            else ld4(sA + u * nca * kp * 128, P.a_bytes, &P.mapA, &P.mapA2, W.mt * nca, mine.p0);
+        }
         break;
     }
     case TK_F2: {
@@ -277,16 +281,24 @@ __device__ __forceinline__ void issue_loads(const TcParams &P, const Work &W, in
         break;
     }
     case TK_OB1: {
-        // stage kit = term kit, all of K = r: A = its W-bar from the rotated
+        // stage kit = terms kit tps .., all of K = r each: A = W-bar from the rotated
         // slot (M = 128 tiled pq positions, K rows r < kr8 = o rounded up to a
         // k-step (8 tf32, 16 bf16), MN-major, one box of kr8 rows per CK
         // positions, rows past o zero-filled); B = t2T rows l, K-major, one
         // box per CK of r
         const int kr8 = PREC ? (o + 15) / 16 * 16 : (o + 7) / 8 * 8, nkc = (kr8 + CK - 1) / CK;
         constexpr int nca = 128 / CK;
-        arm((uint32_t)nca * kr8 * 128u + (uint32_t)nkc * o * 128u);
-        if (lane == 0) ld4(sA, P.a_bytes, &P.mapA, &P.mapA2, W.mt * nca, mine.p1);
-        else if (lane <= nkc) ldB((lane - 1) * o * 128u, CK * (lane - 1), 0, mine.p0);
+        const int nt = TPS == 1 ? 1 : min(TPS, W.nterms - kit * TPS), u = lane >> 1;
+        arm((uint32_t)nt * (nca * kr8 + nkc * o) * 128u);
+        if (TPS == 1) {
+            if (lane == 0) ld4(sA, P.a_bytes, &P.mapA, &P.mapA2, W.mt * nca, mine.p1);
+            else if (lane <= nkc) ldB((lane - 1) * o * 128u, CK * (lane - 1), 0, mine.p0);
+        } else if (u < nt) {
+            if (lane & 1)
+                for (int c = 0; c < nkc; ++c) ldB((u * nkc + c) * o * 128u, CK * c, 0, mine.p0);
+            else
+                ld4(sA + u * nca * kr8 * 128, P.a_bytes, &P.mapA, &P.mapA2, W.mt * nca, mine.p1);
+        }
         break;
     }
     default: {  // TK_OB2
@@ -323,9 +335,10 @@ struct MmaOps {
     uint64_t a, b;        // first stage, first k-step (hi planes)
     uint32_t da, db;      // steps per k-step
     uint32_t lo_a, lo_b;  // distance of the lo planes (BF16x3)
-    int ksteps;           // k-steps of a stage
+    int ksteps;           // k-steps of a stage (TB, OB1: of a term)
+    uint32_t ta, tb;      // TB, OB1: distance of a stage's terms
 };
-template <int KIND, int PREC>
+template <int KIND, int PREC, int TPS>
 __device__ __forceinline__ MmaOps mma_ops(const TcParams &P, uint32_t sbase) {
     constexpr int CK = PREC ? 64 : 32;
     constexpr int KS = PREC ? 16 : 8;                    // K per MMA
@@ -347,20 +360,17 @@ __device__ __forceinline__ MmaOps mma_ops(const TcParams &P, uint32_t sbase) {
     M.db = (bmn ? MN_STEP : 32u) >> 4;
     M.lo_a = (uint32_t)P.a_bytes >> 4;
     M.lo_b = (uint32_t)P.b_bytes >> 4;
+    M.ta = M.lo_a / TPS;
+    M.tb = M.lo_b / TPS;
     M.ksteps = KIND == TK_TB || KIND == TK_OB1 ? (int)kr / KS : CK / KS;
     return M;
 }
 
-// off: the stage's offset in 16-byte units; id: instruction descriptor of the item
-template <int KIND, int PREC, bool CG2 = false>
-__device__ __forceinline__ void issue_mmas(const TcParams &P, const MmaOps &M, uint32_t id, int kit, uint32_t off,
-                                           uint32_t tacc, bool first) {
+// the MMAs of ksteps k-steps from descriptors da, db
+template <int KIND, int PREC, bool CG2>
+__device__ __forceinline__ void issue_ksteps(const TcParams &P, const MmaOps &M, uint32_t id, int ksteps, uint64_t da,
+                                             uint64_t db, uint32_t tacc, uint32_t acc) {
     constexpr int CK = PREC ? 64 : 32, KS = PREC ? 16 : 8;
-    int ksteps = M.ksteps;
-    // K = l (F2) runs past o in the last chunk: its zero-filled k-steps are not issued
-    if (KIND == TK_F2) ksteps = min(ksteps, (P.o - CK * kit + KS - 1) / KS);
-    uint64_t da = M.a + off, db = M.b + off;
-    uint32_t acc = first ? 0u : 1u;
 #pragma unroll 4
     for (int kk = 0; kk < ksteps; ++kk) {
         if (CG2) {
@@ -387,6 +397,23 @@ __device__ __forceinline__ void issue_mmas(const TcParams &P, const MmaOps &M, u
         db += M.db;
         // OB1's B is K-major with one row block (o rows of 128 bytes) per CK of K
         if (KIND == TK_OB1 && (kk + 1) % (CK / KS) == 0) db += (uint32_t)P.o * 8u - 8u;
+    }
+}
+
+// off: the stage's offset in 16-byte units; id: instruction descriptor of the item
+template <int KIND, int PREC, bool CG2, int TPS>
+__device__ __forceinline__ void issue_mmas(const TcParams &P, const MmaOps &M, const Work &W, uint32_t id, int kit,
+                                           uint32_t off, uint32_t tacc) {
+    constexpr int CK = PREC ? 64 : 32, KS = PREC ? 16 : 8;
+    const uint64_t da = M.a + off, db = M.b + off;
+    if (KIND == TK_TB || KIND == TK_OB1) {
+        const int nt = TPS == 1 ? 1 : min(TPS, W.nterms - kit * TPS);
+        for (int u = 0; u < nt; ++u)
+            issue_ksteps<KIND, PREC, CG2>(P, M, id, M.ksteps, da + u * M.ta, db + u * M.tb, tacc, kit + u ? 1u : 0u);
+    } else {
+        // K = l (F2) runs past o in the last chunk: its zero-filled k-steps are not issued
+        const int ksteps = KIND == TK_F2 ? min(M.ksteps, (P.o - CK * kit + KS - 1) / KS) : M.ksteps;
+        issue_ksteps<KIND, PREC, CG2>(P, M, id, ksteps, da, db, tacc, kit ? 1u : 0u);
     }
 }
 
@@ -597,7 +624,7 @@ __device__ __forceinline__ void epilogue(const TcParams &P, const Work &W, uint3
 // both CTAs, its commits arrive on the stage-empty and accumulator-full
 // barriers of both CTAs, and both CTAs' epilogue warps arrive on the leader's
 // accumulator-empty barriers.  Accumulators are double-buffered.
-template <int KIND, int PREC, bool CG2 = false>
+template <int KIND, int PREC, bool CG2 = false, int TPS = 1>
 __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_constant__ TcParams P) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -655,10 +682,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
         // of TB and OB1, left the tensor pipe waiting on this warp: at nocc=48/
         // nvir=300 TF32, F1 112 -> 97 ms, VB 110 -> 92, TB 100 -> 86, OB1 55 -> 42,
         // OB2 52 -> 38 ms of a step; at nocc=16/nvir=72 TB 11.6 -> 7.3 ms).
-        constexpr bool PER_STAGE = KIND == TK_TB || KIND == TK_OB1;   // one term per stage
+        constexpr bool PER_STAGE = KIND == TK_TB || KIND == TK_OB1;   // tps terms per stage
         auto get_work = [&](int w) {
             Work W{};
-            if (w < P.nwork) decode<KIND, PREC>(P, w, W);
+            if (w < P.nwork) decode<KIND, PREC, TPS>(P, w, W);
             return W;
         };
         auto get_entry = [&](const Work &W, int first) {
@@ -677,19 +704,20 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
             int eidb = 0, jobb = 0;   // TB, OB1: the next 32 terms of this item
             for (int kit = 0; kit < W.nk; ++kit) {
                 if (PER_STAGE) {
-                    const int u = kit & 31;
+                    const int first = kit * TPS, u = first & 31;
                     if (kit > 0 && u == 0) mine = term_ops<KIND, PREC>(P, eidb, jobb);
-                    if (u == 0) eidb = get_entry(W, kit + 32);
+                    if (u == 0) eidb = get_entry(W, first + 32);
                     if (u == 16) jobb = P.jobs[eidb / 6];
                 }
                 if (!tc::mbar_wait(bar(kBarEmpty + s), ph, err)) ok = false;
                 if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
                 TermOps T = mine;
                 if (PER_STAGE) {
-                    T.p0 = __shfl_sync(0xffffffffu, mine.p0, kit & 31);
-                    T.p1 = __shfl_sync(0xffffffffu, mine.p1, kit & 31);
+                    const int t = TPS == 1 ? kit & 31 : (kit * TPS + (lane >> 1)) & 31;
+                    T.p0 = __shfl_sync(0xffffffffu, mine.p0, t);
+                    T.p1 = __shfl_sync(0xffffffffu, mine.p1, t);
                 }
-                issue_loads<KIND, PREC, CG2>(P, W, kit, sbase + s * P.stage_bytes, bar(s), T, lane, rank,
+                issue_loads<KIND, PREC, CG2, TPS>(P, W, kit, sbase + s * P.stage_bytes, bar(s), T, lane, rank,
                                              CG2 ? tc::mapa(bar(s), 0) : 0u);
                 ++issued;
                 if (++s == S) { s = 0; ph ^= 1u; }
@@ -708,13 +736,13 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
             constexpr bool amn = KIND == TK_TB || KIND == TK_OB1 || KIND == TK_OB2, bmn = KIND == TK_TB || KIND == TK_F2;
-            const MmaOps M = mma_ops<KIND, PREC>(P, sbase);
+            const MmaOps M = mma_ops<KIND, PREC, TPS>(P, sbase);
             int s = 0, wi = 0;
             uint32_t ph = 0;   // stage and its phase, stepped (a division by S each stage cost more than its MMAs)
             bool ok = true;
             for (int w = cid; w < P.nwork && ok; w += ncl, ++wi) {
                 Work W;
-                decode<KIND, PREC>(P, w, W);
+                decode<KIND, PREC, TPS>(P, w, W);
                 // CTA pair: M = 256 (128 rows in each CTA), B rows split between the CTAs
                 const uint32_t id = tc::idesc(PREC ? 1 : 2, CG2 ? 256 : 128, W.N, amn, bmn);
                 // paired kinds use both TMEM halves for one item: single-buffered
@@ -725,7 +753,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
                 for (int kit = 0; kit < W.nk; ++kit) {
                     if (!tc::mbar_wait(bar(s), ph, err)) { ok = false; break; }
                     tc::fence_after();
-                    issue_mmas<KIND, PREC, CG2>(P, M, id, kit, (uint32_t)(s * P.stage_bytes) >> 4, tacc, kit == 0);
+                    issue_mmas<KIND, PREC, CG2, TPS>(P, M, W, id, kit, (uint32_t)(s * P.stage_bytes) >> 4, tacc);
                     if (CG2) tc::mma_commit_pair(bar(kBarEmpty + s));
                     else tc::mma_commit(bar(kBarEmpty + s));
                     if (++s == S) { s = 0; ph ^= 1u; }
@@ -744,7 +772,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
         int wi = 0;
         for (int w = cid; w < P.nwork; w += ncl, ++wi) {
             Work W;
-            decode<KIND, PREC>(P, w, W);
+            decode<KIND, PREC, TPS>(P, w, W);
             if (CG2) W.mt = 2 * W.mt + (int)rank;   // this CTA's 128-row half of the item
             const int buf = PAIRED ? 0 : (wi & 1), use = PAIRED ? wi : (wi >> 1);
             if (!tc::mbar_wait(bar(kBarAccFull + buf), use & 1, err)) break;
@@ -1139,18 +1167,18 @@ void mixed_release(MixedOperands *mo, cudaStream_t st) {
 
 constexpr int kSmemMax = 232448;
 
-template <int KIND, int PREC>
+template <int KIND, int PREC, int TPS = 1>
 static int launch_tc(TcParams &P, cudaStream_t st) {
     if (P.nwork <= 0) return CT_OK;
     const int smem = P.stages * P.stage_bytes + 1024 + 256 + epi_active(KIND) * ebuf_floats(KIND) * 4;
     if (smem > kSmemMax) return CT_ERR_SHAPE;
-    if (smem_optin(reinterpret_cast<const void *>(tc_gemm_kernel<KIND, PREC>), kSmemMax) != cudaSuccess)
+    if (smem_optin(reinterpret_cast<const void *>(tc_gemm_kernel<KIND, PREC, false, TPS>), kSmemMax) != cudaSuccess)
         return CT_ERR_CUDA;
     const int sms = md().sms;
     const int grid = P.nwork < sms ? P.nwork : sms;
     // at least ~116 KB so that a second CTA never shares the SM's tensor memory
     const int smem_req = smem < 120 * 1024 ? 120 * 1024 : smem;
-    tc_gemm_kernel<KIND, PREC><<<grid, kThreads, smem_req, st>>>(P);
+    tc_gemm_kernel<KIND, PREC, false, TPS><<<grid, kThreads, smem_req, st>>>(P);
     return cudaGetLastError() == cudaSuccess ? CT_OK : CT_ERR_CUDA;
 }
 
@@ -1200,6 +1228,18 @@ static void set_stages(TcParams &P, int a_bytes, int b_bytes, int prec, int kind
     P.stage_bytes = (prec ? 2 : 1) * (a_bytes + b_bytes);
     int s = (kSmemMax - 1024 - 256 - epi_active(kind) * ebuf_floats(kind) * 4) / P.stage_bytes;
     P.stages = s > kMaxStages ? kMaxStages : s;
+}
+
+// TB, OB1: terms of k K-rows a stage holds.  A stage costs its two issuing threads
+// about 0.4 us whatever it holds, more than a term of up to 16 rows takes otherwise:
+// TF32 t2-bar / vooo-bar 3.27 / 3.23 -> 1.46 / 1.48 ms with four terms at nocc=8/
+// nvir=60, 4.32 / 4.20 -> 3.52 / 3.50 ms with two at nocc=16/nvir=72.
+static int terms_per_stage(int k) { return k <= 8 ? 4 : (k <= 16 ? 2 : 1); }
+
+template <int KIND, int PREC> static int launch_terms(TcParams &P, int tps, cudaStream_t st) {
+    if (tps == 4) return launch_tc<KIND, PREC, 4>(P, st);
+    if (tps == 2) return launch_tc<KIND, PREC, 2>(P, st);
+    return launch_tc<KIND, PREC, 1>(P, st);
 }
 
 template <int PREC>
@@ -1344,9 +1384,10 @@ static int mixed_wave_p(const WaveView &w, const EpiArgs &e, const ct_grads *g, 
             P.groups = w.tb_groups; P.entries = w.tb_entries;
             P.nwork = w.n_tb_groups * P.m_tiles * P.n_tiles;
             P.out = g->t2T;
-            set_stages(P, (128 / CK) * kp * 128, (P.tb_n / CK) * kp * 128, PREC, TK_TB);
+            const int tps = terms_per_stage(kp);
+            set_stages(P, tps * (128 / CK) * kp * 128, tps * (P.tb_n / CK) * kp * 128, PREC, TK_TB);
             if (prof) prof(PK_MTB, 0, pctx);
-            if ((rc = launch_tc<TK_TB, PREC>(P, st)) != CT_OK) return rc;
+            if ((rc = launch_terms<TK_TB, PREC>(P, tps, st)) != CT_OK) return rc;
             if (prof) prof(PK_MTB, 1, pctx);
         }
         // ---- OB1: D[tiled pq,l], A = rotated Wbar (tiled pq, r, slot) MN-major box(CK, o8),
@@ -1362,9 +1403,10 @@ static int mixed_wave_p(const WaveView &w, const EpiArgs &e, const ct_grads *g, 
             P.groups = w.xgroups; P.entries = w.x_entries;
             P.nwork = w.n_xgroups * P.m_tiles;
             P.out = g->vooo;
-            set_stages(P, 128 * kr8 * (PREC ? 2 : 4), ((kr8 + CK - 1) / CK) * o * 128, PREC, TK_OB1);
+            const int tps = terms_per_stage(kr8);
+            set_stages(P, tps * 128 * kr8 * (PREC ? 2 : 4), tps * ((kr8 + CK - 1) / CK) * o * 128, PREC, TK_OB1);
             if (prof) prof(PK_MOB1, 0, pctx);
-            if ((rc = launch_tc<TK_OB1, PREC>(P, st)) != CT_OK) return rc;
+            if ((rc = launch_terms<TK_OB1, PREC>(P, tps, st)) != CT_OK) return rc;
             if (prof) prof(PK_MOB1, 1, pctx);
         }
         // ---- OB2: D[l,(t,r)], A = voof rows (p,q8) (l,q8,Q,xp) MN-major, B = rotated Wbar
