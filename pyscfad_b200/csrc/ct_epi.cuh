@@ -15,34 +15,16 @@ __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gmem_src)
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// W-bar storage of the epilogue: WB 0 = the scratch type as is (float64 path);
-// 1 = float rounded to the nearest tf32 (it feeds tf32 tensor-core GEMMs, whose
-// MMA would otherwise truncate); 2 = float kept whole in shared memory and
-// written out as bf16 hi/lo planes (BF16x3).
-template <typename ST, int WB> __device__ __forceinline__ ST wbar_store(double x) {
+// W-bar as staged by the mixed path's epilogue: WB 1 = float rounded to the
+// nearest tf32 (it feeds tf32 tensor-core GEMMs, whose MMA would otherwise
+// truncate); 0 = float kept whole (BF16x3 splits it on the way out).
+template <int WB> __device__ __forceinline__ float wbar_store(float x) {
     if (WB == 1) {
         uint32_t r;
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"((float)x));
-        return (ST)__uint_as_float(r);
+        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+        return __uint_as_float(r);
     }
-    return (ST)x;
-}
-
-// Element of a block-orbit owned by thread slot q.  T = 8, 256 threads: each
-// warp covers a 2 x 4 x 4 sub-cube (u x w x t), so no coordinate spans more
-// than 4 values within a warp; otherwise the canonical order.
-template <int T, int NTHR>
-__device__ __forceinline__ void loc_of(int q, int (&loc)[3]) {
-    if (T == 8 && NTHR == 256) {
-        const int wq = q & 31, wi = q >> 5;
-        loc[2] = (wq & 3) | ((wi & 1) << 2);
-        loc[1] = ((wq >> 2) & 3) | (((wi >> 1) & 1) << 2);
-        loc[0] = ((wq >> 4) & 1) | (((wi >> 2) & 3) << 1);
-    } else {
-        loc[0] = q / (T * T);
-        loc[1] = (q / T) % T;
-        loc[2] = q % T;
-    }
+    return x;
 }
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -71,51 +53,31 @@ __device__ __forceinline__ void ksum_tree(KSum &k, double &v) {
     }
 }
 
-// One element orbit {perm(i,j,k)} of a staged block-orbit (I,J,K) = (BI,BJ,BK):
-// W, V, r3, the denominator, the job-energy contribution and (vjp) the
-// backward quantities, all in registers (ccsd_t_vjp.c:9-117 per element;
-// lno_ccsd_t.c:6-29).  Staged tiles: Gs[sigma][buffer d] blocks of BLK
+// One element orbit {perm(i,j,k)} of a staged block-orbit (I,J,K) = (BI,BJ,BK)
+// of the mixed path: W, V, r3, the denominator, the job-energy contribution and
+// (vjp) the backward quantities, all in registers (ccsd_t_vjp.c:9-117 per
+// element; lno_ccsd_t.c:6-29).  Staged tiles: Gs[sigma][buffer d] blocks of BLK
 // elements with u-stride TP, V tiles VA/VB[sigma][slot][T^2], t1/fvo rows
-// Us/Ws[sigma][64].  Writes W-bar in place into Gs, ybar to Yg (the job's
-// ybar slot) and this element's mo_energy-bar partial to tmp_s.
-// AT is the arithmetic type of W, V, r3 and the bars (double on the float64
-// path, float on the mixed path); the denominator, the energy terms and the
-// mo_energy-bar partials are float64 in both.
-//
-// DIRECT: W-bar goes straight to the job's slots in global memory (Sg = slot
-// 0, slot stride o^3) instead of into Gs.  TMP_OUT: the element's
-// mo_energy-bar partial is returned in tmp_out instead of tmp_s.
-// QRT: the job's slots are qr-tiled (the mixed path's layout): element (i,j,k)
-// of a slot at i o^2 + (j/8) 8o + (k/8) 64 + (j%8) 8 + k%8; else plain (i,j,k).
-// YST: ybar goes to a shared-memory staging buffer Yg laid out like the G
-// tiles (index off[s]) instead of to global memory; the caller flushes it.
-template <typename AT, typename ST, typename VT, int T, int TP, int BLK, int WB, bool DIRECT = false,
-          bool TMP_OUT = DIRECT, bool QRT = false, bool YST = false>
+// Us/Ws[3][64] of a, b, c.  Writes W-bar in place into Gs, ybar to the staging
+// buffer Yg laid out like the G tiles (the caller flushes both) and this
+// element's mo_energy-bar partial to tmp.  W, V, r3 and the bars are float; the
+// denominator, the energy terms and the mo_energy-bar partials are float64.
+template <int T, int TP, int BLK, int WB>
 __device__ __forceinline__ void orbit_element(const int (&loc)[3], int BI, int BJ, int BK, const int (&dmap)[6],
-                                              ST *Gs, const VT *VA, const VT *VB, const VT *Us, const VT *Ws,
-                                              const double *eocc, double *tmp_s, ST *Yg, int o, double fac,
+                                              float *Gs, const float *VA, const float *VB, const float *Us,
+                                              const float *Ws, const double *eocc, float *Yg, int o, double fac,
                                               double eabc, double eb, bool vjp, KSum &eacc, double &vir_acc,
-                                              bool with_fvo = true, ST *Sg = nullptr, double *tmp_out = nullptr,
-                                              bool lno = false) {
+                                              bool with_fvo, double &tmp, bool lno) {
     constexpr int T2 = T * T;
-    const int cq = (loc[0] * T + loc[1]) * T + loc[2];   // canonical slot of this element
-    if (TMP_OUT) *tmp_out = 0.0;
-    else tmp_s[cq] = 0.0;
+    tmp = 0.0;
     const int ijk[3] = {BI * T + loc[0], BJ * T + loc[1], BK * T + loc[2]};
-    auto gidx = [o](int i, int j, int k) -> long long {
-        return QRT ? (long long)i * o * o + (j >> 3) * 8 * o + (k >> 3) * 64 + (j & 7) * 8 + (k & 7)
-                   : ((long long)i * o + j) * o + k;
-    };
     if (ijk[0] >= o || ijk[1] >= o || ijk[2] >= o) return;
     if ((BI == BJ && loc[0] < loc[1]) || (BJ == BK && loc[1] < loc[2])) return;
-    int off[6], gr[6];
-    int lp[6][2];
+    int off[6], vp[6];
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
         off[s] = dmap[s] * BLK + loc[kR(s, 0)] * TP + loc[kR(s, 1)] * T + loc[kR(s, 2)];
-        lp[s][0] = loc[kR(s, 0)];
-        lp[s][1] = loc[kR(s, 1)];
-        gr[s] = ijk[kR(s, 2)];
+        vp[s] = loc[kR(s, 0)] * T + loc[kR(s, 1)];
     }
     bool first[6];
 #pragma unroll
@@ -125,22 +87,31 @@ __device__ __forceinline__ void orbit_element(const int (&loc)[3], int BI, int B
         for (int t = 0; t < s; ++t) f = f && (off[t] != off[s]);
         first[s] = f;
     }
-    AT W[6], Y[6], Z[6];
+    // t1 and fvo of the three virtuals at the three occupieds: nine values each
+    float u[3][3], fv[3][3];
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            u[m][q] = Us[m * 64 + ijk[q]];
+            fv[m][q] = with_fvo ? Ws[m * 64 + ijk[q]] : 0.f;
+        }
+    float W[6], Y[6], Z[6];
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
-        AT ws = 0, vs = 0;
+        float ws = 0, vs = 0;
 #pragma unroll
         for (int sg = 0; sg < 6; ++sg) {
             const int cs = kComp(s, sg);
-            ws += (AT)Gs[sg * 6 * BLK + off[cs]];
-            const int vi = (sg * 6 + cs) * T2 + lp[cs][0] * T + lp[cs][1];
-            vs += (AT)VA[vi] * (AT)Us[sg * 64 + gr[cs]];
-            if (with_fvo) vs += (AT)VB[vi] * (AT)Ws[sg * 64 + gr[cs]];
+            ws += Gs[sg * 6 * BLK + off[cs]];
+            const int vi = (sg * 6 + cs) * T2 + vp[cs];
+            vs += VA[vi] * u[kR(sg, 2)][kR(cs, 2)];
+            if (with_fvo) vs += VB[vi] * fv[kR(sg, 2)][kR(cs, 2)];
         }
         W[s] = ws;
-        Y[s] = ws + (AT)0.5 * vs;
+        Y[s] = ws + 0.5f * vs;
     }
-    r3_orbit<AT>(Y, Z);
+    r3_orbit<float>(Y, Z);
     // one reciprocal per element: d3 = fac / D; the orbit's distinct W.Z
     // products share d3, so they are summed before the compensated add, and
     // the mo_energy-bar partial eb d3^2 / fac = eb fac / D^2 reuses 1/D
@@ -157,59 +128,32 @@ __device__ __forceinline__ void orbit_element(const int (&loc)[3], int BI, int B
         // thread only); the projection follows in a separate kernel
 #pragma unroll
         for (int s = 0; s < 6; ++s) {
-            Gs[off[s]] = (ST)W[s];
-            Gs[6 * BLK + off[s]] = (ST)((double)Z[s] * rden);
+            Gs[off[s]] = W[s];
+            Gs[6 * BLK + off[s]] = (float)((double)Z[s] * rden);
         }
         return;
     }
     if (vjp) {
-        const AT ebd3 = (AT)(eb * d3);
-        AT zb[6], wb[6];
-        const double tmp = eb * d3 * rden * wz;
+        const float ebd3 = (float)(eb * d3);
+        float zb[6], wb[6];
+        tmp = eb * d3 * rden * wz;
 #pragma unroll
         for (int s = 0; s < 6; ++s) {
             zb[s] = ebd3 * W[s];
             wb[s] = ebd3 * Z[s];
         }
-        AT yb[6];
-        r3_orbit<AT>(zb, yb);
+        float yb[6];
+        r3_orbit<float>(zb, yb);
 #pragma unroll
-        for (int s = 0; s < 6; ++s) wb[s] += yb[s];
-        if (TMP_OUT) *tmp_out = tmp;
-        else tmp_s[cq] = tmp;
+        for (int s = 0; s < 6; ++s) wb[s] = wbar_store<WB>(wb[s] + yb[s]);
         vir_acc += tmp;
-        if (DIRECT) {
-            // global positions of the orbit's elements; a position shared by
-            // several slots keeps the last slot's value, as the in-place path does
-            const long long o3 = (long long)o * o * o;
-            long long gi[6];
-            bool last[6];
 #pragma unroll
-            for (int s2 = 0; s2 < 6; ++s2) {
-                gi[s2] = gidx(ijk[kR(s2, 0)], ijk[kR(s2, 1)], ijk[kR(s2, 2)]);
-                bool l = true;
+        for (int sg = 0; sg < 6; ++sg)
 #pragma unroll
-                for (int t = s2 + 1; t < 6; ++t) l = l && (off[t] != off[s2]);
-                last[s2] = l;
-            }
-#pragma unroll
-            for (int sg = 0; sg < 6; ++sg)
-#pragma unroll
-                for (int s2 = 0; s2 < 6; ++s2)
-                    if (last[s2]) Sg[sg * o3 + gi[s2]] = wbar_store<ST, WB>((double)wb[kComp(s2, kInv(sg))]);
-        } else {
-#pragma unroll
-            for (int sg = 0; sg < 6; ++sg)
-#pragma unroll
-                for (int s = 0; s < 6; ++s) Gs[sg * 6 * BLK + off[s]] = wbar_store<ST, WB>((double)wb[kComp(s, kInv(sg))]);
-        }
-        // ybar straight to its slot (each element of the cube belongs to one orbit)
+            for (int s = 0; s < 6; ++s) Gs[sg * 6 * BLK + off[s]] = wb[kComp(s, kInv(sg))];
 #pragma unroll
         for (int s = 0; s < 6; ++s)
-            if (first[s]) {
-                if (YST) Yg[off[s]] = (ST)yb[s];
-                else Yg[gidx(ijk[kR(s, 0)], ijk[kR(s, 1)], ijk[kR(s, 2)])] = (ST)yb[s];
-            }
+            if (first[s]) Yg[off[s]] = yb[s];
     }
 }
 
@@ -220,18 +164,13 @@ __device__ __forceinline__ void orbit_element(const int (&loc)[3], int BI, int B
 // sum A q, so z_bar = eb A / D, w_bar = eb B + r3(z_bar), v_bar = r3(z_bar)
 // (the canonical chain of orbit_element with those two products replaced)
 // and the mo_energy-bar partial is eb A q / D.  W-bar goes in place into
-// groups 0-5 (stored as wbar_store<ST, WB>), ybar to its slot.  Arithmetic
-// in float64 on both paths (there is no V term to form here).
-// TMP_OUT, QRT, YST as for orbit_element: the partial returned in tmp_out;
-// ybar addressed in the qr-tiled layout; ybar into the staging tiles Yg.
-template <typename ST, int T, int TP, int BLK, int WB = 0, bool TMP_OUT = false, bool QRT = false,
-          bool YST = false>
+// groups 0-5, ybar to its staging buffer.  Arithmetic in float64 (there is no V
+// term to form here).
+template <int T, int TP, int BLK, int WB>
 __device__ __forceinline__ void orbit_lno_bar(const int (&loc)[3], int BI, int BJ, int BK, const int (&dmap)[6],
-                                              ST *Gs, const double *eocc, double *tmp_s, ST *Yg, int o, double eabc,
-                                              double eb, double &vir_acc, double *tmp_out = nullptr) {
-    const int cq = (loc[0] * T + loc[1]) * T + loc[2];
-    if (TMP_OUT) *tmp_out = 0.0;
-    else tmp_s[cq] = 0.0;
+                                              float *Gs, const double *eocc, float *Yg, int o, double eabc, double eb,
+                                              double &vir_acc, double &tmp) {
+    tmp = 0.0;
     const int ijk[3] = {BI * T + loc[0], BJ * T + loc[1], BK * T + loc[2]};
     if (ijk[0] >= o || ijk[1] >= o || ijk[2] >= o) return;
     if ((BI == BJ && loc[0] < loc[1]) || (BJ == BK && loc[1] < loc[2])) return;
@@ -257,7 +196,7 @@ __device__ __forceinline__ void orbit_lno_bar(const int (&loc)[3], int BI, int B
         wb[s] = eb * B;
         if (first[s]) aq += A * q;
     }
-    const double tmp = eb * rden * aq;
+    tmp = eb * rden * aq;
     double yb[6];
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
@@ -267,25 +206,17 @@ __device__ __forceinline__ void orbit_lno_bar(const int (&loc)[3], int BI, int B
         yb[s] = t;
         wb[s] += t;
     }
-    if (TMP_OUT) *tmp_out = tmp;
-    else tmp_s[cq] = tmp;
     vir_acc += tmp;
+    float w[6];
+#pragma unroll
+    for (int s = 0; s < 6; ++s) w[s] = wbar_store<WB>((float)wb[s]);
 #pragma unroll
     for (int sg = 0; sg < 6; ++sg)
 #pragma unroll
-        for (int s = 0; s < 6; ++s) Gs[sg * 6 * BLK + off[s]] = wbar_store<ST, WB>(wb[kComp(s, kInv(sg))]);
+        for (int s = 0; s < 6; ++s) Gs[sg * 6 * BLK + off[s]] = w[kComp(s, kInv(sg))];
 #pragma unroll
     for (int s = 0; s < 6; ++s)
-        if (first[s]) {
-            if (YST) {
-                Yg[off[s]] = (ST)yb[s];
-            } else {
-                const int i = ijk[kR(s, 0)], j = ijk[kR(s, 1)], k = ijk[kR(s, 2)];
-                const long long gi = QRT ? (long long)i * o * o + (j >> 3) * 8 * o + (k >> 3) * 64 + (j & 7) * 8 + (k & 7)
-                                         : ((long long)i * o + j) * o + k;
-                Yg[gi] = (ST)yb[s];
-            }
-        }
+        if (first[s]) Yg[off[s]] = (float)yb[s];
 }
 
 }  // namespace ctb

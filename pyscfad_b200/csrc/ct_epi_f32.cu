@@ -27,12 +27,11 @@ struct Smem {
     static constexpr size_t g_bytes = sizeof(float) * 36 * BLK;      // one buffer of G tiles
     static constexpr size_t v_bytes = sizeof(float) * 36 * T2;       // one buffer of VA (or VB)
     static constexpr size_t buf_bytes = g_bytes + 2 * v_bytes;
-    static constexpr size_t u_off = 2 * buf_bytes;                   // float[6][64]
-    static constexpr size_t w_off = u_off + sizeof(float) * 6 * 64;  // float[6][64]
-    static constexpr size_t occ_off = w_off + sizeof(float) * 6 * 64;        // double[64]
-    static constexpr size_t eocc_off = occ_off + sizeof(double) * 64;        // double[64]
-    static constexpr size_t tmp_off = eocc_off + sizeof(double) * 64;        // double[T3]
-    static constexpr size_t y_off = tmp_off + sizeof(double) * T3;           // float[2][6 * BLK]: ybar staging
+    static constexpr size_t u_off = 2 * buf_bytes;                   // float[3][64]: t1T rows a, b, c
+    static constexpr size_t w_off = u_off + sizeof(float) * 3 * 64;  // float[3][64]: fvo rows a, b, c
+    static constexpr size_t occ_off = w_off + sizeof(float) * 3 * 64;             // double[NTHR / 32][64]
+    static constexpr size_t eocc_off = occ_off + sizeof(double) * (NTHR / 32) * 64;   // double[64]
+    static constexpr size_t y_off = eocc_off + sizeof(double) * 64;               // float[2][6 * BLK]: ybar staging
     static constexpr size_t y_bytes = sizeof(float) * 6 * BLK;
     static constexpr size_t bytes = y_off + 2 * y_bytes;
 };
@@ -85,67 +84,88 @@ struct OrbitBlocks {
     }
 };
 
-// cp.async of block-orbit `it`'s G tiles and V tiles into buffer (G, VA, VB).
-// lbar (LNO backward pass): the z/D cube and the two parts of the A and B
-// cubes (slots 1-5) into tile groups 0-4, and no V tiles.
-__device__ __forceinline__ void issue_stage(const BlockIter &it, const OrbitBlocks &ob, const float *S, long long o3,
-                                            int o, float *G, float *VA, float *VB, const float *vvf, const float *t2f,
-                                            const long long *vv_off, const long long *tt_off, int tid, bool with_fvo,
-                                            bool lbar = false) {
-    const int ng = lbar ? 5 : 6, s0 = lbar ? 1 : 0;
+// A thread's share of the staging: piece e3 = 4 (tid & 127) of an 8^3 block of
+// slots sg0 = tid / 128 and sg0 + 4 (two of them for 256 threads), and up to three
+// of the 16-byte pieces of the V tiles.  All that depends on the thread alone is
+// worked out once per job, so that a block-orbit costs it a few additions per copy
+// (the kernel is bound by its instructions: with that, the t1 and fvo values read
+// once per orbit and the occupied-energy sums kept per warp instead of added by
+// atomics, the epilogue takes 187 -> 156 ms of a nocc=48/nvir=300 TF32 block, 127 ->
+// 107 ms of a BF16x3 VJP at nocc=32/nvir=100, 8.9 -> 7.6 ms at nocc=16/nvir=72).
+struct Share {
+    int sg0, soff, goff;          // offsets of the piece in a staged block and in a slot's block
+    const float *vsrc[3];         // V piece: source at block (0, 0), null if none
+    int vdst[3], vk[3];           // its place in VA (VB follows) and the axes of its P and Q blocks (4 k0 + k1)
+    __device__ __forceinline__ void set(int tid, int o, const float *vvf, const float *t2f, const long long *vv_off,
+                                        const long long *tt_off, bool with_fvo) {
+        const int e3 = (tid & 127) * 4, u = e3 >> 6;
+        sg0 = tid >> 7;
+        soff = u * TP + (e3 & 63);
+        goff = u * o * o + (e3 & 63);
+        constexpr unsigned int KR01 = (0u | 1u << 2) | (0u | 2u << 2) << 4 | (1u | 0u << 2) << 8 |
+                                      (1u | 2u << 2) << 12 | (2u | 0u << 2) << 16 | (2u | 1u << 2) << 20;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const int i = tid + q * NTHR, which = i / (36 * 16), jj = i - which * (36 * 16);
+            const int tile = jj >> 4, piece = jj & 15, sg = tile / 6, cc = tile - 6 * sg;
+            const bool in = i < (with_fvo ? 2 : 1) * 36 * 16;
+            vsrc[q] = in ? (which ? t2f + tt_off[sg] : vvf + vv_off[sg]) + (piece >> 1) * o + (piece & 1) * 4 : nullptr;
+            vdst[q] = (which * 36 + tile) * T2 + (piece >> 1) * T + (piece & 1) * 4;
+            vk[q] = ((KR01 >> (4 * cc)) & 3) * 4 + ((KR01 >> (4 * cc + 2)) & 3);
+        }
+    }
+};
+// element offset of slot s's block in a qr-tiled slot: row u of it is 64 contiguous
+// floats at u o^2 from there
+__device__ __forceinline__ int block_at(const OrbitBlocks &ob, int s, int o) {
+    return (ob.bs[s][0] * o + ob.bs[s][1]) * T * o + ob.bs[s][2] * T * T;
+}
+
+// cp.async of block-orbit `it`'s G tiles and V tiles into buffer G (VA and VB
+// behind it).  lbar (LNO backward pass): the z/D cube and the two parts of the
+// A and B cubes (slots 1-5) into tile groups 0-4, and no V tiles.
+__device__ __forceinline__ void issue_stage(const BlockIter &it, const OrbitBlocks &ob, const Share &sh, const float *S,
+                                            long long o3, int o, float *G, int tid, bool lbar) {
+    const float *src = S + (sh.sg0 + (lbar ? 1 : 0)) * o3 + sh.goff;
+    float *dst = G + sh.sg0 * 6 * BLK + sh.soff;
+    const bool more = tid < (lbar ? 128 : 256);
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
         if (!ob.fresh[s]) continue;
-        const int d = ob.dmap[s];
-        const int p0 = ob.bs[s][0] * T, q0 = ob.bs[s][1] * T, r0 = ob.bs[s][2] * T;
-        // ng slots x 128 16-byte pieces of an 8^3 block
-        for (int j = tid; j < ng * 128; j += NTHR) {
-            const int sg = j >> 7, e3 = (j & 127) * 4;
-            const int u = e3 >> 6;
-            // qr-tiled slot: row u of the block is 64 contiguous floats
-            cp_async16(G + (sg * 6 + d) * BLK + u * TP + (e3 & 63),
-                       S + (sg + s0) * o3 + (long long)(p0 + u) * o * o + q0 * o + 8 * r0 + (e3 & 63));
-        }
+        const float *g = src + block_at(ob, s, o);
+        cp_async16(dst + ob.dmap[s] * BLK, g);
+        if (more) cp_async16(dst + (24 + ob.dmap[s]) * BLK, g + 4 * o3);
     }
     if (lbar) return;
-    // V tiles: for each term sg and slot cc, the T x T tile (rows P, columns Q)
-    // on the blocks of slot cc's first two axes; 2 x 16 pieces per tile
-    constexpr unsigned int KR01 = (0u | 1u << 2) | (0u | 2u << 2) << 4 | (1u | 0u << 2) << 8 | (1u | 2u << 2) << 12 |
-                                  (2u | 0u << 2) << 16 | (2u | 1u << 2) << 20;
-    for (int j = tid; j < (with_fvo ? 2 : 1) * 36 * 16; j += NTHR) {
-        const int which = j / (36 * 16), jj = j - which * (36 * 16);
-        const int tile = jj >> 4, piece = jj & 15;
-        const int sg = tile / 6, cc = tile - 6 * sg;
-        const int k0 = (KR01 >> (4 * cc)) & 3, k1 = (KR01 >> (4 * cc + 2)) & 3;
-        const int P = (k0 == 0 ? it.I : (k0 == 1 ? it.J : it.K)) * T + (piece >> 1);
-        const int Q = (k1 == 0 ? it.I : (k1 == 1 ? it.J : it.K)) * T + (piece & 1) * 4;
-        const long long src = (which ? tt_off[sg] : vv_off[sg]) + (long long)P * o + Q;
-        cp_async16((which ? VB : VA) + tile * T2 + (piece >> 1) * T + (piece & 1) * 4, (which ? t2f : vvf) + src);
-    }
+    float *V = G + 36 * BLK;
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+        if (sh.vsrc[q]) {
+            const int k0 = sh.vk[q] >> 2, k1 = sh.vk[q] & 3;
+            const int P = k0 == 0 ? it.I : (k0 == 1 ? it.J : it.K), Q = k1 == 0 ? it.I : (k1 == 1 ? it.J : it.K);
+            cp_async16(V + sh.vdst[q], sh.vsrc[q] + (P * o + Q) * T);
+        }
 }
 
 // W-bar (tf32-rounded floats) of a finished block-orbit, written in place of
 // its G tiles in buffer G, out to the job's slots 0-5 in 16-byte pieces along
 // r.  A thread flushes exactly the pieces it fetches into the same buffer with
-// issue_stage (piece j of every tile belongs to thread j mod NTHR), and its
-// global stores consume its shared loads, so the buffer can be refilled right
-// after without another barrier.
-// With nsg = 2 (LNO energy) only slots 0-1 leave: the W and z/D cubes the
+// issue_stage, and its global stores consume its shared loads, so the buffer
+// can be refilled right after without another barrier.
+// With lno (LNO energy) only slots 0-1 leave: the W and z/D cubes the
 // element orbits wrote there in place of the G tiles.
-__device__ __forceinline__ void flush_wbar(const OrbitBlocks &ob, const float *G, float *S, long long o3, int o,
-                                           int tid, int nsg = 6) {
+__device__ __forceinline__ void flush_wbar(const OrbitBlocks &ob, const Share &sh, const float *G, float *S,
+                                           long long o3, int o, int tid, bool lno = false) {
+    float *dst = S + sh.sg0 * o3 + sh.goff;
+    const float *src = G + sh.sg0 * 6 * BLK + sh.soff;
+    const bool some = !lno || tid < 256, more = !lno && tid < 256;
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
         if (!ob.fresh[s]) continue;
-        const int d = ob.dmap[s];
-        const int p0 = ob.bs[s][0] * T, q0 = ob.bs[s][1] * T, r0 = ob.bs[s][2] * T;
-        for (int j = tid; j < nsg * 128; j += NTHR) {
-            const int sg = j >> 7, e3 = (j & 127) * 4;
-            const int u = e3 >> 6, ww = (e3 >> 3) & 7, t = e3 & 7;
-            (void)ww; (void)t;
-            const float4 x = *reinterpret_cast<const float4 *>(G + (sg * 6 + d) * BLK + u * TP + (e3 & 63));
-            *reinterpret_cast<float4 *>(S + sg * o3 + (long long)(p0 + u) * o * o + q0 * o + 8 * r0 + (e3 & 63)) = x;
-        }
+        float *g = dst + block_at(ob, s, o);
+        const int d = ob.dmap[s] * BLK;
+        if (some) *reinterpret_cast<float4 *>(g) = *reinterpret_cast<const float4 *>(src + d);
+        if (more) *reinterpret_cast<float4 *>(g + 4 * o3) = *reinterpret_cast<const float4 *>(src + 24 * BLK + d);
     }
 }
 
@@ -182,18 +202,14 @@ __device__ __forceinline__ void flush_wbar_bf16(const OrbitBlocks &ob, const flo
 
 // ybar of a finished block-orbit, staged in shared memory in the layout of the
 // G tiles (block d of the orbit at d * BLK), out to the job's slot 6 with
-// 16-byte stores: each block is eight runs of 64 contiguous floats there.
-__device__ __forceinline__ void flush_ybar(const OrbitBlocks &ob, const float *Y, float *S6, int o, int tid) {
+// 16-byte stores: each block is eight runs of 64 contiguous floats there.  128
+// threads take a block.
+__device__ __forceinline__ void flush_ybar(const OrbitBlocks &ob, const Share &sh, const float *Y, float *S6, int o) {
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
-        if (!ob.fresh[s]) continue;
-        const int d = ob.dmap[s];
-        const int p0 = ob.bs[s][0] * T, q0 = ob.bs[s][1] * T, r0 = ob.bs[s][2] * T;
-        for (int j = tid; j < 128; j += NTHR) {
-            const int e3 = j * 4, u = e3 >> 6;
-            const float4 x = *reinterpret_cast<const float4 *>(Y + d * BLK + u * TP + (e3 & 63));
-            *reinterpret_cast<float4 *>(S6 + (long long)(p0 + u) * o * o + q0 * o + 8 * r0 + (e3 & 63)) = x;
-        }
+        if (!ob.fresh[s] || (s & 3) != sh.sg0) continue;
+        *reinterpret_cast<float4 *>(S6 + block_at(ob, s, o) + sh.goff) =
+            *reinterpret_cast<const float4 *>(Y + ob.dmap[s] * BLK + sh.soff);
     }
 }
 
@@ -211,12 +227,7 @@ __global__ void __launch_bounds__(NTHR, 1) epi_pipe_kernel(const WaveView w, con
     float *Ws = reinterpret_cast<float *>(esm + Smem::w_off);
     double *occ_acc = reinterpret_cast<double *>(esm + Smem::occ_off);
     double *eocc = reinterpret_cast<double *>(esm + Smem::eocc_off);
-    double *tmp_s = reinterpret_cast<double *>(esm + Smem::tmp_off);
     auto bufG = [&](int i) { return reinterpret_cast<float *>(esm + i * Smem::buf_bytes); };
-    auto bufA = [&](int i) { return reinterpret_cast<float *>(esm + i * Smem::buf_bytes + Smem::g_bytes); };
-    auto bufB = [&](int i) {
-        return reinterpret_cast<float *>(esm + i * Smem::buf_bytes + Smem::g_bytes + Smem::v_bytes);
-    };
     auto bufY = [&](int i) { return reinterpret_cast<float *>(esm + Smem::y_off + i * Smem::y_bytes); };
     __shared__ long long vv_off[6], tt_off[6];
 
@@ -241,15 +252,14 @@ __global__ void __launch_bounds__(NTHR, 1) epi_pipe_kernel(const WaveView w, con
         vv_off[tid] = ((long long)(x * v + y) * o) * o;
         tt_off[tid] = ((long long)(y * v + x) * o) * o;
     }
-    for (int i = tid; i < o; i += NTHR) { occ_acc[i] = 0.0; eocc[i] = e.mo_energy[i]; }
+    for (int i = tid; i < o; i += NTHR) eocc[i] = e.mo_energy[i];
+    for (int i = tid; i < (NTHR / 32) * 64; i += NTHR) occ_acc[i] = 0.0;
     int fvo_nz = 0;
-    for (int i = tid; i < 6 * o; i += NTHR) {
-        const int sg = i / o, r = i - sg * o;
-        int x, y, z;
-        term_xyz(sg, a, b, c, x, y, z);
-        Us[sg * 64 + r] = (float)e.t1T[z * o + r];
-        const double f = e.fvo[z * o + r];
-        Ws[sg * 64 + r] = (float)f;
+    for (int i = tid; i < 3 * 64; i += NTHR) {
+        const int m = i >> 6, r = i & 63, z = m == 0 ? a : (m == 1 ? b : c);
+        const double f = r < o ? e.fvo[z * o + r] : 0.0;
+        Us[i] = r < o ? (float)e.t1T[z * o + r] : 0.f;
+        Ws[i] = (float)f;
         fvo_nz |= (f != 0.0);
     }
     // the fvo part of V (and its t2T tiles) is skipped when this job's fvo rows are zero
@@ -260,7 +270,6 @@ __global__ void __launch_bounds__(NTHR, 1) epi_pipe_kernel(const WaveView w, con
     const double eb = e.et_bar;
     const int nb = o / T;
     const int nbo = nb * (nb + 1) * (nb + 2) / 6;
-    constexpr bool STAGED = WB == 1 || WB == 2;   // W-bar staged in the G tiles
     // BF16x3: this job's hi / lo planes (plane jl*6 + sigma of npl = 6 n_jobs)
     __nv_bfloat16 *whi = nullptr, *wlo = nullptr;
     if (WB == 2) {
@@ -271,41 +280,43 @@ __global__ void __launch_bounds__(NTHR, 1) epi_pipe_kernel(const WaveView w, con
     BlockIter cur, nxt;
     OrbitBlocks ob_cur, ob_nxt, ob_prev;
     ob_cur.set(cur);
-    issue_stage(cur, ob_cur, S, o3, o, bufG(0), bufA(0), bufB(0), e.vvoo_f, e.t2_f, vv_off, tt_off, tid, with_fvo,
-                lbar);
+    Share sh;
+    sh.set(tid, o, e.vvoo_f, e.t2_f, vv_off, tt_off, with_fvo);
+    issue_stage(cur, ob_cur, sh, S, o3, o, bufG(0), tid, lbar);
     cp_async_commit();
-    int loc[3];
-    loc_of<T, 256>(tid, loc);   // 16 warps: warp w covers a 2x4x4 sub-cube
+    // the thread's element of a block: a warp covers a 2 x 4 x 4 sub-cube, so no
+    // coordinate spans more than 4 values within it
+    const int lq = tid & 31, lw = tid >> 5;
+    const int loc[3] = {(lq >> 4) | ((lw >> 2) << 1), ((lq >> 2) & 3) | (((lw >> 1) & 1) << 2), (lq & 3) | ((lw & 1) << 2)};
     for (int bo = 0; bo < nbo; ++bo) {
         const int bi = bo & 1;
         cp_async_wait_all();
         __syncthreads();  // stage bo landed for every thread; buffer bi^1 is free
-        if (WB == 1 && vjp && bo > 0) flush_wbar(ob_prev, bufG(bi ^ 1), S, o3, o, tid);
-        if (lno && bo > 0) flush_wbar(ob_prev, bufG(bi ^ 1), S, o3, o, tid, 2);
+        if (((WB == 1 && vjp) || lno) && bo > 0) flush_wbar(ob_prev, sh, bufG(bi ^ 1), S, o3, o, tid, lno);
         if (WB == 2 && vjp && bo > 0) flush_wbar_bf16(ob_prev, bufG(bi ^ 1), whi, wlo, o3, o, tid);
-        if (vjp && bo > 0) flush_ybar(ob_prev, bufY(bi ^ 1), S + 6 * o3, o, tid);
+        if (vjp && bo > 0) flush_ybar(ob_prev, sh, bufY(bi ^ 1), S + 6 * o3, o);
         if (WB == 2 && vjp && bo > 0) __syncthreads();   // bf16 pieces span two refill pieces
         if (bo + 1 < nbo) {
             nxt = cur;
             nxt.next();
             ob_nxt.set(nxt);
-            issue_stage(nxt, ob_nxt, S, o3, o, bufG(bi ^ 1), bufA(bi ^ 1), bufB(bi ^ 1), e.vvoo_f, e.t2_f, vv_off,
-                        tt_off, tid, with_fvo, lbar);
+            issue_stage(nxt, ob_nxt, sh, S, o3, o, bufG(bi ^ 1), tid, lbar);
             cp_async_commit();
         }
         float *G = bufG(bi);
+        const float *VA = G + 36 * BLK, *VB = VA + 36 * T2;
         // W-bar into the staged G tiles (TF32) or straight to the float slots
         // (BF16x3); mo_energy-bar partials reduced in the warp
         double tmp = 0.0;
         if (lbar)
-            orbit_lno_bar<float, T, TP, BLK, (WB == 1 ? 1 : 0), true, true, true>(
-                loc, cur.I, cur.J, cur.K, ob_cur.dmap, G, eocc, tmp_s, bufY(bi), o, eabc, eb, vir_acc, &tmp);
+            orbit_lno_bar<T, TP, BLK, (WB == 1 ? 1 : 0)>(loc, cur.I, cur.J, cur.K, ob_cur.dmap, G, eocc, bufY(bi), o,
+                                                         eabc, eb, vir_acc, tmp);
         else
-            orbit_element<float, float, float, T, TP, BLK, (WB == 1 ? 1 : 0), !STAGED, true, true, true>(
-                loc, cur.I, cur.J, cur.K, ob_cur.dmap, G, bufA(bi), bufB(bi), Us, Ws, eocc, tmp_s, bufY(bi), o, fac,
-                eabc, eb, vjp, eacc, vir_acc, with_fvo, S, &tmp, lno);
+            orbit_element<T, TP, BLK, (WB == 1 ? 1 : 0)>(loc, cur.I, cur.J, cur.K, ob_cur.dmap, G, VA, VB, Us, Ws,
+                                                         eocc, bufY(bi), o, fac, eabc, eb, vjp, eacc, vir_acc,
+                                                         with_fvo, tmp, lno);
         if (vjp) {
-            // lane bits: 0-1 -> loc[2], 2-3 -> loc[1], 4 -> loc[0] (low bits; loc_of)
+            // lane bits: 0-1 -> loc[2], 2-3 -> loc[1], 4 -> loc[0] (low bits)
             const int lane = tid & 31;
             double s0 = tmp, s1 = tmp, s2 = tmp;
 #pragma unroll
@@ -316,9 +327,14 @@ __global__ void __launch_bounds__(NTHR, 1) epi_pipe_kernel(const WaveView w, con
             s2 += __shfl_xor_sync(0xffffffffu, s2, 4);
             s2 += __shfl_xor_sync(0xffffffffu, s2, 8);
             s2 += __shfl_xor_sync(0xffffffffu, s2, 16);
-            if ((lane & 15) == 0) atomicAdd(&occ_acc[cur.I * T + loc[0]], -s0);
-            if ((lane & 19) == 0) atomicAdd(&occ_acc[cur.J * T + loc[1]], -s1);
-            if ((lane & 28) == 0) atomicAdd(&occ_acc[cur.K * T + loc[2]], -s2);
+            // the warp's own sums, one axis after the other (blocks may coincide)
+            double *occ = occ_acc + (tid >> 5) * 64;
+            if ((lane & 15) == 0) occ[cur.I * T + loc[0]] -= s0;
+            __syncwarp();
+            if ((lane & 19) == 0) occ[cur.J * T + loc[1]] -= s1;
+            __syncwarp();
+            if ((lane & 28) == 0) occ[cur.K * T + loc[2]] -= s2;
+            __syncwarp();
         }
         ob_prev = ob_cur;
         cur = nxt;
@@ -332,11 +348,10 @@ __global__ void __launch_bounds__(NTHR, 1) epi_pipe_kernel(const WaveView w, con
     double es = eacc.s, ec = eacc.c, vt = vir_acc;
     warp_ksum(es, ec, vt, 16);
     if (lane == 0) { wred[0][warp] = es; wred[1][warp] = ec; wred[2][warp] = vt; }
-    __syncthreads();  // also orders every warp's occ_acc atomics and W-bar tiles before the flushes below
-    if (WB == 1 && vjp) flush_wbar(ob_prev, bufG((nbo - 1) & 1), S, o3, o, tid);
-    if (lno) flush_wbar(ob_prev, bufG((nbo - 1) & 1), S, o3, o, tid, 2);
+    __syncthreads();  // also orders every warp's occ_acc sums and W-bar tiles before the flushes below
+    if ((WB == 1 && vjp) || lno) flush_wbar(ob_prev, sh, bufG((nbo - 1) & 1), S, o3, o, tid, lno);
     if (WB == 2 && vjp) flush_wbar_bf16(ob_prev, bufG((nbo - 1) & 1), whi, wlo, o3, o, tid);
-    if (vjp) flush_ybar(ob_prev, bufY((nbo - 1) & 1), S + 6 * o3, o, tid);
+    if (vjp) flush_ybar(ob_prev, sh, bufY((nbo - 1) & 1), S + 6 * o3, o);
     if (warp == 0) {
         const bool in = lane < NTHR / 32;
         es = in ? wred[0][lane] : 0.0;
@@ -353,8 +368,12 @@ __global__ void __launch_bounds__(NTHR, 1) epi_pipe_kernel(const WaveView w, con
             }
         }
     }
-    if (vjp)
-        for (int i = tid; i < o; i += NTHR) atomicAdd(&e.mo_energy_bar[i], occ_acc[i]);
+    if (vjp && tid < o) {
+        double x = 0.0;
+#pragma unroll
+        for (int q = 0; q < NTHR / 32; ++q) x += occ_acc[q * 64 + tid];
+        atomicAdd(&e.mo_energy_bar[tid], x);
+    }
 }
 
 template <int WB>
