@@ -144,7 +144,7 @@ __device__ __forceinline__ void store_stage(int s, int np, double *Ws, double *Q
 // One job per CTA.  VJP: the energy, the A12/B12 (slots 2, 3) and A0/B0
 // (slots 4, 5) cubes and the job's mat_bar partial eb C; otherwise the energy.
 template <int NT, typename CT, bool QRT, bool VJP>
-__global__ void __launch_bounds__(Cfg<NT>::NTHR, NT <= 4 ? 2 : 1) proj_kernel(const WaveView w, const EpiArgs e,
+__global__ void __launch_bounds__(Cfg<NT>::NTHR, NT == 2 ? 5 : (NT <= 4 ? 2 : 1)) proj_kernel(const WaveView w, const EpiArgs e,
                                                                              CT *scratch) {
     using C = Cfg<NT>;
     constexpr int R = C::R, S = C::S, SC = C::SC, CG = C::CG;
@@ -324,13 +324,18 @@ static cudaError_t launch_nt(const WaveView &w, const EpiArgs &e, CT *scratch, c
     return cudaGetLastError();
 }
 
-// nocc <= 32: the 4-tile build (256 threads, 44 KB); else the 8-tile one (512 threads, 104 KB)
+// nocc <= 16 / 32 / 48 / 64: 2, 4, 6 or 8 tiles (128 to 512 threads, 20 to 104 KB).
+// VJP projections, ms: nocc=14/nvir=50 5.7 -> 1.5 (two tiles against four), nocc=40/
+// nvir=50 120 -> 64 and, float cubes, 117 -> 61 (six against eight).
 template <typename CT, bool QRT, bool VJP>
 static cudaError_t launch(const WaveView &w, const EpiArgs &e, CT *scratch, cudaStream_t st) {
     if (w.n_jobs <= 0) return cudaSuccess;
     if (!e.lno_mat || e.o < 1 || e.o > 64 || (VJP && !e.lno_mat_bar_part) || (QRT && e.o % 8 != 0))
         return cudaErrorInvalidValue;
-    return e.o <= 32 ? launch_nt<4, CT, QRT, VJP>(w, e, scratch, st) : launch_nt<8, CT, QRT, VJP>(w, e, scratch, st);
+    if (e.o <= 16) return launch_nt<2, CT, QRT, VJP>(w, e, scratch, st);
+    if (e.o <= 32) return launch_nt<4, CT, QRT, VJP>(w, e, scratch, st);
+    if (e.o <= 48) return launch_nt<6, CT, QRT, VJP>(w, e, scratch, st);
+    return launch_nt<8, CT, QRT, VJP>(w, e, scratch, st);
 }
 
 // mat_bar += the jobs' partials: 32 elements per CTA, 32 thread rows taking
