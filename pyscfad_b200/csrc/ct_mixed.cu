@@ -1231,12 +1231,18 @@ static void set_stages(TcParams &P, int a_bytes, int b_bytes, int prec, int kind
 }
 
 // TB, OB1: terms of k K-rows a stage holds.  A stage costs its two issuing threads
-// about 0.4 us whatever it holds, more than a term of up to 16 rows takes otherwise:
-// TF32 t2-bar / vooo-bar 3.27 / 3.23 -> 1.46 / 1.48 ms with four terms at nocc=8/
-// nvir=60, 4.32 / 4.20 -> 3.52 / 3.50 ms with two at nocc=16/nvir=72.
-static int terms_per_stage(int k) { return k <= 8 ? 4 : (k <= 16 ? 2 : 1); }
+// about 0.4 us whatever it holds, more than a short term takes otherwise; past 24
+// rows (TB) or 32 (OB1) fewer, larger stages in flight cost more than that.  t2-bar /
+// vooo-bar in ms, TF32: nocc=8/nvir=60 3.27 / 3.23 (one term) -> 1.41 / 1.47 (four) ->
+// 1.19 / 1.16 (eight); nocc=16/nvir=72 4.32 / 4.20 -> 3.41 / 3.39 (two) -> 2.86 / 2.83
+// (four); nocc=24/nvir=60 3.98 / 4.62 -> 3.72 / 3.77 (two); nocc=32/nvir=60 6.23 / 7.60
+// -> 7.19 / 6.69 (two); vooo-bar of a nocc=48/nvir=300 block 38.4 -> 40.3 (two).
+static int terms_per_stage(int kind, int k) {
+    return k <= 8 ? 8 : (k <= 16 ? 4 : (k <= (kind == TK_TB ? 24 : 32) ? 2 : 1));
+}
 
 template <int KIND, int PREC> static int launch_terms(TcParams &P, int tps, cudaStream_t st) {
+    if (tps == 8) return launch_tc<KIND, PREC, 8>(P, st);
     if (tps == 4) return launch_tc<KIND, PREC, 4>(P, st);
     if (tps == 2) return launch_tc<KIND, PREC, 2>(P, st);
     return launch_tc<KIND, PREC, 1>(P, st);
@@ -1372,6 +1378,7 @@ static int mixed_wave_p(const WaveView &w, const EpiArgs &e, const ct_grads *g, 
             // items of 256 columns; of 128 where those would leave SMs without one
             // (few virtuals and a small o^2): the same sums per element either way
             P.tb_n = w.n_tb_groups * P.m_tiles * (int)((o2 + 255) / 256) < md().sms ? 128 : 256;
+            P.tb_n = std::min(P.tb_n, (int)(o2 + CK - 1) / CK * CK);   // nocc = 8: 64 columns in all
             P.n_tiles = (int)((o2 + P.tb_n - 1) / P.tb_n);
             // a row's last chunk runs into the next row (and past the last row into the
             // vooo copy): virtuals past v, whose output rows are not stored
@@ -1384,7 +1391,7 @@ static int mixed_wave_p(const WaveView &w, const EpiArgs &e, const ct_grads *g, 
             P.groups = w.tb_groups; P.entries = w.tb_entries;
             P.nwork = w.n_tb_groups * P.m_tiles * P.n_tiles;
             P.out = g->t2T;
-            const int tps = terms_per_stage(kp);
+            const int tps = terms_per_stage(TK_TB, kp);
             set_stages(P, tps * (128 / CK) * kp * 128, tps * (P.tb_n / CK) * kp * 128, PREC, TK_TB);
             if (prof) prof(PK_MTB, 0, pctx);
             if ((rc = launch_terms<TK_TB, PREC>(P, tps, st)) != CT_OK) return rc;
@@ -1403,7 +1410,7 @@ static int mixed_wave_p(const WaveView &w, const EpiArgs &e, const ct_grads *g, 
             P.groups = w.xgroups; P.entries = w.x_entries;
             P.nwork = w.n_xgroups * P.m_tiles;
             P.out = g->vooo;
-            const int tps = terms_per_stage(kr8);
+            const int tps = terms_per_stage(TK_OB1, kr8);
             set_stages(P, tps * 128 * kr8 * (PREC ? 2 : 4), tps * ((kr8 + CK - 1) / CK) * o * 128, PREC, TK_OB1);
             if (prof) prof(PK_MOB1, 0, pctx);
             if ((rc = launch_terms<TK_OB1, PREC>(P, tps, st)) != CT_OK) return rc;
