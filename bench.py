@@ -95,9 +95,12 @@ def roofline_units(kind, mode, o, v):
     es = 8 if mode == "fp64" else 4
     if kind in GEMM_OV or kind in GEMM_OO:
         f = 12.0 * o ** 3 * (v if kind in GEMM_OV else o)
+        if kind == 0:
+            f += 12.0 * o ** 4   # the float64 W build takes F2 in the same pass
         return ("tensor", f * (3.0 if mode == "bf16x3" else 1.0), "TFLOP/s")
     if kind == 2:
-        return ("hbm", 13.0 * o ** 3 * es + 12.0 * o * o * es, "GB/s")
+        # float64: six G slots in, three w-bar cubes and ybar out
+        return ("hbm", (10.0 if mode == "fp64" else 13.0) * o ** 3 * es + 12.0 * o * o * es, "GB/s")
     if kind == 3:
         return ("hbm", 3.0 * o ** 3 * es + 12.0 * o * o * 8, "GB/s")
     return ("hbm", 8.0, "GB/s")
