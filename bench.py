@@ -314,9 +314,11 @@ def gpu_arm(args, rank, world, dist):
     if L.ct_peak_probe(1, ctypes.byref(pk)) == 0:
         res["fp64_dfma_peak"] = pk.value
 
-    # CPU baseline (rank 0 at N=1): the reference's compiled kernel on a bounded sample
+    # CPU baseline (rank 0 at N=1): the reference's compiled kernel on a bounded
+    # sample, where it has been built
     cpu = None
-    if rank == 0 and world == 1 and not args.no_cpu:
+    from oracle import ref
+    if rank == 0 and world == 1 and not args.no_cpu and ref.available():
         host = host_inputs(Ld)
         cpu = cpu_reference_sample(host, target_s=12.0)
         del host
@@ -547,7 +549,12 @@ def main():
         if rank != 0:
             return
         import torch
+        from oracle import ref
         from pyscfad_b200 import synth
+        if not ref.available():
+            print(json.dumps({"impl": "reference", "unavailable": "the reference's C kernels are not built "
+                              "(make -C oracle needs its checkout)"}), flush=True)
+            return
         Ld = synth.device_layouts(O, V, NAUX, SEED, device="cuda")
         host = host_inputs(Ld)
         val, info = cpu_reference_sample(host, steps=args.steps, warmup=min(args.warmup, 1))
