@@ -249,6 +249,8 @@ int ct_t3_update(int nocc, int nvir, const double *mo_energy, const double *t3_c
  * The same update from t3 and the occupied Fock block (its diagonal is ignored)
  * instead of from too_m: t3_new = t3_c + (P3(tvv) - P3(foo' t3)) / d3, with the
  * foo' products formed inside.  nocc <= 64.  t3_new must not alias the inputs.
+ * The faster of the two up to nocc = 9 and at even nocc <= 20; past that
+ * ct_t3_update with the product formed as one GEMM (except for small arrays).
  * work: device, CT_T3_STEP_WORK doubles of scratch for the two sums.
  */
 #define CT_T3_STEP_WORK 4096

@@ -12,11 +12,13 @@ The reference forms t3[i,j,k,a,b,c] with JAX einsums.  Here:
     the Fock blocks without their diagonals: fvv' t3 on the first virtual index
     is one plain GEMM (cuBLAS); the foo' products, the P3 sums, the division
     and the fixed-order sums of |t3_new - t3|^2 and of the energy are one
-    kernel (``ct_t3_step``).
+    kernel (``ct_t3_step``).  At sizes where that kernel is the slower one
+    (``_one_kernel_step``) foo' t3 is a GEMM too, on an occupied-major copy of
+    t3 that the update writes for the next step (``ct_t3_update``).
 ``t3`` is returned as the reference's [i,j,k,a,b,c] view.  DIIS (the
 reference's optional ``run_diis``) and the implicit-differentiation backward
 of ``make_implicit_diff`` are not built.  Memory: five (v^3 o^3) float64
-arrays on the device.
+arrays on the device, eight with the occupied-major copies.
 """
 from __future__ import annotations
 
@@ -58,6 +60,22 @@ def _offdiag(f):
     return f
 
 
+def _one_kernel_step(nocc: int, nvir: int) -> bool:
+    """ct_t3_step or, where False, a GEMM for foo' t3 and ct_t3_update.
+
+    The step stages its cubes in shared memory at even nocc <= 20 and is then
+    the faster one at every nvir (a cycle at nocc=8/nvir=40 0.69 against 1.35
+    ms, nocc=20/nvir=28 5.5 against 7.3).  Elsewhere it reads nocc elements of
+    three cubes through L1 for each element: faster than a second GEMM while
+    nocc is small or the arrays are (nocc=9/nvir=28 0.59 against 0.88 ms,
+    nocc=13/nvir=14 0.35 against 0.65, nocc=19/nvir=8 0.56 against 0.69), slower
+    beyond (nocc=13/nvir=28 2.09 against 1.96 ms, nocc=19/nvir=14 1.45 against
+    1.11, nocc=24/nvir=16 4.5 against 2.2, nocc=48/nvir=8 22.5 against 2.7)."""
+    if nocc % 2 == 0:
+        return nocc <= 20
+    return nocc <= 9 or (nocc < 20 and nocc * nocc * nvir <= 3300)
+
+
 def iterative_kernel(mycc, eris=None, t1=None, t2=None, t3=None, max_cycle=50, tol=1e-8, tolnormt=1e-6,
                      verbose=None, stats: dict | None = None):
     """(conv, E, t3) of the iterative (T) solver (pyscfad/cc/ccsd_t_slow.py:262-293).
@@ -88,10 +106,16 @@ def iterative_kernel(mycc, eris=None, t1=None, t2=None, t3=None, max_cycle=50, t
     et = float(torch.sum(cur * t3x))
     tvv, new = torch.empty_like(t3c), torch.empty_like(t3c)
     sums = torch.zeros(2, dtype=torch.float64, device=dev)
-    work = torch.empty(native.T3_STEP_WORK, dtype=torch.float64, device=dev)
+    one = _one_kernel_step(nocc, nvir)
+    if one:
+        work = torch.empty(native.T3_STEP_WORK, dtype=torch.float64, device=dev)
+    else:
+        cur_m = cur.permute(3, 0, 1, 2, 4, 5).contiguous()     # [i][a][b][c][j][k]
+        too_m, new_m = torch.empty_like(t3c), torch.empty_like(t3c)
     conv = False
     ncyc = 0
     ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)] if stats is not None else None
+    ptrs = lambda *ts: [ctypes.c_void_p(x.data_ptr()) for x in ts]  # noqa: E731
     with torch.cuda.device(dev):
         if ev:
             ev[0].record()
@@ -99,9 +123,17 @@ def iterative_kernel(mycc, eris=None, t1=None, t2=None, t3=None, max_cycle=50, t
             ncyc += 1
             # fvv' t3 on the first virtual index; the step forms the foo' products itself
             torch.mm(fvv, cur.view(nvir, -1), out=tvv.view(nvir, -1))
-            p = [ctypes.c_void_p(x.data_ptr()) for x in (L["mo_energy"], foo, t3c, tvv, cur, t3x, new, sums, work)]
-            st = native.lib().ct_t3_step(nocc, nvir, *p, triples._stream(dev))
-            native.check(st, "ct_t3_step")
+            if one:
+                st = native.lib().ct_t3_step(nocc, nvir, *ptrs(L["mo_energy"], foo, t3c, tvv, cur, t3x, new, sums,
+                                                               work), triples._stream(dev))
+                native.check(st, "ct_t3_step")
+            else:
+                # foo' t3 on the first occupied index of the occupied-major copy
+                torch.mm(foo, cur_m.view(nocc, -1), out=too_m.view(nocc, -1))
+                st = native.lib().ct_t3_update(nocc, nvir, *ptrs(L["mo_energy"], t3c, tvv, too_m, cur, t3x, new,
+                                                                 new_m, sums), triples._stream(dev))
+                native.check(st, "ct_t3_update")
+                cur_m, new_m = new_m, cur_m
             normt2, e_new = sums.tolist()
             cur, new = new, cur
             eold, et = et, e_new
