@@ -17,6 +17,7 @@
 // split as (x / div, x % div) and weighted by two strides, which covers every
 // permuted layout above.
 #include <cuda_runtime.h>
+#include <cooperative_groups.h>
 #include <algorithm>
 #include <climits>
 #include "ct_common.cuh"
@@ -40,7 +41,10 @@ __host__ __device__ inline Ix ix_two(int div, long long s1, long long s0) { retu
 
 constexpr int BM = 128, BN = 64, BK = 8, NTHR = 256, STAGES = 4;
 constexpr int LDA = BM + 4, LDB = BN + 4;   // 4 mod 16 doubles: conflict-free fragments
+constexpr int LDC = BN + 2;                  // a part's sums, read by the other CTAs of its cluster
 constexpr size_t kSmem = sizeof(double) * STAGES * BK * (LDA + LDB);
+constexpr size_t kSmemParts = sizeof(double) * BM * LDC > kSmem ? sizeof(double) * BM * LDC : kSmem;
+constexpr int kMaxParts = 8;                 // the portable cluster size
 
 // One operand's slice of a K step: W x BK elements, NL per thread.  MF:
 // consecutive threads take consecutive rows (m or n) of one k, so a thread's
@@ -100,7 +104,7 @@ __global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int
     const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
     Loader<BM, AMF> la;
     Loader<BN, BNF> lb;
-    // gridDim.z parts of K (whole steps); more than one part adds atomically
+    // gridDim.z parts of K (whole steps), one CTA of a cluster each
     const int steps = (K + BK - 1) / BK;
     const int sb = (int)((long long)steps * blockIdx.z / gridDim.z);
     const int nk = (int)((long long)steps * (blockIdx.z + 1) / gridDim.z) - sb;
@@ -137,6 +141,32 @@ __global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int
                 for (int j = 0; j < 4; ++j) dmma(d[i][j], a[i], b[j]);
         }
     }
+    if (gridDim.z > 1) {
+        // the parts' sums meet in the order of the parts, so that the result does
+        // not depend on which CTA ends first: each CTA leaves its tile in shared
+        // memory and adds up its share of the elements
+        cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+        const int parts = gridDim.z;
+        __syncthreads();   // the ring is no longer read
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<double2 *>(dsm + (wm + 8 * i + g) * LDC + wn + 8 * j + 2 * c) =
+                    make_double2(d[i][j][0], d[i][j][1]);
+        cl.sync();
+        for (int e = blockIdx.z * NTHR + threadIdx.x; e < BM * BN; e += parts * NTHR) {
+            const int ml = e / BN, nl = e % BN, m = m0 + ml, n = n0 + nl;
+            if (m >= M || n >= N) continue;
+            double s = 0.0;
+            for (int q = 0; q < parts; ++q) s += cl.map_shared_rank(dsm, q)[ml * LDC + nl];
+            double *dst = C + (long long)(m / cr.div) * cr.s1 + (long long)(m % cr.div) * cr.s0 +
+                          (long long)(n / cc.div) * cc.s1 + (long long)(n % cc.div) * cc.s0;
+            *dst = acc ? *dst + alpha * s : alpha * s;
+        }
+        cl.sync();   // no CTA leaves while another reads its tile
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int m = m0 + wm + 8 * i + g;
@@ -149,8 +179,7 @@ __global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int
                 const int n = n0 + wn + 8 * j + 2 * c + h;
                 if (n >= N) continue;
                 double *dst = C + rm + (long long)(n / cc.div) * cc.s1 + (long long)(n % cc.div) * cc.s0;
-                if (gridDim.z > 1) atomicAdd(dst, alpha * d[i][j][h]);
-                else *dst = acc ? *dst + alpha * d[i][j][h] : alpha * d[i][j][h];
+                *dst = acc ? *dst + alpha * d[i][j][h] : alpha * d[i][j][h];
             }
     }
 }
@@ -163,12 +192,24 @@ static cudaError_t gemm(int M, int N, int K, const Opd &A, const Opd &B, double 
     // An accumulating product with few tiles (the factor gradients: naux rows)
     // splits K so that two CTAs per SM have work, each part >= 64 steps
     const long long tiles = (long long)grid.x * grid.y;
-    if (acc && tiles < 296) grid.z = (unsigned)std::max(1LL, std::min(592 / tiles, (long long)K / (64 * BK)));
+    if (acc && tiles < 296)
+        grid.z = (unsigned)std::max(1LL, std::min(std::min<long long>(592 / tiles, kMaxParts), (long long)K / (64 * BK)));
+    const size_t smem = grid.z > 1 ? kSmemParts : kSmem;
     auto go = [&](auto kern) {
-        const cudaError_t ce = smem_optin(reinterpret_cast<const void *>(kern), (int)kSmem);
+        const cudaError_t ce = smem_optin(reinterpret_cast<const void *>(kern), (int)smem);
         if (ce != cudaSuccess) return ce;
-        kern<<<grid, NTHR, kSmem, st>>>(M, N, K, A, B, C, cr, cc, alpha, acc ? 1 : 0);
-        return cudaGetLastError();
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(NTHR);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = at.val.clusterDim.y = 1;
+        at.val.clusterDim.z = grid.z;
+        cfg.attrs = &at;
+        cfg.numAttrs = grid.z > 1 ? 1 : 0;
+        return cudaLaunchKernelEx(&cfg, kern, M, N, K, A, B, C, cr, cc, alpha, acc ? 1 : 0);
     };
     // consecutive threads along the operand's contiguous index
     if (A.r.s0 == 1) return B.c.s0 == 1 ? go(gemm_strided_kernel<true, true>) : go(gemm_strided_kernel<true, false>);
