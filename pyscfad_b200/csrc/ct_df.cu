@@ -20,6 +20,7 @@
 #include <cooperative_groups.h>
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include "ct_common.cuh"
 #include "ct_internal.h"
 #include "../../include/pyscfad_b200.h"
@@ -39,12 +40,11 @@ struct Opd {
 __host__ __device__ inline Ix ix_plain(long long s) { return Ix{INT_MAX, 0, s}; }
 __host__ __device__ inline Ix ix_two(int div, long long s1, long long s0) { return Ix{div, s1, s0}; }
 
-constexpr int BM = 128, BN = 64, BK = 8, NTHR = 256, STAGES = 4;
-constexpr int LDA = BM + 4, LDB = BN + 4;   // 4 mod 16 doubles: conflict-free fragments
+constexpr int BN = 64, BK = 16, NTHR = 256, STAGES = 3;
 constexpr int LDC = BN + 2;                  // a part's sums, read by the other CTAs of its cluster
-constexpr size_t kSmem = sizeof(double) * STAGES * BK * (LDA + LDB);
-constexpr size_t kSmemParts = sizeof(double) * BM * LDC > kSmem ? sizeof(double) * BM * LDC : kSmem;
-constexpr int kMaxParts = 8;                 // the portable cluster size
+// 4 mod 16 doubles per row: conflict-free fragments
+constexpr size_t ring_bytes(int bm) { return sizeof(double) * STAGES * BK * (bm + 4 + BN + 4); }
+static_assert(sizeof(double) * 64 * LDC <= ring_bytes(64), "a part's tile takes the ring's place");
 
 // One operand's slice of a K step: W x BK elements, NL per thread.  MF:
 // consecutive threads take consecutive rows (m or n) of one k, so a thread's
@@ -89,19 +89,24 @@ template <int W, bool MF> struct Loader {
     }
 };
 
-// C[m,n] = alpha sum_k A[m,k] B[k,n] (+ C[m,n] when acc); 128 x 64 tiles, 8 warps
-// of 32 x 32 (4 x 4 DMMA tiles), K steps of 8 in a four-stage cp.async ring.
-// Bound by the DMMA pipe: a 64 x 64 tile with one shared buffer and 8 DMMAs per
-// six fragment loads ran the nocc=16/nvir=120/naux=360 producer and its VJP
-// (69 GFLOP) in 4.6 ms of kernels, this one in 3.3 ms (21 of 37 TFLOP/s).
-template <bool AMF, bool BNF>
+// C[m,n] = alpha sum_k A[m,k] B[k,n] (+ C[m,n] when acc); BM x 64 tiles, 8 warps
+// of 32 x (BM / 4), K steps of 16 in a three-stage cp.async ring.  BM = 64 for
+// few tiles and for sums in parts, 128 for many (launch_cost below).  Few tiles
+// are bound by the latency of a K step: one step of a lone CTA takes 1.1 us with
+// 64 rows and 1.8 with 128 (K steps of 8 with 128 rows, in four stages, 0.9 for
+// half the K).  Many are bound by the DMMA pipe: the vvop product of
+// nocc=16/nvir=120/naux=360 takes 0.96 ms with 128 rows (23 of 37 TFLOP/s), 1.03
+// with 64 and 0.99 with 128 and steps of 8; a 64 x 64 tile with one shared buffer
+// took 1.04.
+template <int BM, bool AMF, bool BNF>
 __global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int K, Opd A, Opd B, double *C, Ix cr,
                                                                Ix cc, double alpha, int acc) {
+    constexpr int LDA = BM + 4, LDB = BN + 4, WN = BM / 4, NT = WN / 8;
     extern __shared__ __align__(16) double dsm[];
     double *As = dsm, *Bs = dsm + STAGES * BK * LDA;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+    const int wm = (warp / (BN / WN)) * 32, wn = (warp % (BN / WN)) * WN;
     Loader<BM, AMF> la;
     Loader<BN, BNF> lb;
     // gridDim.z parts of K (whole steps), one CTA of a cluster each
@@ -110,11 +115,11 @@ __global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int
     const int nk = (int)((long long)steps * (blockIdx.z + 1) / gridDim.z) - sb;
     la.init(A.r, A.c, m0, M, sb * BK);
     lb.init(B.c, B.r, n0, N, sb * BK);
-    double d[4][4][2];
+    double d[4][NT][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) d[i][j][0] = d[i][j][1] = 0.0;
+        for (int j = 0; j < NT; ++j) d[i][j][0] = d[i][j][1] = 0.0;
     auto issue = [&](int s) {
         if (s < nk) {
             la.copy(As + (s % STAGES) * BK * LDA, A.p, A.c, (sb + s) * BK, K);
@@ -132,16 +137,18 @@ __global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int
         const double *b_ = Bs + (s % STAGES) * BK * LDB + c * LDB + wn + g;
 #pragma unroll
         for (int kk = 0; kk < BK; kk += 4) {
-            double a[4], b[4];
+            double a[4], b[NT];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { a[i] = a_[kk * LDA + 8 * i]; b[i] = b_[kk * LDB + 8 * i]; }
+            for (int i = 0; i < 4; ++i) a[i] = a_[kk * LDA + 8 * i];
+#pragma unroll
+            for (int j = 0; j < NT; ++j) b[j] = b_[kk * LDB + 8 * j];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) dmma(d[i][j], a[i], b[j]);
+                for (int j = 0; j < NT; ++j) dmma(d[i][j], a[i], b[j]);
         }
     }
-    if (gridDim.z > 1) {
+    if (BM == 64 && gridDim.z > 1) {
         // the parts' sums meet in the order of the parts, so that the result does
         // not depend on which CTA ends first: each CTA leaves its tile in shared
         // memory and adds up its share of the elements
@@ -151,7 +158,7 @@ __global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < NT; ++j)
                 *reinterpret_cast<double2 *>(dsm + (wm + 8 * i + g) * LDC + wn + 8 * j + 2 * c) =
                     make_double2(d[i][j][0], d[i][j][1]);
         cl.sync();
@@ -173,7 +180,7 @@ __global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int
         if (m >= M) continue;
         const long long rm = (long long)(m / cr.div) * cr.s1 + (long long)(m % cr.div) * cr.s0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < NT; ++j)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int n = n0 + wn + 8 * j + 2 * c + h;
@@ -184,36 +191,73 @@ __global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int
     }
 }
 
+// Time of CTAs on `slots` single places (two a place share its SM's DMMA pipe) in
+// units of one CTA's: a pair takes 2, a last one alone 1.4.
+static double launch_cost(double ctas, double slots) {
+    const int n = (int)std::ceil(ctas / slots);
+    return 2.0 * (n / 2) + (n % 2 ? 1.4 : 0.0);
+}
+
+// The numbers of parts of a K sum, and the CTAs that are resident in clusters of so
+// many, of all (cudaOccupancyMaxActiveClusters on 148 SMs: a cluster stays within a
+// GPC, whose SMs do not divide by every size; 35 tiles of K 10,400 take 221 us
+// in eight parts and 163 in seven).
+constexpr int kNumParts = 6, kParts[kNumParts] = {1, 2, 3, 4, 6, 8};
+constexpr double kResident[kNumParts] = {1.0, 1.0, 279.0 / 296, 284.0 / 296, 270.0 / 296, 264.0 / 296};
+
+template <int BM>
+static cudaError_t launch(int M, int N, int K, const Opd &A, const Opd &B, double *C, Ix cr, Ix cc, double alpha,
+                          bool acc, int parts, cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((N + BN - 1) / BN, (M + BM - 1) / BM, parts);
+    if (cfg.gridDim.y > 65535) return cudaErrorInvalidValue;
+    cfg.blockDim = dim3(NTHR);
+    cfg.dynamicSmemBytes = ring_bytes(BM);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = parts;
+    cfg.attrs = &at;
+    cfg.numAttrs = parts > 1 ? 1 : 0;
+    auto go = [&](auto kern) {
+        const cudaError_t ce = smem_optin(reinterpret_cast<const void *>(kern), (int)ring_bytes(BM));
+        return ce != cudaSuccess ? ce : cudaLaunchKernelEx(&cfg, kern, M, N, K, A, B, C, cr, cc, alpha, acc ? 1 : 0);
+    };
+    // consecutive threads along the operand's contiguous index
+    if (A.r.s0 == 1)
+        return B.c.s0 == 1 ? go(gemm_strided_kernel<BM, true, true>) : go(gemm_strided_kernel<BM, true, false>);
+    return B.c.s0 == 1 ? go(gemm_strided_kernel<BM, false, true>) : go(gemm_strided_kernel<BM, false, false>);
+}
+
 static cudaError_t gemm(int M, int N, int K, const Opd &A, const Opd &B, double *C, Ix cr, Ix cc, double alpha,
                         bool acc, cudaStream_t st) {
     if (M <= 0 || N <= 0 || K <= 0) return cudaSuccess;
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    if (grid.y > 65535) return cudaErrorInvalidValue;
-    // An accumulating product with few tiles (the factor gradients: naux rows)
-    // splits K so that two CTAs per SM have work, each part >= 64 steps
-    const long long tiles = (long long)grid.x * grid.y;
-    if (acc && tiles < 296)
-        grid.z = (unsigned)std::max(1LL, std::min(std::min<long long>(592 / tiles, kMaxParts), (long long)K / (64 * BK)));
-    const size_t smem = grid.z > 1 ? kSmemParts : kSmem;
-    auto go = [&](auto kern) {
-        const cudaError_t ce = smem_optin(reinterpret_cast<const void *>(kern), (int)smem);
-        if (ce != cudaSuccess) return ce;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = grid;
-        cfg.blockDim = dim3(NTHR);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute at{};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = at.val.clusterDim.y = 1;
-        at.val.clusterDim.z = grid.z;
-        cfg.attrs = &at;
-        cfg.numAttrs = grid.z > 1 ? 1 : 0;
-        return cudaLaunchKernelEx(&cfg, kern, M, N, K, A, B, C, cr, cc, alpha, acc ? 1 : 0);
-    };
-    // consecutive threads along the operand's contiguous index
-    if (A.r.s0 == 1) return B.c.s0 == 1 ? go(gemm_strided_kernel<true, true>) : go(gemm_strided_kernel<true, false>);
-    return B.c.s0 == 1 ? go(gemm_strided_kernel<false, true>) : go(gemm_strided_kernel<false, false>);
+    int dev = 0, sms = 0;
+    cudaError_t ce = cudaGetDevice(&dev);
+    if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (ce != cudaSuccess) return ce;
+    const long long nt = (N + BN - 1) / BN, t64 = nt * ((M + 63) / 64), t128 = nt * ((M + 127) / 128);
+    // An accumulating product (the factor gradients: naux rows, long K) takes the
+    // number of K parts with the least launch cost x K per part, where a part's
+    // start and its share of the sum cost as much as 64 rows of K.  Over 148 products
+    // of nocc 2-48 / nvir 20-250 the choice is 2% behind the best number of parts on
+    // average (25% at most, below 20 us) and at no size behind one 64 x 64 tile with
+    // one shared buffer.  E.g. dLov of nocc=8/nvir=60/naux=204 (32 tiles, K 4080):
+    // 62 us in eight parts, 292 in one, 314 with the shared buffer.
+    int parts = 1;
+    if (acc) {
+        double best = 0.0;
+        for (int i = 0; i < kNumParts; ++i) {
+            const int z = kParts[i], rows = (K + BK * z - 1) / (BK * z) * BK + 64;
+            const double cost = launch_cost((double)t64 * z, sms * kResident[i]) * rows;
+            if (i == 0 || cost < best) { best = cost; parts = z; }
+        }
+    }
+    // 128-row tiles do a tile pair's work in 1.85 of one tile's time, where they fill the rounds of the GPU
+    if (parts == 1 && 1.85 * launch_cost((double)t128, sms) < launch_cost((double)t64, sms))
+        return launch<128>(M, N, K, A, B, C, cr, cc, alpha, acc, 1, st);
+    return launch<64>(M, N, K, A, B, C, cr, cc, alpha, acc, parts, st);
 }
 
 }  // namespace df
