@@ -539,6 +539,21 @@ static double scratch_budget_mb(Workspace &W) {
 }
 
 static bool use_cube(int o, int mode) { return mode == CT_MODE_FP64 && cube_size(o); }
+// An energy over few jobs with many virtuals takes the slot path: on the cube path
+// one CTA per job walks the whole F1 sum alone, the slot path cuts a job into 3 nocc / 2
+// CTAs.  Job lists in us, cube against slots.  While SMs are idle the slots are the
+// faster (one job: nocc=4/nvir=200 191 / 147, nocc=20/nvir=300 467 / 193; 100 jobs:
+// nocc=16/nvir=200 302 / 237, nocc=22/nvir=200 469 / 409), with more virtuals up to
+// more jobs (148 jobs: nvir=128 nocc=17 283 / 348, nvir=300 553 / 512).  From nvir =
+// 256 they stay so up to 5 / 4 nvir jobs (300 jobs: nocc=20/nvir=300 1291 / 938,
+// nocc=8/nvir=450 465 / 388), except at nocc 17-19, where two cube CTAs run per
+// SM (200 jobs at nocc=18/nvir=300 591 / 639).  At nvir=80 the two are within 70 us
+// of each other.
+static bool few_jobs(const Workspace &W, long long jobs, int o, int v) {
+    if (v < 128) return false;
+    if (256 * jobs <= (long long)W.sm_count * std::min(v, 256)) return true;
+    return v >= 256 && 4 * jobs <= 5LL * v && (o <= 16 || o >= 20);
+}
 
 // Jobs per wave: as many as the scratch budget holds (at most 8192), rounded
 // down to a multiple of two CTAs per SM so the per-job kernels fill whole
@@ -643,8 +658,9 @@ static int run_waves(Workspace &W, const Plan &P, const ct_problem *p, int mode,
                      const EpiArgs &ea, const MixedOperands &mo, double *lno_mat_bar, cudaStream_t st) {
     const int o = p->nocc, v = p->nvir, n = o + v;
     const double *lno_mat = ea.lno_mat;
-    const bool cube = use_cube(o, mode) && !ea.t3_c;
-    if (cube && !vjp && !lno_mat) {
+    const bool energy = !vjp && !lno_mat;
+    const bool cube = use_cube(o, mode) && !ea.t3_c && !(energy && few_jobs(W, (long long)P.jobs.size(), o, v));
+    if (cube && energy) {
         // no scratch: every job of the plan in one launch
         CT_PROF(PK_F1);
         CT_CK(cube_energy(P.d_jobs, (int)P.jobs.size(), ea, p->vooo, st));
