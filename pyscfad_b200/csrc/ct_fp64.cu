@@ -635,8 +635,10 @@ cudaError_t f32_vterm(const WaveView &w, const EpiArgs &e, const float *scratch,
 // CTA sums a fixed contiguous chunk (Neumaier pairs, merged down fixed shuffle
 // trees), then one CTA merges the partials the same way.  A single thread
 // merging the 2048 values of its CTA, and one more the 256 partials, took 57 us
-// whatever n was; the trees take 6 us at n = 220 and 9 us at n = 295,240.
-constexpr int kRedThreads = 256;
+// whatever n was; the trees take 6 us at n = 220 and 9 us at n = 295,240.  Past a
+// million values the adds of a thread are the time: 1024 threads a CTA there
+// (n = 1.67e8, nvir = 1000: 251 us against 574 with 256, and 295 of the serial merge).
+constexpr int kRedThreads = 256, kRedThreadsLong = 1024;
 
 // the pair (s, c) of a CTA's threads merged in a fixed order; valid in thread 0
 __device__ __forceinline__ KSum block_ksum(KSum k) {
@@ -661,12 +663,13 @@ __device__ __forceinline__ KSum block_ksum(KSum k) {
 }
 
 // out: nullable; with it (a single CTA) the sum itself, else this CTA's pair into part
-__global__ void __launch_bounds__(kRedThreads) reduce_energy_part_kernel(const double *job_e, long long n,
+__global__ void __launch_bounds__(kRedThreadsLong) reduce_energy_part_kernel(const double *job_e, long long n,
                                                                          double *part, double *out) {
     const long long chunk = (n + gridDim.x - 1) / gridDim.x;
     const long long lo = blockIdx.x * chunk, hi = lo + chunk < n ? lo + chunk : n;
     KSum k;
-    for (long long i = lo + threadIdx.x; i < hi; i += kRedThreads) k.add(job_e[i]);
+#pragma unroll 4
+    for (long long i = lo + threadIdx.x; i < hi; i += blockDim.x) k.add(job_e[i]);
     k = block_ksum(k);
     if (threadIdx.x == 0) {
         if (out) {
@@ -705,7 +708,8 @@ cudaError_t reduce_energy_1cta(const double *job_e, long long n, double *e_out, 
 cudaError_t reduce_energy(const double *job_e, long long n, double *e_out, double *work, cudaStream_t st) {
     // one CTA up to 8 values a thread (the second launch costs more than it saves)
     const int parts = n <= 8 * kRedThreads ? 1 : (int)(n / kRedThreads < kReduceParts ? n / kRedThreads : kReduceParts);
-    reduce_energy_part_kernel<<<parts, kRedThreads, 0, st>>>(job_e, n, work, parts == 1 ? e_out : nullptr);
+    const int threads = n > (1LL << 20) ? kRedThreadsLong : kRedThreads;
+    reduce_energy_part_kernel<<<parts, threads, 0, st>>>(job_e, n, work, parts == 1 ? e_out : nullptr);
     if (parts > 1) reduce_energy_final_kernel<<<1, kRedThreads, 0, st>>>(work, parts, e_out);
     return cudaGetLastError();
 }
