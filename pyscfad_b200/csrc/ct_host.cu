@@ -424,8 +424,6 @@ struct Workspace {
     int n_orb = 0;
     double *e_tmp = nullptr;
     double *red_work = nullptr;     // 2 * kReduceParts partial sums
-    double *lno_part = nullptr;     // LNO VJP: per-job partials of mat_bar, one wave
-    long long lno_part_n = 0;
     HostPathCache hp;
     Prof prof;
     cudaEvent_t prof_open[kProfKinds] = {};
@@ -443,9 +441,6 @@ struct Workspace {
         if (orbits) cudaFree(orbits);
         if (e_tmp) cudaFree(e_tmp);
         if (red_work) cudaFree(red_work);
-        if (lno_part) cudaFree(lno_part);
-        lno_part = nullptr;
-        lno_part_n = 0;
         scratch = nullptr; job_e = nullptr; orbits = nullptr; e_tmp = nullptr; red_work = nullptr;
         scratch_bytes = 0; job_e_n = 0; orb_o = -1; n_orb = 0;
         hp.release();
@@ -571,9 +566,21 @@ static int max_wave_jobs(Workspace &W, int o, int mode) {
     return (int)mw;
 }
 
+// the wave scratch: the jobs' slots (and the BF16x3 planes behind them), then one
+// wave's partials of an LNO VJP's mat_bar.  Every call holds all of it, so that
+// after any call at this nocc and mode no other one allocates it (a call under stream
+// capture must not).
+static size_t slots_bytes(int o, int mode, int max_wave) {
+    const size_t b = (size_t)max_wave * kSlots * (size_t)o * o * o * scratch_elt(mode)
+                   + (mode == CT_MODE_FP64 ? 0 : (size_t)(max_wave * mixed_extra_bytes_per_job(o, mode)));
+    return (b + 15) / 16 * 16;
+}
+static size_t scratch_need(int o, int mode, int max_wave) {
+    return slots_bytes(o, mode, max_wave) + (size_t)max_wave * o * o * sizeof(double);
+}
+
 static int ensure_common(Workspace &W, int o, int v, int mode, int max_wave) {
-    const size_t need = (size_t)max_wave * kSlots * (size_t)o * o * o * scratch_elt(mode)
-                      + (mode == CT_MODE_FP64 ? 0 : (size_t)(max_wave * mixed_extra_bytes_per_job(o, mode)));
+    const size_t need = scratch_need(o, mode, max_wave);
     if (need > W.scratch_bytes) {
         if (W.scratch) cudaFree(W.scratch);
         W.scratch = nullptr;
@@ -965,20 +972,12 @@ static int run_lno_vjp_locked(Workspace &W, const ct_problem *p, int mode, const
         if ((rc = upload_plan(W.block)) != CT_OK) { W.block.free_dev(); W.block = Plan(); return rc; }
         P = &W.block;
     }
-    const long long n_part = (long long)mw * p->nocc * p->nocc;
-    if (n_part > W.lno_part_n) {
-        if (W.lno_part) cudaFree(W.lno_part);
-        W.lno_part = nullptr;
-        W.lno_part_n = 0;
-        CT_CK(cudaMalloc(&W.lno_part, n_part * sizeof(double)));
-        W.lno_part_n = n_part;
-    }
     LnoSel sel;
     sel.mat = mat;
     sel.a0 = 0; sel.a1 = v;
     sel.b0 = b0; sel.b1 = b1; sel.c0 = c0; sel.c1 = c1;
     sel.mat_bar = mat_bar;
-    sel.part = W.lno_part;
+    sel.part = reinterpret_cast<double *>(static_cast<char *>(W.scratch) + slots_bytes(p->nocc, mode, mw));
     return run_plan(W, *P, p, mode, true, et_bar, g, W.job_e, e_out, st, &sel);
 }
 
@@ -1145,8 +1144,7 @@ long long ct_workspace_bytes(int nocc, int nvir, int mode, int with_vjp) {
         Workspace tmp;   // no device: the default budget and SM count
         mw = max_wave_jobs(tmp, nocc, mode);
     }
-    return mw * kSlots * (long long)nocc * nocc * nocc * (long long)scratch_elt(mode)
-         + (mode == CT_MODE_FP64 ? 0 : (long long)(mw * mixed_extra_bytes_per_job(nocc, mode)))
+    return (long long)scratch_need(nocc, mode, (int)mw)
          + (mode == CT_MODE_FP64 ? 0 : (long long)mixed_operand_bytes(nocc, nvir, mode))
          + n_sorted(nvir) * 8LL + (long long)nocc * nocc * nocc * 4LL;
 }
