@@ -84,6 +84,7 @@ def flops_per_job(o, v):
 # profiled kernel kinds (ct_profile_read ids) of the tensor-core contractions
 GEMM_OV = {0, 4, 5, 10, 11, 12}      # 12 o^3 v flops per job (F1, VB, TB)
 GEMM_OO = {1, 6, 7, 13, 14, 15}      # 12 o^4 flops per job (F2, OB1, OB2)
+CUBE_MAX_O = 24                      # float64 at nocc 2..CUBE_MAX_O: one kernel per job (ct_cube.cu)
 
 
 def roofline_units(kind, mode, o, v):
@@ -91,8 +92,11 @@ def roofline_units(kind, mode, o, v):
     the contractions (bf16x3 issues three bf16 products per product, counted
     as issued tensor flops), bytes for the orbit epilogue (reads the six
     G slots and the V-term tiles, writes the six W-bar slots and ybar) and
-    the V-term kernel (reads ybar once per axis)."""
+    the V-term kernel (reads ybar once per axis).  Float64 at nocc 2-24: kind 0
+    is the whole job kernel of a VJP, every contraction but the t2-bar GEMM."""
     es = 8 if mode == "fp64" else 4
+    if kind == 0 and mode == "fp64" and 2 <= o <= CUBE_MAX_O:
+        return ("tensor", 12.0 * o ** 3 * (2 * v + 3 * o), "TFLOP/s")
     if kind in GEMM_OV or kind in GEMM_OO:
         f = 12.0 * o ** 3 * (v if kind in GEMM_OV else o)
         if kind == 0:
@@ -262,6 +266,8 @@ def gpu_arm(args, rank, world, dist):
                   7: "t2 vooo-bar GEMM (OB2)", 8: "energy reduction", 9: "mixed operand prep",
                   10: "tcgen05 W-build GEMM", 11: "tcgen05 vvop-bar GEMM", 12: "tcgen05 t2-bar GEMM",
                   13: "tcgen05 vooo W term (F2)", 14: "tcgen05 vooo-bar GEMM (OB1)", 15: "tcgen05 t2 vooo-bar GEMM (OB2)"}
+    if mode == "fp64" and 2 <= O <= CUBE_MAX_O:
+        kind_names[0] = "job kernel (W, epilogue, V-term, VB, OB1, OB2)"
     dom = max(prof, key=lambda k: prof[k][0]) if prof else None
     res["dominant"] = dom
     if dom is not None:
