@@ -31,6 +31,17 @@ def _time(fn, reps):
     return t0.elapsed_time(t1) / reps
 
 
+def kind_names(mode: str, nocc: int) -> dict:
+    """Names of the profile kinds (ct_profile_read) of an LNO call.  Float64 at
+    nocc 2-24 runs a job's passes in one kernel each (ct_cube.cu)."""
+    kinds = {0: "W build", 2: "orbit epilogue", 3: "V-term / LNO energy projection", 4: "VB", 5: "TB", 6: "OB1",
+             7: "OB2", 8: "reductions / LNO VJP projection", 9: "operand preparation", 10: "F1 (tcgen05)",
+             11: "VB (tcgen05)", 12: "TB (tcgen05)", 13: "F2 (tcgen05)", 14: "OB1 (tcgen05)", 15: "OB2 (tcgen05)"}
+    if mode == "fp64" and 2 <= nocc <= 24:
+        kinds.update({0: "job kernel, forward pass", 3: "LNO energy projection", 4: "job kernel, backward pass"})
+    return kinds
+
+
 def main(argv=None):
     ap = argparse.ArgumentParser()
     ap.add_argument("--nocc", type=int, default=32)
@@ -53,10 +64,7 @@ def main(argv=None):
     }
     # per-kernel device time of one LNO energy call and one LNO VJP call
     L_ = native.lib()
-    kinds = {0: "F1", 1: "F2", 2: "orbit epilogue", 3: "V-term / LNO energy projection", 4: "VB", 5: "TB",
-             6: "OB1", 7: "OB2", 8: "reductions / LNO VJP projection", 9: "operand preparation",
-             10: "F1 (tcgen05)", 11: "VB (tcgen05)", 12: "TB (tcgen05)", 13: "F2 (tcgen05)", 14: "OB1 (tcgen05)",
-             15: "OB2 (tcgen05)"}
+    kinds = kind_names(a.mode, a.nocc)
     runs = [("lno_energy", lambda: triples.lno_energy(L, mat, mode=a.mode)),
             ("lno_energy_vjp", lambda: triples.lno_energy_vjp(L, mat, 1.0, grads, mb, mode=a.mode))]
     for name, fn in runs:
