@@ -22,3 +22,11 @@ def test_bars_match_fp64(o, v, mode, cuda_dev):
     for k in ("t2T", "vooo", "vvop"):
         err = float(torch.linalg.norm(g[k] - g64[k]))
         assert err <= GRAD_TOL[mode] * float(torch.linalg.norm(g64[k])), (k, err)
+
+
+@pytest.mark.parametrize("mode", ["tf32", "bf16x3"])
+@pytest.mark.parametrize("o,v", [(32, 3), (32, 8), (8, 30), (16, 21), (48, 4)])
+def test_bars_match_fp64_by_terms_per_stage(o, v, mode, cuda_dev):
+    """nocc 32 (two terms of vooo-bar, one of t2-bar a stage), eight and four terms
+    a stage over lists that do not divide by them, one term at nocc 48."""
+    test_bars_match_fp64(o, v, mode, cuda_dev)
