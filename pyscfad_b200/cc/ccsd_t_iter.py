@@ -102,7 +102,9 @@ def iterative_kernel(mycc, eris=None, t1=None, t2=None, t3=None, max_cycle=50, t
     if t3 is None:
         cur = t3c.clone()
     else:
-        cur = torch.as_tensor(t3, dtype=torch.float64).to(dev).permute(3, 4, 5, 0, 1, 2).contiguous()
+        # a copy: the cycles write both of their arrays, and a t3 of this solver is a view of one
+        cur = torch.as_tensor(t3, dtype=torch.float64).to(dev).permute(3, 4, 5, 0, 1, 2)
+        cur = cur.clone(memory_format=torch.contiguous_format)
     et = float(torch.sum(cur * t3x))
     tvv, new = torch.empty_like(t3c), torch.empty_like(t3c)
     sums = torch.zeros(2, dtype=torch.float64, device=dev)
