@@ -42,9 +42,10 @@ __host__ __device__ inline Ix ix_two(int div, long long s1, long long s0) { retu
 
 constexpr int BN = 64, BK = 16, NTHR = 256, STAGES = 3;
 constexpr int LDC = BN + 2;                  // a part's sums, read by the other CTAs of its cluster
-// 4 mod 16 doubles per row: conflict-free fragments
-constexpr size_t ring_bytes(int bm) { return sizeof(double) * STAGES * BK * (bm + 4 + BN + 4); }
-static_assert(sizeof(double) * 64 * LDC <= ring_bytes(64), "a part's tile takes the ring's place");
+constexpr int kFold = 32;                    // K steps after which the sums fold
+// the ring, 4 mod 16 doubles per row (conflict-free fragments), and the sums behind it
+constexpr int ring_doubles(int bm) { return STAGES * BK * (bm + 4 + BN + 4); }
+constexpr size_t smem_bytes(int bm, bool sums) { return sizeof(double) * (size_t)(ring_doubles(bm) + (sums ? bm * LDC : 0)); }
 
 // One operand's slice of a K step: W x BK elements, NL per thread.  MF:
 // consecutive threads take consecutive rows (m or n) of one k, so a thread's
@@ -98,12 +99,14 @@ template <int W, bool MF> struct Loader {
 // nocc=16/nvir=120/naux=360 takes 0.96 ms with 128 rows (23 of 37 TFLOP/s), 1.03
 // with 64 and 0.99 with 128 and steps of 8; a 64 x 64 tile with one shared buffer
 // took 1.04.
+// The sums of the 64-row build fold and may run in parts.
 template <int BM, bool AMF, bool BNF>
 __global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int K, Opd A, Opd B, double *C, Ix cr,
                                                                Ix cc, double alpha, int acc) {
     constexpr int LDA = BM + 4, LDB = BN + 4, WN = BM / 4, NT = WN / 8;
+    constexpr bool SUMS = BM == 64;
     extern __shared__ __align__(16) double dsm[];
-    double *As = dsm, *Bs = dsm + STAGES * BK * LDA;
+    double *As = dsm, *Bs = dsm + STAGES * BK * LDA, *Cs = dsm + ring_doubles(BM);
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
     const int wm = (warp / (BN / WN)) * 32, wn = (warp % (BN / WN)) * WN;
@@ -129,7 +132,26 @@ __global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int
     };
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) issue(s);
+    // the accumulators are folded into this thread's elements of Cs every kFold
+    // steps: a chain of K / 4 additions loses up to sqrt(K / 512) more (dLov of
+    // nocc=16/nvir=120/naux=360, K 16,320: 7e-16 of the norm against 4.4e-15 in one
+    // chain), for 1% of the time
+    bool folded = false;
+    auto each = [&](auto f) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+                f(*reinterpret_cast<double2 *>(Cs + (wm + 8 * i + g) * LDC + wn + 8 * j + 2 * c), d[i][j]);
+    };
     for (int s = 0; s < nk; ++s) {
+        if (SUMS && s > 0 && s % kFold == 0) {
+            each([&](double2 &x, double (&y)[2]) {
+                x = folded ? make_double2(x.x + y[0], x.y + y[1]) : make_double2(y[0], y[1]);
+                y[0] = y[1] = 0.0;
+            });
+            folded = true;
+        }
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         __syncthreads();   // step s landed for every thread; step s - 1's buffer is free
         issue(s + STAGES - 1);
@@ -148,25 +170,21 @@ __global__ void __launch_bounds__(NTHR, 2) gemm_strided_kernel(int M, int N, int
                 for (int j = 0; j < NT; ++j) dmma(d[i][j], a[i], b[j]);
         }
     }
-    if (BM == 64 && gridDim.z > 1) {
+    if (SUMS && folded)
+        each([&](double2 &x, double (&y)[2]) { y[0] += x.x; y[1] += x.y; });
+    if (SUMS && gridDim.z > 1) {
         // the parts' sums meet in the order of the parts, so that the result does
         // not depend on which CTA ends first: each CTA leaves its tile in shared
         // memory and adds up its share of the elements
         cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
         const int parts = gridDim.z;
-        __syncthreads();   // the ring is no longer read
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < NT; ++j)
-                *reinterpret_cast<double2 *>(dsm + (wm + 8 * i + g) * LDC + wn + 8 * j + 2 * c) =
-                    make_double2(d[i][j][0], d[i][j][1]);
+        each([&](double2 &x, double (&y)[2]) { x = make_double2(y[0], y[1]); });
         cl.sync();
         for (int e = blockIdx.z * NTHR + threadIdx.x; e < BM * BN; e += parts * NTHR) {
             const int ml = e / BN, nl = e % BN, m = m0 + ml, n = n0 + nl;
             if (m >= M || n >= N) continue;
             double s = 0.0;
-            for (int q = 0; q < parts; ++q) s += cl.map_shared_rank(dsm, q)[ml * LDC + nl];
+            for (int q = 0; q < parts; ++q) s += cl.map_shared_rank(Cs, q)[ml * LDC + nl];
             double *dst = C + (long long)(m / cr.div) * cr.s1 + (long long)(m % cr.div) * cr.s0 +
                           (long long)(n / cc.div) * cc.s1 + (long long)(n % cc.div) * cc.s0;
             *dst = acc ? *dst + alpha * s : alpha * s;
@@ -212,7 +230,8 @@ static cudaError_t launch(int M, int N, int K, const Opd &A, const Opd &B, doubl
     cfg.gridDim = dim3((N + BN - 1) / BN, (M + BM - 1) / BM, parts);
     if (cfg.gridDim.y > 65535) return cudaErrorInvalidValue;
     cfg.blockDim = dim3(NTHR);
-    cfg.dynamicSmemBytes = ring_bytes(BM);
+    // short sums need no room behind the ring
+    cfg.dynamicSmemBytes = smem_bytes(BM, BM == 64 && (parts > 1 || K > kFold * BK));
     cfg.stream = st;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
@@ -221,7 +240,7 @@ static cudaError_t launch(int M, int N, int K, const Opd &A, const Opd &B, doubl
     cfg.attrs = &at;
     cfg.numAttrs = parts > 1 ? 1 : 0;
     auto go = [&](auto kern) {
-        const cudaError_t ce = smem_optin(reinterpret_cast<const void *>(kern), (int)ring_bytes(BM));
+        const cudaError_t ce = smem_optin(reinterpret_cast<const void *>(kern), (int)cfg.dynamicSmemBytes);
         return ce != cudaSuccess ? ce : cudaLaunchKernelEx(&cfg, kern, M, N, K, A, B, C, cr, cc, alpha, acc ? 1 : 0);
     };
     // consecutive threads along the operand's contiguous index
