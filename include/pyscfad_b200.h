@@ -360,6 +360,7 @@ int ct_df_layouts(int nocc, int nvir, int naux, const double *Loo, const double 
  * vooo_bar and vvop_bar into dLoo (naux, nocc, nocc), dLov (naux, nocc, nvir)
  * and dRt (naux, nvir, nmo), the gradient of Rt = R transposed in its last two
  * axes (Rt is passed too); the caller splits dRt into the Lov and Lvv parts.
+ * All sums run in a fixed order: the same inputs give the same bits.
  */
 int ct_df_factor_bar(int nocc, int nvir, int naux, const double *Loo, const double *Lov, const double *Rt,
                      const double *vooo_bar, const double *vvop_bar, double *dLoo, double *dLov, double *dRt,

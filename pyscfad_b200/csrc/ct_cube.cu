@@ -81,8 +81,9 @@ __global__ void __launch_bounds__(MAXT, MINB) job_kernel(const Args A) {
     const int g = lane >> 2, c4 = lane & 3;
     const int sj = A.sj, si = A.si;
     constexpr int HR = 4 * MT;   // F1/F2 rows of a term (o <= HR)
-    // k-steps of B requested ahead: one is enough with two CTAs per SM (two spill;
-    // nocc=16/nvir=120 energy 84 against 89 ms), two with one (31.5 against 33.0 ms)
+    // k-steps of B requested ahead: one is enough with two CTAs per SM (two spill more;
+    // nocc=16/nvir=120 energy 84 against 89 ms), two with one (31.5 against 33.0 ms).
+    // With one, eight of the builds in use spill 4 to 28 bytes.
     constexpr int PF = MT == 6 ? 2 : 1;
     double *W = sm;                          // the cube, (i, j, k) at i si + j sj + k
     double *St = W + A.cube_sz;              // GEMM staging, later the V-term tiles

@@ -25,9 +25,9 @@ namespace ctb {
 // loads: staging the blocks in shared memory (64-thread CTAs, 36 tiles of 4^3)
 // spent 4000 instructions per block-orbit on addresses, copies and barriers and
 // wrote six W-bar cubes: 50 -> 31 ms over the 6,213 jobs of a nocc=48/nvir=300
-// slab block, 307 -> 94 ms for all jobs of nocc=33/nvir=64 with fvo.  w-bar goes to slots 0-2 as three copies of one cube,
-// [i][j][k], [i][k][j] and [j][k][i]: each W-bar_sigma is one of them with r
-// contiguous (ct_pair.cu).
+// slab block, 307 -> 94 ms for all jobs of nocc=33/nvir=64 with fvo.  w-bar goes
+// to slots 0-2 as three copies of one cube, [i][j][k], [i][k][j] and [j][k][i]:
+// each W-bar_sigma is one of them with r contiguous (ct_pair.cu).
 // ---------------------------------------------------------------------------
 enum EpiMode { E_ENERGY, E_VJP, E_LNO_FWD, E_LNO_BWD, E_T3 };
 constexpr int kEpiThreads = 256, kEpiWarps = kEpiThreads / 32;

@@ -53,9 +53,10 @@ cudaError_t smem_optin(const void *kernel, int bytes) {
     return cudaSuccess;
 }
 
-// The float64 path that keeps a job's cube in shared memory (ct_cube.cu): its
-// largest cube, V tiles and partials take 193 KB at nocc = 24.  nocc = 1 stays
-// on the slot path (a cube of one element).
+// The float64 path that keeps a job's cube in shared memory (ct_cube.cu): the cube,
+// the larger of the GEMM staging and the V tiles, and the gradients' partials take
+// up to 222 of the 227 KB (nocc = 24 with 97-112 virtuals).  nocc = 1 stays on the
+// slot path (a cube of one element).
 static bool cube_size(int o) { return o >= 2 && o <= kCubeMaxO; }
 
 struct Plan {

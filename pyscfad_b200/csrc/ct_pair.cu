@@ -1,5 +1,6 @@
-// Float64 GEMMs of the slot path (nocc > 24, nocc = 1, the iterative solver's
-// seed) on the float64 tensor pipe.  The operations per term t = (job, sigma)
+// Float64 GEMMs of the slot path (nocc > 24, nocc = 1; the W build also for the
+// iterative solver's seed, the allocation-free energy and energies over few jobs at
+// every nocc) on the float64 tensor pipe.  The operations per term t = (job, sigma)
 // with (x, y, z) as in ct_common.cuh:
 //   W    G_t[p,qr]  = sum_f vvop[x,y,p,o+f] t2T[z,f,qr] - sum_l vooo[x,pq,l] t2T[z,y,l,r]
 //                                                     (get_wv, ccsd_t.c:98-152)

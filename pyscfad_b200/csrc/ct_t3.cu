@@ -7,12 +7,16 @@
 //   t3_new = (P6(W + V) + P3(fvv' t3) - P3(foo' t3)) / d3
 //          = t3_c + (P3(tvv) - P3(too)) / d3,
 // P3(x)[abc][ijk] = x[abc][ijk] + x[bac][jik] + x[cba][kji] (:174-176), with
-// fvv', foo' the Fock blocks without their diagonals.  The caller forms the
-// two products as plain GEMMs: tvv = fvv' t3 on the first virtual index of
-// the [a][b][c][i][j][k] array, too = foo' t3 on the first occupied index of
-// an occupied-major copy [i][a][b][c][j][k], which this kernel also writes
-// for the next step (t3_new_m).  It applies P3, divides by d3 and forms, in a
-// fixed order, |t3_new - t3|^2 and the energy sum t3_new t3_x.
+// fvv', foo' the Fock blocks without their diagonals.  The caller forms
+// tvv = fvv' t3 on the first virtual index of the [a][b][c][i][j][k] array as a
+// plain GEMM.  Two kernels apply P3, divide by d3 and form, in a fixed order,
+// |t3_new - t3|^2 and the energy sum t3_new t3_x:
+//   step_kernel    forms the foo' products itself from t3's cubes (ct_t3_step);
+//                  the faster one up to nocc = 9 and at even nocc <= 20
+//   update_kernel  takes too = foo' t3 on the first occupied index of an
+//                  occupied-major copy [i][a][b][c][j][k], formed by the caller
+//                  as a second GEMM, and writes that copy for the next step
+//                  (ct_t3_update)
 #include <cuda_runtime.h>
 #include <algorithm>
 #include "ct_common.cuh"
@@ -103,16 +107,18 @@ __global__ void sum_kernel(const double *__restrict__ part, double *__restrict__
 // which drops the occupied-major copy (written each step and read as four more
 // arrays).  A CTA takes a sorted triple a >= b >= c at a time and its up to six
 // orderings one after the other, so that the cubes of tvv and t3 that P3 pairs
-// are re-read from L2.  Bound by memory: 5 arrays (t3, tvv, t3_c, t3_x in,
-// t3_new out) of v^3 o^3 doubles.
+// are re-read from L2.  The floor is memory: 5 arrays (t3, tvv, t3_c, t3_x in,
+// t3_new out) of v^3 o^3 doubles, 202 us at the copy rate at nocc=8/nvir=40.
 // With nocc even and <= kStepMaxO (PAIRED) the ordering's three t3 cubes are
 // staged in shared memory and a thread owns a 2 x 2 x 2 block of (i, j, k): per m
-// nine 16-byte shared loads feed 24 multiply-adds (one element a thread takes six
-// 8-byte loads for 3 and was bound by them: 768 us a step at nocc=8/nvir=40,
-// 466 us as blocks, against 202 us for the five arrays at the copy rate).  Two
-// CTAs of 256 threads' registers: more resident warps or fewer registers
-// measured slower (499 us unbounded, 625 us at three).
-// Otherwise one element a thread, t3 read through L1.
+// nine 16-byte shared loads feed 24 multiply-adds.  Bound by L1/TEX (81% in ncu,
+// DRAM 39%): 466 us at nocc=8/nvir=40; one element a thread takes six 8-byte
+// loads for 3 multiply-adds, 768 us.  Two CTAs of 256 threads' registers: more
+// resident warps or fewer registers measured slower (499 us unbounded, 625 us at
+// three).
+// Otherwise one element a thread, t3 read through L1: 2 nocc loads of three cubes
+// an element, so that from nocc = 11 (for large arrays) a GEMM and update_kernel
+// are faster (nocc=24/nvir=16 4.5 ms a cycle against 2.2); the caller chooses.
 constexpr int kStepMaxO = 20, kStepThreads = 256, kStepBlocks = CT_T3_STEP_WORK / 2;
 
 struct StepSums {
